@@ -277,9 +277,12 @@ int se_linsys_assemble(se_linsys* ls);
 int se_linsys_solve(se_linsys* ls, int remove_null_space, se_solve_stats* stats);
 /* Several solves in one call (the batched ensemble; no counterpart in the
  * reference, which solves one system at a time through the same Solve).
- * Systems using SE_METHOD_CG and the same polynomial order run as one
- * persistent cooperative launch (up to 256 per launch) whose launch shape is
- * chosen by a built-in autotuner on the first batch of a given signature;
+ * Systems using SE_METHOD_CG and the same polynomial order run in persistent
+ * cooperative launches, each solve on a team of blocks of its own with its
+ * whole state on the chip. A group with a system that does not fit (above
+ * about 600,000 unknowns) or has an SVV term runs as one launch (up to 256
+ * systems) whose shape is chosen by a built-in autotuner on the first batch
+ * of a given signature;
  * SE_METHOD_FDM systems run their solve graphs overlapped on a pool of 8
  * streams. stats (nullable) gets one entry per system; the return value is
  * SE_ERR_NOT_CONVERGED if any system diverged. The caller's stream is ordered

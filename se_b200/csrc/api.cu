@@ -258,6 +258,13 @@ struct se_linsys {
   int* d_active;
   unsigned* d_err;
   int grid, nseg, seg_begin, seg_end;
+  // FP64 CG on the chip (cg_patch.cu): its cut, packets (allocated by the
+  // first such solve) and result; patch_seq counts the launches on d_pkts
+  bool patch;
+  PatchPlan pplan;
+  PatchPkt* d_pkts;
+  PatchResult* d_pres;
+  unsigned long long patch_seq;
   cudaEvent_t ev[3];  // FDM solve: graph start, graph end, state copied to the host
   // fast diagonalization (built on the first FDM solve)
   bool fdm_ready;
@@ -531,6 +538,8 @@ void linsys_free(se_linsys* ls) {
   dfree(ls->d_bar);
   dfree(ls->d_active);
   dfree(ls->d_err);
+  dfree(ls->d_pkts);
+  dfree(ls->d_pres);
   dfree(ls->d_rescount);
   dfree(ls->X1);
   dfree(ls->X2);
@@ -595,6 +604,9 @@ int linsys_alloc(se_linsys* ls) {
   CK(cudaGetDevice(&dev));
   const int grid = cg_plan(dev, ls->op.d[0].N, cg_tiles(ls->op), 1, &ls->resident);
   if (grid <= 0) return fail(SE_ERR_CUDA, "cannot size the cooperative CG launch");
+  int sms = 0;
+  CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+  ls->patch = patch_plan(ls->op, sms, &ls->pplan);
   Schedule S = make_schedule({&ls->op}, grid);
   ls->grid = (int)S.block_begin.size() - 1;
   ls->nseg = S.nseg;
@@ -618,9 +630,103 @@ int linsys_alloc(se_linsys* ls) {
   return SE_OK;
 }
 
+// Sequence numbers of one launch: a reduction takes one, an iteration at most
+// three, so a launch of 2^31 - 1 iterations stays below the next one's first.
+constexpr int kPatchSeqShift = 34;
+
+PatchSolve make_patch(const OpDev& op, const double* b, double* x, double rtol, double atol,
+                      double dtol, int max_it, int norm_type, int remove_null,
+                      const PatchPlan& plan, PatchPkt* pkts, unsigned long long launch) {
+  PatchSolve ps;
+  std::memset(&ps, 0, sizeof(ps));
+  ps.d[0] = op.d[0];
+  ps.d[1] = op.d[1];
+  ps.G0 = op.G[0];
+  ps.n = op.G[0] * op.G[1];
+  ps.alpha = op.alpha;
+  ps.bx = op.beta[0];
+  ps.by = op.beta[1];
+  ps.b = b;
+  ps.x = x;
+  ps.rtol = rtol;
+  ps.atol = atol;
+  ps.dtol = dtol;
+  ps.max_it = max_it;
+  ps.norm_type = norm_type;
+  ps.remove_null = remove_null;
+  ps.gx = plan.gx;
+  ps.gy = plan.gy;
+  ps.edge_stride = plan.edge_stride;
+  ps.slots = pkts;
+  ps.edges = pkts + 3 * kPatchLine * (size_t)plan.gx * plan.gy;
+  ps.seq0 = launch << kPatchSeqShift;
+  return ps;
+}
+
+PatchLaunch patch_launch(const OpDev& op, int blocks, bool in_registers, size_t smem,
+                         PatchResult* res) {
+  PatchLaunch L;
+  std::memset(&L, 0, sizeof(L));
+  L.N = op.d[0].N;
+  L.blocks = blocks;
+  L.in_registers = in_registers;
+  L.smem = smem;
+  L.res = res;
+  L.Kh = op.Kh;
+  L.w = op.w;
+  return L;
+}
+
+// The state a finished on-chip solve reports, in the streaming kernel's form.
+CgSolve patch_state(const PatchResult& r) {
+  CgSolve st;
+  std::memset(&st, 0, sizeof(st));
+  st.dp = r.dp;
+  st.rnorm0 = r.rnorm0;
+  st.beta = r.beta;
+  st.its = r.its;
+  st.reason = r.reason;
+  st.done = 1;
+  return st;
+}
+
+// Run the on-chip CG for A x = b (the system's cut fits); fills stats.
+int run_cg_patch(se_linsys* ls, const double* b, double* x, double rtol, double atol, double dtol,
+                 int max_it, int remove_null, CgSolve* out_state, float* kernel_ms) {
+  cudaStream_t s = g_stream;
+  if (!ls->d_pkts) {
+    int rc;
+    const size_t np = patch_packets(ls->pplan);
+    if ((rc = dalloc(&ls->d_pres, 1)) || (rc = dalloc(&ls->d_pkts, np))) return rc;
+    CK(cudaMemsetAsync(ls->d_pkts, 0, sizeof(PatchPkt) * np, s));
+    CK(cudaMemsetAsync(ls->d_pres, 0, sizeof(PatchResult), s));
+  }
+  const PatchSolve ps = make_patch(ls->op, b, x, rtol, atol, dtol, max_it, ls->opts.norm_type,
+                                   remove_null, ls->pplan, ls->d_pkts, ++ls->patch_seq);
+  PatchLaunch L = patch_launch(ls->op, ls->pplan.gx * ls->pplan.gy, ls->pplan.in_registers,
+                               ls->pplan.smem, ls->d_pres);
+  L.one = &ps;
+  if (!ls->ev[0]) {
+    CK(cudaEventCreate(&ls->ev[0]));
+    CK(cudaEventCreate(&ls->ev[1]));
+  }
+  CK(cudaEventRecord(ls->ev[0], s));
+  CK(launch_cg_patch(L, s));
+  CK(cudaEventRecord(ls->ev[1], s));
+  PatchResult r;
+  CK(cudaMemcpyAsync(&r, ls->d_pres, sizeof(r), cudaMemcpyDeviceToHost, s));
+  CK(cudaStreamSynchronize(s));
+  if (kernel_ms) CK(cudaEventElapsedTime(kernel_ms, ls->ev[0], ls->ev[1]));
+  if (r.err == ps.seq0) return fail(SE_ERR_TIMEOUT, "CG packet wait timed out");
+  *out_state = patch_state(r);
+  return SE_OK;
+}
+
 // Run the persistent CG for A x = b on this system's schedule; fills stats.
 int run_cg(se_linsys* ls, const double* b, double* x, double rtol, double atol, double dtol,
            int max_it, int remove_null, CgSolve* out_state, float* kernel_ms, int lowp = 0) {
+  if (lowp == 0 && ls->patch)
+    return run_cg_patch(ls, b, x, rtol, atol, dtol, max_it, remove_null, out_state, kernel_ms);
   CgSolve cs = make_solve(ls, b, x, rtol, atol, dtol, max_it, remove_null);
   cudaStream_t s = g_stream;
   CK(cudaMemcpyAsync(ls->d_solve, &cs, sizeof(cs), cudaMemcpyHostToDevice, s));
@@ -1755,7 +1861,8 @@ int grow(T** p, size_t* cap, size_t need) {
   return SE_OK;
 }
 
-// Launch-shape autotuner for batched CG: for a batch signature (order,
+// Launch-shape autotuner for batched CG of systems that do not all fit the
+// on-chip kernel: for a batch signature (order,
 // number of solves, tile count rounded up to a power of two) it times short
 // capped runs (30 iterations) of each candidate -- the register-resident
 // mode when it fits, and the streaming mode at 1, 2 and 4 blocks per SM --
@@ -1822,11 +1929,168 @@ int run_cg_batch_once(int dev, std::vector<se_linsys*>& sys, const std::vector<c
   return SE_OK;
 }
 
+// Batched on-chip CG: every solve gets a team of blocks of its own (no team
+// waits for another), several teams a launch. Solves are sorted by estimated
+// work and cut into launches that fit the device at their smallest teams;
+// each launch's spare blocks then go, one cut at a time, to the solve that
+// would finish last (iterations grow with the longer side's element count at
+// equal order, an iteration costs its reductions' latency plus the cut's
+// work). Packing beats giving one solve the whole device: an iteration's two
+// reductions (about 2 us) do not shrink with more blocks.
+constexpr double kPatchLatency = 4500.0;  // cycles of an iteration's reductions
+struct PatchWs {
+  PatchPkt* pkts = nullptr;
+  PatchSolve* solves = nullptr;
+  int* cta = nullptr;
+  PatchResult* res = nullptr;
+  size_t cap_pkts = 0, cap_solves = 0, cap_cta = 0, cap_res = 0;
+  unsigned long long seq = 0;
+};
+PatchWs g_patch[64];
+// best cut for every block count, by order and element counts
+std::map<std::tuple<int, int, int, int>, std::vector<PatchPlan>> g_patch_tables;
+
+int run_patch_group(int dev, std::vector<se_linsys*>& sys, int remove_null,
+                    std::vector<CgSolve>& out, float* ms) {
+  int sms = 0;
+  CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+  const int cap = std::min(sms, kPatchMaxBlocks), n = (int)sys.size();
+  std::vector<const std::vector<PatchPlan>*> tab(n);
+  std::vector<int> g(n), order(n);
+  auto its = [&](int i) { return (double)std::max(sys[i]->op.d[0].nE, sys[i]->op.d[1].nE); };
+  auto time = [&](int i, int blocks) {
+    return its(i) * (kPatchLatency + (*tab[i])[blocks].cost);
+  };
+  for (int i = 0; i < n; i++) {
+    const OpDev& op = sys[i]->op;
+    std::vector<PatchPlan>& t =
+        g_patch_tables[std::make_tuple(cap, op.d[0].N, op.d[0].nE, op.d[1].nE)];
+    if (t.empty()) {
+      t.resize(cap + 1);
+      patch_plan_table(op, cap, t.data());
+    }
+    tab[i] = &t;
+    g[i] = 1;
+    while (g[i] < cap && t[g[i]].gx == 0) g[i]++;
+    order[i] = i;
+  }
+  std::sort(order.begin(), order.end(), [&](int a, int b) {
+    const double ta = its(a) * sys[a]->n, tb = its(b) * sys[b]->n;
+    return ta != tb ? ta > tb : a < b;
+  });
+  std::vector<int> first = {0};  // launches: ranges of `order`
+  int used = 0;
+  for (int k = 0; k < n; k++) {
+    if (used + g[order[k]] > cap) {
+      first.push_back(k);
+      used = 0;
+    }
+    used += g[order[k]];
+  }
+  first.push_back(n);
+  const int nl = (int)first.size() - 1;
+  for (int l = 0; l < nl; l++) {
+    int spare = cap;
+    for (int k = first[l]; k < first[l + 1]; k++) spare -= g[order[k]];
+    std::vector<char> stuck(n, 0);
+    for (;;) {
+      int w = -1;
+      for (int k = first[l]; k < first[l + 1]; k++)
+        if (!stuck[order[k]] && (w < 0 || time(order[k], g[order[k]]) > time(w, g[w])))
+          w = order[k];
+      if (w < 0) break;
+      int to = g[w] + 1;
+      while (to <= std::min(cap, g[w] + spare) && (*tab[w])[to].cost >= 0.98 * (*tab[w])[g[w]].cost)
+        to++;
+      if (to > std::min(cap, g[w] + spare)) {
+        stuck[w] = 1;
+        continue;
+      }
+      spare -= to - g[w];
+      g[w] = to;
+    }
+  }
+  // solves, teams and packets of every launch
+  PatchWs& W = g_patch[dev];
+  cudaStream_t s = g_stream;
+  size_t npk = 0;
+  for (int i = 0; i < n; i++) npk += patch_packets((*tab[i])[g[i]]);
+  int rc;
+  if (W.cap_pkts < npk) {
+    if ((rc = grow(&W.pkts, &W.cap_pkts, npk))) return rc;
+    CK(cudaMemsetAsync(W.pkts, 0, sizeof(PatchPkt) * W.cap_pkts, s));
+  }
+  W.seq++;
+  std::vector<PatchSolve> solves(n);
+  std::vector<int> cta;
+  std::vector<int> cta_first;
+  size_t at = 0;
+  for (int l = 0; l < nl; l++) {
+    cta_first.push_back((int)cta.size());
+    const int base = (int)cta.size();
+    for (int k = first[l]; k < first[l + 1]; k++) {
+      const int i = order[k];
+      se_linsys* ls = sys[i];
+      const PatchPlan& p = (*tab[i])[g[i]];
+      solves[i] = make_patch(ls->op, ls->f, ls->x, ls->opts.rtol, ls->opts.atol, ls->opts.dtol,
+                             ls->opts.max_it, ls->opts.norm_type, remove_null, p, W.pkts + at,
+                             W.seq);
+      solves[i].cta0 = (int)cta.size() - base;
+      at += patch_packets(p);
+      cta.insert(cta.end(), (size_t)p.gx * p.gy, i);
+    }
+  }
+  cta_first.push_back((int)cta.size());
+  if ((rc = grow(&W.solves, &W.cap_solves, (size_t)n)) || (rc = grow(&W.cta, &W.cap_cta, cta.size())) ||
+      (rc = grow(&W.res, &W.cap_res, (size_t)n)))
+    return rc;
+  CK(cudaMemcpyAsync(W.solves, solves.data(), sizeof(PatchSolve) * n, cudaMemcpyHostToDevice, s));
+  CK(cudaMemcpyAsync(W.cta, cta.data(), sizeof(int) * cta.size(), cudaMemcpyHostToDevice, s));
+  CK(cudaMemsetAsync(W.res, 0, sizeof(PatchResult) * n, s));
+  cudaEvent_t e0, e1;
+  CK(cudaEventCreate(&e0));
+  CK(cudaEventCreate(&e1));
+  CK(cudaEventRecord(e0, s));
+  cudaError_t le = cudaSuccess;
+  for (int l = 0; l < nl && le == cudaSuccess; l++) {
+    // one kernel form for the launch: all state in registers if every cut has it
+    bool regs = true;
+    for (int k = first[l]; k < first[l + 1]; k++)
+      regs = regs && (*tab[order[k]])[g[order[k]]].in_registers;
+    size_t smem = 0;
+    for (int k = first[l]; k < first[l + 1]; k++) {
+      const se_linsys* ls = sys[order[k]];
+      smem = std::max(smem, patch_smem_bytes(ls->op, (*tab[order[k]])[g[order[k]]], regs));
+    }
+    PatchLaunch L = patch_launch(sys[0]->op, cta_first[l + 1] - cta_first[l], regs, smem, W.res);
+    L.solves = W.solves;
+    L.cta_solve = W.cta + cta_first[l];
+    le = launch_cg_patch(L, s);
+  }
+  CK(cudaEventRecord(e1, s));
+  std::vector<PatchResult> res(n);
+  CK(cudaMemcpyAsync(res.data(), W.res, sizeof(PatchResult) * n, cudaMemcpyDeviceToHost, s));
+  CK(cudaStreamSynchronize(s));
+  if (ms) cudaEventElapsedTime(ms, e0, e1);
+  cudaEventDestroy(e0);
+  cudaEventDestroy(e1);
+  if (le != cudaSuccess) return cuda_fail(le, "batched CG launch");
+  out.resize(n);
+  for (int i = 0; i < n; i++) {
+    if (res[i].err == solves[i].seq0) return fail(SE_ERR_TIMEOUT, "CG packet wait timed out");
+    out[i] = patch_state(res[i]);
+  }
+  return SE_OK;
+}
+
 int solve_cg_group(std::vector<se_linsys*>& sys, int remove_null, std::vector<CgSolve>& out, float* ms) {
   int dev = 0;
   CK(cudaGetDevice(&dev));
   std::lock_guard<std::mutex> lk(g_batch_mu);
   const int N = sys[0]->op.d[0].N;
+  bool patch = true;
+  for (const se_linsys* ls : sys) patch = patch && ls->patch;
+  if (patch) return run_patch_group(dev, sys, remove_null, out, ms);
   std::vector<const OpDev*> ops;
   long ntiles = 0;
   for (se_linsys* ls : sys) {
@@ -3122,6 +3386,42 @@ extern "C" int se_helmholtz_solve_noalloc(const int nEls[2], int N, const double
                                         kNoAllocTileDoubles);
   unsigned* words = reinterpret_cast<unsigned*>(partials + kNoAllocPartialDoubles + kNoAllocSolveDoubles +
                                                 kNoAllocTileDoubles + kNoAllocBeginDoubles);
+
+  // on the chip, as the allocating path: packets over the vectors z, p0, p1
+  // and w, which that solve does not use (zeroed: they may hold anything)
+  int sms = 0;
+  CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
+  PatchPlan plan;
+  if (patch_plan(op, sms, &plan) && sizeof(PatchPkt) * patch_packets(plan) <= sizeof(double) * 4 * vn) {
+    cudaStream_t st = g_stream;
+    PatchPkt* pk = reinterpret_cast<PatchPkt*>(z);
+    PatchResult* d_res = reinterpret_cast<PatchResult*>(d_solve);
+    const PatchSolve ps = make_patch(op, f, x, o.rtol, o.atol, o.dtol, o.max_it, o.norm_type,
+                                     remove_null_space, plan, pk, 1);
+    PatchLaunch L = patch_launch(op, plan.gx * plan.gy, plan.in_registers, plan.smem, d_res);
+    L.one = &ps;
+    CK(cudaMemsetAsync(pk, 0, sizeof(PatchPkt) * patch_packets(plan), st));
+    CK(cudaMemsetAsync(d_res, 0, sizeof(PatchResult), st));
+    CK(launch_lift(op, md, sol_dev, lift, st));
+    CK(launch_rhs_assemble(op, md, rhs_dev, lift, f, st));
+    CK(launch_cg_patch(L, st));
+    PatchResult r;
+    CK(cudaMemcpyAsync(&r, d_res, sizeof(r), cudaMemcpyDeviceToHost, st));
+    CK(launch_update_field(op, md, x, sol_dev, st));
+    CK(cudaStreamSynchronize(st));
+    if (r.err == ps.seq0) return fail(SE_ERR_TIMEOUT, "CG packet wait timed out");
+    if (stats) {
+      stats->reason = r.reason;
+      stats->its = r.its;
+      stats->outer_its = 0;
+      stats->rnorm = r.dp;
+      stats->rnorm0 = r.rnorm0;
+      stats->kernel_ms = 0.0;
+    }
+    if (r.reason < 0)
+      return fail(SE_ERR_NOT_CONVERGED, "KSP diverged, reason %d after %d its", r.reason, r.its);
+    return SE_OK;
+  }
 
   // schedule: same tile order, mode and contiguous block chunks as the
   // allocating path

@@ -1,6 +1,10 @@
 // Persistent, deterministic Jacobi-preconditioned CG over a batch of
 // Helmholtz/Poisson solves of one polynomial order N, sm_100a.
 //
+// FP64 solves that fit the chip run cg_patch.cu's kernel; this one serves what
+// does not: systems above about 600,000 unknowns, SVV operators, and the
+// reduced-precision apply.
+//
 // One cooperative launch runs every iteration of every solve in the batch.
 // The unknown grid of each solve is cut into tiles of kCgTileX x kCgTileY
 // unknowns, assigned in contiguous chunks to the resident blocks, one

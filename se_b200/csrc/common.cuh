@@ -263,6 +263,68 @@ int cg_max_grid(int device, int N, bool resident, int nsolves, int lowp = 0);
 cudaError_t launch_cg(const CgBatch& batch, int grid, int N, bool resident, cudaStream_t s,
                       int lowp = 0);
 
+// CG with the whole iteration state on the chip (cg_patch.cu): a solve cut
+// into gx x gy patches of elements, one block each.
+struct PatchPkt {  // a value and its sequence number, stored and read as one 16-byte word
+  double v;
+  unsigned long long seq;
+};
+struct PatchSolve {
+  Dir d[2];
+  int G0;             // unknowns per row
+  int n;              // unknowns
+  double alpha, bx, by;
+  const double* b;
+  double* x;
+  double rtol, atol, dtol;
+  int max_it, norm_type, remove_null;
+  int gx, gy, cta0;   // patches, first block of this solve
+  int edge_stride;    // packets of one patch edge, whole lines
+  int pad;
+  PatchPkt* slots;    // sum packets: 3 arrays of one line per patch (128-byte aligned)
+  PatchPkt* edges;    // 4 edge_stride gx gy edge packets
+  unsigned long long seq0;  // first sequence number: above any used on these packets before,
+                            // with room for the reductions of max_it iterations
+};
+struct PatchResult {
+  double dp, rnorm0, beta;
+  int its, reason;
+  unsigned long long err;  // seq0 of the launch whose wait gave up
+};
+struct PatchPlan {
+  int gx, gy, edge_stride;
+  bool in_registers;  // every block's nodes fit the kernel form with all state in registers
+  size_t smem;
+  double cost;  // modelled cycles of an iteration's work
+};
+struct PatchLaunch {
+  int N, blocks;
+  bool in_registers;
+  size_t smem;
+  const PatchSolve* one;     // host: the solve of a single-solve launch
+  const PatchSolve* solves;  // device: a batch's solves (then one is null)
+  const int* cta_solve;      // device: solve of each block (batch)
+  PatchResult* res;          // device, one per solve
+  const double* Kh;          // host: (N+1)^2 element stiffness and N+1 weights
+  const double* w;
+};
+constexpr int kPatchThreads = 512;
+constexpr int kPatchMaxBlocks = 160;
+constexpr int kPatchLine = 8;  // packets of a 128-byte line
+constexpr int kPatchSmemMax = 224 * 1024;
+// The cut of an operator over at most max_blocks blocks; false: it does not
+// fit on the chip (or has an SVV term).
+bool patch_plan(const OpDev& op, int max_blocks, PatchPlan* out);
+// The best cut for every block count 0..max_blocks (gx == 0: it does not fit).
+void patch_plan_table(const OpDev& op, int max_blocks, PatchPlan* out);
+// Shared memory of a plan's blocks in one of the two kernel forms.
+size_t patch_smem_bytes(const OpDev& op, const PatchPlan& p, bool in_registers);
+// Sum and edge packets of a plan.
+inline size_t patch_packets(const PatchPlan& p) {
+  return (size_t)p.gx * p.gy * (3 * kPatchLine + 4 * (size_t)p.edge_stride);
+}
+cudaError_t launch_cg_patch(const PatchLaunch& L, cudaStream_t s);
+
 // Device-resident parameters and state of an FDM refinement loop.
 struct FdmParams {
   double rtol, atol, dtol;

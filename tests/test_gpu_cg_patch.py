@@ -1,0 +1,103 @@
+"""The on-chip CG (patches of elements, one block each) at the edges of its
+range: single elements, two elements around a periodic direction, element
+counts that no cut divides, the largest patch of each kernel form and the
+first size beyond it, every norm and null-space mode, and batches whose teams
+need several launches.
+
+Tolerances: iteration counts within 2 of the oracle's and solutions at rtol
+1e-12 within 1e-8 of its magnitude, as for every CG solve of the suite; where
+the oracle's matrix would be too large, against the fast-diagonalization
+solution of the same system; batched against single solves 1e-10.
+"""
+import numpy as np
+import pytest
+
+from test_gpu_linsys import build
+
+pytestmark = pytest.mark.gpu
+
+P, CH, BOX = (True, True), (True, False), (False, False)
+NONE, TB, ALL = (False,) * 4, (True, True, False, False), (True,) * 4
+
+SMALL = [
+    (1, 1, 12, (0.0, 0.0), (1.0, 2.0), BOX, ALL),
+    (1, 1, 3, (0.0, 0.0), (1.0, 1.0), BOX, NONE),
+    (2, 2, 2, (-1.0, 0.0), (1.0, 1.0), P, NONE),
+    (2, 5, 9, (0.0, 0.0), (1.0, 1.0), CH, TB),
+    (31, 1, 5, (0.0, 0.0), (7.0, 1.0), BOX, NONE),
+    (13, 11, 8, (0.0, 0.0), (1.0, 1.0), CH, TB),
+    (19, 17, 6, (0.0, -1.0), (2.0, 1.0), P, NONE),
+    (7, 9, 11, (0.0, 0.0), (1.0, 1.0), BOX, ALL),
+]
+
+
+@pytest.mark.parametrize("case", range(len(SMALL)))
+@pytest.mark.parametrize("norm", [0, 1, 2])
+def test_matches_oracle(segpu, oracle, case, norm):
+    om, m, fs, fr, ls, A, f2v, v2f, sol, rhs = build(segpu, oracle, SMALL[case], -3.0, -1.0, 1.0,
+                                                     True, seed=case + 40)
+    ref, st = oracle.helmholtz_solve(om, sol, rhs, -3.0, -1.0, 1.0, bcs=SMALL[case][6], quirk=True,
+                                     rtol=1e-12, norm_type=norm)
+    ls.set_opts(segpu.solver_opts(rtol=1e-12, norm_type=norm))
+    out = ls.Solve("helm_")
+    assert st["reason"] == out["reason"] == 2
+    assert abs(out["its"] - st["its"]) <= 2, (out, st)
+    got = fs.vals
+    assert np.abs(got - ref).max() <= 1e-8 * np.abs(ref).max()
+    assert np.array_equal(got[f2v < 0], sol[f2v < 0])
+
+
+def smooth(S, ne, p, lam, method, rtol=1e-11):
+    m = S.Mesh("m", list(ne), "legendre", p, [0, 0], [1, 1], [True, True])
+    b = S.BCs(False, False, False, False, m)
+    X = m.verts
+    u, f = S.Field("u", m, 1, b), S.Field("f", m, 1, b)
+    f.vals = np.cos(2 * np.pi * X[:, 0]) * np.sin(4 * np.pi * X[:, 1]) + 0.2
+    ls = S.HelmholtzEqn(u, f, -lam, -1.0, 1.0, 0,
+                        S.solver_opts(rtol=rtol, mode=S.MODE_EXACT, method=method))
+    return m, u, f, ls
+
+
+# 148 patches of at most 2048 nodes (all state in registers), of at most 4096,
+# and beyond (the streaming kernel)
+@pytest.mark.parametrize("ne,p", [((64, 64), 8), ((70, 72), 8), ((81, 80), 8), ((100, 104), 8),
+                                  ((150, 3), 12), ((3, 260), 4)])
+def test_large_matches_fast_diagonalization(segpu, ne, p):
+    out = {}
+    for method in (segpu.METHOD_CG, segpu.METHOD_FDM):
+        m, u, f, ls = smooth(segpu, ne, p, 20.0, method)
+        assert ls.Solve()["reason"] == 2
+        out[method] = u.vals
+    ref = out[segpu.METHOD_FDM]
+    assert np.abs(out[segpu.METHOD_CG] - ref).max() <= 1e-8 * np.abs(ref).max()
+
+
+def test_batch_over_several_launches(segpu):
+    """Four large systems beside 60 small ones: more blocks than one launch
+    holds, teams of one block and of many."""
+    sizes = [(40, 44), (52, 30), (36, 36), (48, 41)] + [(2 + k % 7, 3 + k % 5) for k in range(60)]
+    systems = [smooth(segpu, s, 8, 1.0 + k, segpu.METHOD_CG) for k, s in enumerate(sizes)]
+    singles = []
+    for m, u, f, ls in systems:
+        st = ls.Solve()
+        singles.append((u.vals, st))
+        u.vals = 0.0
+    stats = segpu.solve_batch([s[3] for s in systems])
+    for (m, u, f, ls), (ref, rst), st in zip(systems, singles, stats):
+        assert st["reason"] == rst["reason"] == 2
+        assert abs(st["its"] - rst["its"]) <= 2
+        assert np.abs(u.vals - ref).max() <= 1e-10 * np.abs(ref).max()
+
+
+def test_iteration_limits_and_zero_rhs(segpu):
+    m, u, f, ls = smooth(segpu, (9, 8), 6, 1.0, segpu.METHOD_CG)
+    ls.set_opts(segpu.solver_opts(rtol=1e-12, mode=segpu.MODE_EXACT, max_it=5))
+    st = ls.Solve()
+    assert (st["reason"], st["its"]) == (-3, 5)
+    ls.set_opts(segpu.solver_opts(rtol=1e-12, mode=segpu.MODE_EXACT, max_it=0))
+    assert ls.Solve()["its"] == 0
+    f.vals = 0.0
+    ls.set_opts(segpu.solver_opts(rtol=1e-12, mode=segpu.MODE_EXACT))
+    st = ls.Solve()
+    assert st["its"] == 0 and st["reason"] in (2, 3)
+    assert not np.any(u.vals)
