@@ -232,6 +232,7 @@ struct se_field {
 struct se_advector {
   se_field *field, *vel, *field_prev, *vel_prev;
   se_field* sl;
+  double* mix;  // second order: the half-level velocities' work (null: formed in the gathers)
   int* dep_el;
   double* dep_xy;
   unsigned* err;  // device error bits of this advector's SL kernels
@@ -2140,6 +2141,37 @@ int solve_cg_group(std::vector<se_linsys*>& sys, int remove_null, std::vector<Cg
 }
 }  // namespace
 
+namespace {
+// Whether the coordinate of every vertex along direction k gives back that
+// vertex: the element search and the 1e-8 node snap of the SL kernels on the
+// vertex coordinates, the same operations. Fails only where a coordinate's
+// rounding reaches 1e-8 of an element (a domain some 1e7 elements from 0).
+bool vertices_snap(const MeshDev& m, int k) {
+  for (int t = 0; t < m.nVerts[k]; t++) {
+    const int e = t / m.N;
+    const double a = m.abcissa[t - e * m.N];
+    const double c = (m.min[k] + (double)e * m.dx[k]) + ((a + 1.0) / 2.0) * m.dx[k];
+    int topo;
+    if (std::fabs(c - m.max[k]) <= 1.0e-12) {
+      topo = m.nEls[k] - 1;
+    } else {
+      const double q = (c - m.min[k]) / m.dx[k], integer = std::trunc(q);
+      if (!(integer >= 0.0 && integer < (double)m.nEls[k] + 1.0)) return false;
+      topo = (int)integer;
+      if (topo > 0 && std::fabs(q - integer) <= 1.0e-12) topo--;
+      if (topo >= m.nEls[k]) return false;
+    }
+    double l = ((c - m.min[k]) - (double)topo * m.dx[k]) * m.two_over_dx[k] - 1.0;
+    l = l < -1.0 ? -1.0 : l > 1.0 ? 1.0 : l;
+    int s = -1;
+    for (int i = m.N; i >= 0; i--)
+      if (std::fabs(l - m.abcissa[i]) < 1.0e-8) s = i;
+    if (s < 0 || topo * m.N + s != t) return false;
+  }
+  return true;
+}
+}  // namespace
+
 // =========================================================== C-ABI ========
 extern "C" {
 
@@ -2179,6 +2211,7 @@ int se_mesh_create(const int nEls[2], int N, const double min[2], const double m
     d.max[k] = max[k];
     d.dx[k] = (d.max[k] - d.min[k]) / d.nEls[k];
     d.two_over_dx[k] = 2.0 / d.dx[k];
+    d.inv_dx[k] = 1.0 / d.dx[k];
     d.span[k] = d.max[k] - d.min[k];
     d.nspan[k] = d.min[k] - d.max[k];
   }
@@ -2188,6 +2221,7 @@ int se_mesh_create(const int nEls[2], int N, const double min[2], const double m
     d.w[i] = m->gll.w[i];
   }
   for (int i = 0; i < (N + 1) * (N + 1); i++) d.dC[i] = m->gll.dC[i];
+  d.snaps = vertices_snap(d, 0) && vertices_snap(d, 1);
   m->nVertsTotal = d.nVerts[0] * d.nVerts[1];
   *out = m;
   return SE_OK;
@@ -2716,12 +2750,18 @@ int se_advector_create(se_field* field, se_field* velocity, se_field* field_prev
     delete a;
     return rc;
   }
+  const size_t nv = (size_t)field->mesh->nVertsTotal, n1 = (size_t)field->mesh->dev.N + 1;
+  if (field_prev && nv * n1 * n1 >= kSlMixMin && dalloc(&a->mix, 4 * nv)) {
+    a->mix = nullptr;  // no room: the gathers form them
+    g_err.clear();
+  }
   *out = a;
   return SE_OK;
 }
 int se_advector_destroy(se_advector* adv) {
   if (!adv) return SE_OK;
   se_field_destroy(adv->sl);
+  dfree(adv->mix);
   dfree(adv->dep_el);
   dfree(adv->dep_xy);
   dfree(adv->err);
@@ -2736,7 +2776,7 @@ int se_advect(se_advector* adv, double dt) {
   if (adv->record) CK(cudaMemsetAsync(adv->err, 0, sizeof(unsigned), g_stream));
   CK(launch_sl(me->dev, adv->field->ndofs, adv->field->vals, adv->vel->vals,
                adv->field_prev ? adv->field_prev->vals : nullptr,
-               adv->vel_prev ? adv->vel_prev->vals : nullptr, dt, adv->sl->vals,
+               adv->vel_prev ? adv->vel_prev->vals : nullptr, adv->mix, dt, adv->sl->vals,
                adv->record ? adv->dep_el : nullptr, adv->record ? adv->dep_xy : nullptr,
                adv->err, g_stream));
   return SE_OK;

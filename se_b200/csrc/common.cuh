@@ -29,6 +29,8 @@ struct MeshDev {
   int periodic[2];
   double min[2], max[2], dx[2];
   double two_over_dx[2];  // 2.0/dx, rounded as the reference rounds it
+  double inv_dx[2];       // 1.0/dx
+  int snaps;  // every vertex's coordinates give back that vertex (element search and node snap)
   double span[2];         // max - min
   double nspan[2];        // min - max
   double abcissa[SE_MAXN1];
@@ -104,11 +106,18 @@ __device__ __forceinline__ void dd_fma(double& hi, double& lo, double a, double 
 
 // SL advection. field: [Nv][ndofs]; vel/vel_prev: [Nv][2]; out: [Nv][ndofs].
 // field_prev == nullptr selects the first-order scheme. dep_el/dep_xy are
-// optional recordings of the departure elements/points (all vertices).
+// optional recordings of the departure elements/points (all vertices). mix
+// (second order, nullable): work for the half-level velocities, 4 doubles a
+// vertex; without it they are formed at every gathered vertex.
 cudaError_t launch_sl(const MeshDev& m, int ndofs, const double* field, const double* vel,
-                      const double* field_prev, const double* vel_prev, double dt,
-                      double* out, int* dep_el, double* dep_xy, unsigned* err,
-                      cudaStream_t s);
+                      const double* field_prev, const double* vel_prev, double* mix, double dt,
+                      double* out, int* dep_el, double* dep_xy, unsigned* err, cudaStream_t s);
+// Gathered values of one interpolation over the mesh, nv (N+1)^2, from which
+// the second-order advection forms the half-level velocities once per vertex
+// (a launch more) instead of at every gathered one: at 37,249 vertices, p = 6
+// (1.8M) 16.0 us against 16.5, p = 3 (0.6M) 11.8 against 8.3; at 295,425
+// vertices, p = 6 54 against 65.
+constexpr size_t kSlMixMin = (size_t)2 << 20;
 // Mesh::GlobalToLocal at points (device arrays).
 cudaError_t launch_global_to_local(const MeshDev& m, const double* pts, int npts, int* el,
                                    double* lc, cudaStream_t s);

@@ -27,7 +27,7 @@ __device__ __forceinline__ double vertex_coord(const MeshDev& m, int d, int t) {
   int e = t / m.N;
   double l = m.abcissa[t - e * m.N];
   return xadd(xadd(m.min[d], xmul((double)e, m.dx[d])),
-              xmul(xdiv(xadd(l, 1.0), 2.0), m.dx[d]));
+              xmul(xmul(xadd(l, 1.0), 0.5), m.dx[d]));  // (l + 1) / 2: halving is exact
 }
 
 // Mesh::GetEl along one direction (src/base/Mesh.cpp:109-136). Out-of-mesh
@@ -57,6 +57,30 @@ __device__ __forceinline__ double local_coord(const MeshDev& m, int d, double c,
   return l;
 }
 
+// Element and local coordinate of c along d: get_topo and local_coord, bit
+// for bit, without their division away from element boundaries. (c - min) /
+// dx and the product q with the rounded reciprocal differ by at most a few
+// units in the last place, so where q is below 2^19 and further than 1e-9
+// from an integer both have the same integer part and the boundary
+// tolerances (1e-12) do not apply; the rest takes the division.
+__device__ __forceinline__ int locate(const MeshDev& m, int d, double c, double& l, unsigned* err) {
+  const double off = xsub(c, m.min[d]);
+  const double q = xmul(off, m.inv_dx[d]);
+  const double magic = 6755399441055744.0;  // 1.5 * 2^52: the sum's low bits are rint(q)
+  const double t = xadd(q, magic), r = xsub(t, magic);
+  const bool below = q < r;
+  int topo = __double2loint(t) - (below ? 1 : 0);
+  if (fabs(xsub(q, r)) > 1.0e-9 && q < 524288.0 && (unsigned)topo < (unsigned)m.nEls[d]) {
+    l = xsub(xmul(xsub(off, xmul(below ? xsub(r, 1.0) : r, m.dx[d])), m.two_over_dx[d]), 1.0);
+    if (l < -1.0) l = -1.0;
+    if (l > +1.0) l = +1.0;
+    return topo;
+  }
+  topo = get_topo(m, d, c, err);
+  l = local_coord(m, d, c, topo);
+  return topo;
+}
+
 // Legendre::IsRoot (src/base/Legendre.cpp:293-305): index of the first GLL
 // node within 1e-8, or -1.
 template <int N>
@@ -68,13 +92,20 @@ __device__ __forceinline__ int snap_node(const MeshDev& m, double l) {
   return s;
 }
 
-// GLL cardinal functions at a non-node coordinate: N_j(l) = lambda_j *
-// prod_{k != j} (l - x_k), from prefix and suffix products.
+// Whether any of the N+1 differences may be below 1e-8 in magnitude: their
+// upper words compared as integers (the 1e-8 test proper is snap_node's).
 template <int N>
-__device__ __forceinline__ void cardinal(const MeshDev& m, double l, double* c) {
-  double d[N + 1];
+__device__ __forceinline__ bool near_node(const double (&d)[N + 1]) {
+  unsigned mn = 0xffffffffu;
 #pragma unroll
-  for (int k = 0; k <= N; k++) d[k] = l - m.abcissa[k];
+  for (int k = 0; k <= N; k++) mn = min(mn, (unsigned)__double2hiint(d[k]) << 1);
+  return mn <= 2u * 0x3e45798eu;  // the upper word of 1e-8
+}
+
+// GLL cardinal functions at a non-node coordinate l, d[k] = l - x_k:
+// N_j(l) = lambda_j * prod_{k != j} d[k], from prefix and suffix products.
+template <int N>
+__device__ __forceinline__ void cardinal(const MeshDev& m, const double (&d)[N + 1], double* c) {
   double pre = 1.0;
 #pragma unroll
   for (int k = 0; k <= N; k++) {
@@ -195,30 +226,39 @@ template <int N, class Src>
 __device__ __forceinline__ typename Src::T interp(const MeshDev& m, const Src& src, double gx,
                                                   double gy, int* el_out, unsigned* err) {
   typedef typename Src::T T;
-  int tx = get_topo(m, 0, gx, err), ty = get_topo(m, 1, gy, err);
+  double lx, ly;
+  const int tx = locate(m, 0, gx, lx, err), ty = locate(m, 1, gy, ly, err);
   if (el_out) *el_out = ty * m.nEls[0] + tx;
-  double lx = local_coord(m, 0, gx, tx), ly = local_coord(m, 1, gy, ty);
-  int sx = snap_node<N>(m, lx), sy = snap_node<N>(m, ly);
   const int nvx = m.nVerts[0];
   const int base = ty * N * nvx + tx * N;
-  if (sx >= 0 && sy >= 0) return src(base + sy * nvx + sx);
+  double dx[N + 1], dy[N + 1];
+#pragma unroll
+  for (int k = 0; k <= N; k++) {
+    dx[k] = lx - m.abcissa[k];
+    dy[k] = ly - m.abcissa[k];
+  }
   double cx[N + 1], cy[N + 1];
   T acc = vzero(T());
-  if (sy >= 0) {
-    cardinal<N>(m, lx, cx);
-    T rv[N + 1];
-    src.template row<N>(base + sy * nvx, rv);
+  if (near_node<N>(dx) || near_node<N>(dy)) {
+    const int sx = snap_node<N>(m, lx), sy = snap_node<N>(m, ly);
+    if (sx >= 0 && sy >= 0) return src(base + sy * nvx + sx);
+    if (sy >= 0) {
+      cardinal<N>(m, dx, cx);
+      T rv[N + 1];
+      src.template row<N>(base + sy * nvx, rv);
 #pragma unroll
-    for (int i = 0; i <= N; i++) acc = vfma(cx[i], rv[i], acc);
-    return acc;
-  }
-  cardinal<N>(m, ly, cy);
-  if (sx >= 0) {
+      for (int i = 0; i <= N; i++) acc = vfma(cx[i], rv[i], acc);
+      return acc;
+    }
+    if (sx >= 0) {
+      cardinal<N>(m, dy, cy);
 #pragma unroll
-    for (int j = 0; j <= N; j++) acc = vfma(cy[j], src(base + j * nvx + sx), acc);
-    return acc;
+      for (int j = 0; j <= N; j++) acc = vfma(cy[j], src(base + j * nvx + sx), acc);
+      return acc;
+    }
   }
-  cardinal<N>(m, lx, cx);
+  cardinal<N>(m, dx, cx);
+  cardinal<N>(m, dy, cy);
 #pragma unroll
   for (int j = 0; j <= N; j++) {
     T rv[N + 1];
@@ -253,26 +293,48 @@ __device__ __forceinline__ void store_with_copies(const MeshDev& m, double* out,
   if (m.periodic[0] && m.periodic[1] && i == 0 && j == 0) store<T>(out, nvy * nvx - 1, v);
 }
 
+// ------------------------------------------------------------- advection --
+// What bounds the kernels: the L1 data path (81% busy at p = 8). Every thread
+// gathers (N+1)^2 values an interpolation, and 32 lanes of 16 bytes take at
+// least four cycles whatever they share. Measured (1.64M vertices, p = 8,
+// first order): 171 us, against 209 us with blocks of 8 x 32 vertices, a row
+// of eight vertices to a quarter warp, four divisions and node tests in FP64
+// an interpolation, and the first velocity interpolated at the vertex itself.
+// Sorting a block's points by element first gave 160 us there and nothing at
+// other orders; two points of one element to a thread 175 us.
+constexpr int kSlThreads = 128;  // 14 blocks an SM at 64x64 elements, p = 8: an even last wave
+constexpr int kSlX = 8, kSlY = kSlThreads / kSlX;
+
+// The thread's vertex: eight consecutive lanes (one pass of the L1 data path
+// for 16-byte loads) are a 4 x 2 block of vertices, which seldom falls into
+// more than two elements.
+__device__ __forceinline__ void sl_vertex(int& i, int& j) {
+  const int t = threadIdx.x;
+  i = blockIdx.x * kSlX + ((t & 3) | ((t >> 1) & 4));
+  j = blockIdx.y * kSlY + (((t >> 2) & 1) | ((t >> 3) & 2) | ((t >> 5) << 2));
+}
+
+__device__ __forceinline__ bool owned(const MeshDev& m, int i, int j) {
+  return i < m.nVerts[0] - m.periodic[0] && j < m.nVerts[1] - m.periodic[1];
+}
+
 // Advector::FirstOrder with IntegrateRK2 (src/base/Advector.cpp:136-148,181-201).
 template <int N, class FSrc>
-__global__ void __launch_bounds__(256, 2) sl_first_kernel(const MeshDev m, FSrc field,
-                                                       const double2* __restrict__ vel,
-                                                       double dt, double half_dt,
-                                                       double* __restrict__ out,
-                                                       int* __restrict__ dep_el,
-                                                       double2* __restrict__ dep_xy,
-                                                       unsigned* err) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  const int j = blockIdx.y * blockDim.y + threadIdx.y;
+__global__ void __launch_bounds__(kSlThreads, 4)
+    sl_first_kernel(const MeshDev m, FSrc field, const double2* __restrict__ vel, double dt,
+                    double half_dt, double* __restrict__ out, int* __restrict__ dep_el,
+                    double2* __restrict__ dep_xy, unsigned* err) {
+  int i, j;
+  sl_vertex(i, j);
   const int nvx = m.nVerts[0], nvy = m.nVerts[1];
-  const bool owner = i < nvx - m.periodic[0] && j < nvy - m.periodic[1];
+  const bool owner = owned(m, i, j);
   if (i >= nvx || j >= nvy || (!owner && !dep_el)) return;
-  Vec2 v{vel};
+  const Vec2 v{vel};
   // the tracer near this vertex, where most departure points land: its
   // lines start their way from HBM while the velocity is interpolated
   field.prefetch(j * nvx + i);
   const double ox = vertex_coord(m, 0, i), oy = vertex_coord(m, 1, j);
-  V2 u = interp<N>(m, v, ox, oy, nullptr, err);
+  V2 u = m.snaps ? v(j * nvx + i) : interp<N>(m, v, ox, oy, nullptr, err);
   double xh = wrap(m, 0, xsub(ox, xmul(half_dt, u.a)));
   double yh = wrap(m, 1, xsub(oy, xmul(half_dt, u.b)));
   u = interp<N>(m, v, xh, yh, nullptr, err);
@@ -287,29 +349,25 @@ __global__ void __launch_bounds__(256, 2) sl_first_kernel(const MeshDev m, FSrc 
   if (owner) store_with_copies(m, out, i, j, val);
 }
 
-// Advector::SecondOrder (src/base/Advector.cpp:203-246) with the
-// extrapolated velocities formed on the fly at each gathered vertex.
-template <int N, class FSrc>
-__global__ void __launch_bounds__(256, 2) sl_second_kernel(const MeshDev m, FSrc field,
-                                                        FSrc field_prev,
-                                                        const double2* __restrict__ vel,
-                                                        const double2* __restrict__ vel_prev,
-                                                        double dt, double half_dt,
-                                                        double* __restrict__ out,
-                                                        int* __restrict__ dep_el,
-                                                        double2* __restrict__ dep_xy,
-                                                        unsigned* err) {
-  const int i = blockIdx.x * blockDim.x + threadIdx.x;
-  const int j = blockIdx.y * blockDim.y + threadIdx.y;
+// Advector::SecondOrder (src/base/Advector.cpp:203-246). Half: the source of
+// the velocities extrapolated to the half levels, formed at every gathered
+// vertex (Vec2Mix) or once per vertex by mix_kernel (Vec2), the same bits.
+template <int N, class FSrc, class Half>
+__global__ void __launch_bounds__(kSlThreads, 4)
+    sl_second_kernel(const MeshDev m, FSrc field, FSrc field_prev,
+                     const double2* __restrict__ vel, const double2* __restrict__ vel_prev,
+                     const Half plus_half, const Half minus_half, double dt, double half_dt,
+                     double* __restrict__ out, int* __restrict__ dep_el,
+                     double2* __restrict__ dep_xy, unsigned* err) {
+  int i, j;
+  sl_vertex(i, j);
   const int nvx = m.nVerts[0], nvy = m.nVerts[1];
-  const bool owner = i < nvx - m.periodic[0] && j < nvy - m.periodic[1];
+  const bool owner = owned(m, i, j);
   if (i >= nvx || j >= nvy || (!owner && !dep_el)) return;
   const Vec2Mix plus_one{vel, vel_prev, 2.0, -1.0};
-  const Vec2Mix plus_half{vel, vel_prev, 1.5, -0.5};
-  const Vec2Mix minus_half{vel, vel_prev, 0.5, 0.5};
   const Vec2 v{vel};
   const double ox = vertex_coord(m, 0, i), oy = vertex_coord(m, 1, j);
-  V2 u = interp<N>(m, plus_one, ox, oy, nullptr, err);
+  V2 u = m.snaps ? plus_one(j * nvx + i) : interp<N>(m, plus_one, ox, oy, nullptr, err);
   double xh = wrap(m, 0, xsub(ox, xmul(half_dt, u.a)));
   double yh = wrap(m, 1, xsub(oy, xmul(half_dt, u.b)));
   u = interp<N>(m, plus_half, xh, yh, nullptr, err);
@@ -346,38 +404,56 @@ __global__ void __launch_bounds__(256, 2) sl_second_kernel(const MeshDev m, FSrc
   }
 }
 
-template <int N>
-cudaError_t launch_sl_n(const MeshDev& m, int ndofs, const double* field, const double* vel,
-                        const double* field_prev, const double* vel_prev, double dt, double* out,
-                        int* dep_el, double* dep_xy, unsigned* err, cudaStream_t s) {
-  // a warp covers 8 x 4 vertices, about one element: its departure points
-  // fall in fewer element blocks than a row of 32 vertices' do
-  dim3 block(8, 32);
-  dim3 grid((m.nVerts[0] + 7) / 8, (m.nVerts[1] + 31) / 32);
+// The velocities at t + dt/2 and t - dt/2 (Advector::ExtrapolateVelocities) at
+// every vertex, plus[0, nv) and plus[nv, 2 nv).
+__global__ void __launch_bounds__(256) mix_kernel(int nv, const Vec2Mix plus, const Vec2Mix minus,
+                                                  double2* __restrict__ out) {
+  const int k = blockIdx.x * 256 + threadIdx.x;
+  if (k >= nv) return;
+  const V2 p = plus(k), q = minus(k);
+  out[k] = make_double2(p.a, p.b);
+  out[nv + k] = make_double2(q.a, q.b);
+}
+
+template <int N, class FSrc>
+cudaError_t launch_sl_t(const MeshDev& m, const FSrc field, const FSrc field_prev, bool second,
+                        const double* vel, const double* vel_prev, double* mix, double dt,
+                        double* out, int* dep_el, double* dep_xy, unsigned* err, cudaStream_t s) {
   const double half_dt = 0.5 * dt;
   const double2* v = reinterpret_cast<const double2*>(vel);
   const double2* vm = reinterpret_cast<const double2*>(vel_prev);
   double2* dxy = reinterpret_cast<double2*>(dep_xy);
-  if (!field_prev) {
-    if (ndofs == 1)
-      sl_first_kernel<N, Scalar><<<grid, block, 0, s>>>(m, Scalar{field}, v, dt, half_dt, out,
-                                                         dep_el, dxy, err);
-    else
-      sl_first_kernel<N, Vec2><<<grid, block, 0, s>>>(
-          m, Vec2{reinterpret_cast<const double2*>(field)}, v, dt, half_dt, out, dep_el, dxy,
-          err);
+  const dim3 grid((m.nVerts[0] + kSlX - 1) / kSlX, (m.nVerts[1] + kSlY - 1) / kSlY);
+  if (!second) {
+    sl_first_kernel<N, FSrc><<<grid, kSlThreads, 0, s>>>(m, field, v, dt, half_dt, out, dep_el,
+                                                         dxy, err);
+    return cudaGetLastError();
+  }
+  const Vec2Mix plus{v, vm, 1.5, -0.5}, minus{v, vm, 0.5, 0.5};
+  if (mix) {
+    const int nv = m.nVerts[0] * m.nVerts[1];
+    double2* x = reinterpret_cast<double2*>(mix);
+    mix_kernel<<<(nv + 255) / 256, 256, 0, s>>>(nv, plus, minus, x);
+    sl_second_kernel<N, FSrc, Vec2><<<grid, kSlThreads, 0, s>>>(
+        m, field, field_prev, v, vm, Vec2{x}, Vec2{x + nv}, dt, half_dt, out, dep_el, dxy, err);
   } else {
-    if (ndofs == 1)
-      sl_second_kernel<N, Scalar><<<grid, block, 0, s>>>(m, Scalar{field}, Scalar{field_prev},
-                                                          v, vm, dt, half_dt, out, dep_el, dxy,
-                                                          err);
-    else
-      sl_second_kernel<N, Vec2><<<grid, block, 0, s>>>(
-          m, Vec2{reinterpret_cast<const double2*>(field)},
-          Vec2{reinterpret_cast<const double2*>(field_prev)}, v, vm, dt, half_dt, out, dep_el,
-          dxy, err);
+    sl_second_kernel<N, FSrc, Vec2Mix><<<grid, kSlThreads, 0, s>>>(
+        m, field, field_prev, v, vm, plus, minus, dt, half_dt, out, dep_el, dxy, err);
   }
   return cudaGetLastError();
+}
+
+template <int N>
+cudaError_t launch_sl_n(const MeshDev& m, int ndofs, const double* field, const double* vel,
+                        const double* field_prev, const double* vel_prev, double* mix, double dt,
+                        double* out, int* dep_el, double* dep_xy, unsigned* err, cudaStream_t s) {
+  const bool second = field_prev != nullptr;
+  if (ndofs == 1)
+    return launch_sl_t<N>(m, Scalar{field}, Scalar{field_prev}, second, vel, vel_prev, mix, dt,
+                          out, dep_el, dep_xy, err, s);
+  return launch_sl_t<N>(m, Vec2{reinterpret_cast<const double2*>(field)},
+                        Vec2{reinterpret_cast<const double2*>(field_prev)}, second, vel, vel_prev,
+                        mix, dt, out, dep_el, dep_xy, err, s);
 }
 
 // ------------------------------------------------ point queries (tests) ----
@@ -796,11 +872,11 @@ __global__ void qg_solve_q_kernel(const MeshDev m, Dir dxd, Dir dyd, int G0, dou
   }
 
 cudaError_t launch_sl(const MeshDev& m, int ndofs, const double* field, const double* vel,
-                      const double* field_prev, const double* vel_prev, double dt, double* out,
-                      int* dep_el, double* dep_xy, unsigned* err, cudaStream_t s) {
+                      const double* field_prev, const double* vel_prev, double* mix, double dt,
+                      double* out, int* dep_el, double* dep_xy, unsigned* err, cudaStream_t s) {
   if (m.N < 3) return cudaErrorInvalidValue;
-  SE_DISPATCH_N(m.N, return launch_sl_n<NN>(m, ndofs, field, vel, field_prev, vel_prev, dt, out,
-                                            dep_el, dep_xy, err, s));
+  SE_DISPATCH_N(m.N, return launch_sl_n<NN>(m, ndofs, field, vel, field_prev, vel_prev, mix, dt,
+                                            out, dep_el, dep_xy, err, s));
 }
 
 cudaError_t launch_ns_pressure(const MeshDev& m, int kind, const double* a, const double* p,
