@@ -614,10 +614,8 @@ def read_peaks():
 def apply_kernel_name(p, name):
     """The kernel the library's apply dispatches to for order p."""
     if name != "fp64":
-        return f"apply_tile_kernel<{p}, bf16 -> float>"
-    if 4 <= p <= 8:
-        return f"apply_ef_kernel<{p}> (element-factored FP64 FMA, cp.async staging)"
-    return f"apply_mma_kernel<{p}> (FP64 DMMA element products, TMA-staged tiles)"
+        return f"apply_el_kernel<{p}, bf16, float> (element-factored FP32 FMA)"
+    return f"apply_el_kernel<{p}, double> (element-factored FP64 FMA, cp.async staging)"
 
 
 def run_apply_roofline(ne=768, p=8, reps=20, precisions=("fp64", "bf16_in_fp32_out")):

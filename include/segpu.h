@@ -297,11 +297,8 @@ int se_linsys_solve_batch(se_linsys** systems, int n, int remove_null_space,
  * fills stats (nullable) and returns what se_linsys_solve would have. */
 int se_linsys_solve_async(se_linsys* ls, int remove_null_space);
 int se_linsys_solve_finish(se_linsys* ls, se_solve_stats* stats);
-/* y = A x on vector unknowns (device pointers, vec_size entries each), on
- * the calling thread's stream. Orders 4 to 8 return once the apply is
- * queued; orders 2, 3 and 9 to 12 (a TMA-staged kernel with bounded waits)
- * return after it has finished, with SE_ERR_TIMEOUT if a stage never
- * arrived. */
+/* y = A x on vector unknowns (device pointers, vec_size entries each, not
+ * aliased), queued on the calling thread's stream. */
 int se_linsys_apply(se_linsys* ls, const double* x_dev, double* y_dev);
 /* No counterpart in the reference: x = A^{-1} r by the fast-diagonalization
  * transforms in FP64 (four tensor-core products; exact up to rounding, the

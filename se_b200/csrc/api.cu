@@ -3169,19 +3169,7 @@ int se_linsys_solve_finish(se_linsys* ls, se_solve_stats* stats) {
 }
 int se_linsys_apply(se_linsys* ls, const double* x_dev, double* y_dev) {
   if (!ls || !x_dev || !y_dev) return fail(SE_ERR_ARG, "null argument");
-  // orders 4 to 8 (and SVV systems) run kernels without barrier waits;
-  // the TMA-staged kernel of the other orders reports a barrier that timed
-  // out in the error word, read back here
-  const int N = ls->op.d[0].N;
-  const bool waits = ls->op.gamma == 0.0 && (N < 4 || N > 8);
-  if (waits) CK(cudaMemsetAsync(ls->d_err, 0, sizeof(unsigned), g_stream));
-  CK(launch_op_apply(ls->op, x_dev, y_dev, ls->d_err, g_stream));
-  if (waits) {
-    unsigned err = 0;
-    CK(cudaMemcpyAsync(&err, ls->d_err, sizeof(unsigned), cudaMemcpyDeviceToHost, g_stream));
-    CK(cudaStreamSynchronize(g_stream));
-    if (err & KERR_BARRIER_TIMEOUT) return fail(SE_ERR_TIMEOUT, "apply: a TMA stage never arrived");
-  }
+  CK(launch_op_apply(ls->op, x_dev, y_dev, g_stream));
   return SE_OK;
 }
 int se_linsys_fdm_apply(se_linsys* ls, const double* r_dev, double* x_dev) {

@@ -45,6 +45,7 @@
 #include <vector>
 
 #include "common.cuh"
+#include "kh.cuh"
 
 namespace seg {
 namespace {
@@ -56,25 +57,13 @@ constexpr int kPatchRegs = 4;  // nodes per thread whose whole state stays in re
 constexpr int kLine = kPatchLine;
 constexpr int kPatchPolls = 1 << 22;
 
-// Even/odd halves of the element stiffness Kh (centrosymmetric: Kh[a][b] =
-// Kh[N-a][N-b]): with e_b = v_b + v_{N-b} and d_b = v_b - v_{N-b},
-// (Kh v)_a = sum Ce[a][b] e_b + sum Co[a][b] d_b and (Kh v)_{N-a} = the
-// difference of the two sums.
-template <int N>
-struct Eo {
-  static constexpr int H = (N + 1) / 2;   // node pairs
-  static constexpr int M = (N + 1) & 1;   // 1: a middle node
-  static constexpr int E = H + M;
-  static constexpr int NC = E * E + H * H;  // coefficients
-};
-
 template <int N>
 struct PatchArgs {
   PatchSolve one;            // the solve of a single-solve launch
   const PatchSolve* solves;  // a batch's solves (nullptr: one)
   const int* cta_solve;      // solve of each block (batch)
   PatchResult* res;
-  double cf[Eo<N>::NC];  // Ce [E][E], then Co [H][H]
+  double cf[Eo<N>::NC];  // even/odd halves of Kh (kh.cuh)
   double w[N + 1], kd[N + 1];  // GLL weights, stiffness diagonal
 };
 
@@ -154,45 +143,6 @@ __device__ __forceinline__ void assembled(const Dir& d, const double* w, const d
     ws += w[N];
     ks += kd[N];
   }
-}
-
-// o = Kh v by even/odd halves (coefficients from the parameter bank); returns
-// v . o.
-template <int N>
-__device__ __forceinline__ double kh_product(const PatchArgs<N>& A, const double (&v)[N + 1],
-                                             double (&o)[N + 1]) {
-  constexpr int H = Eo<N>::H, E = Eo<N>::E;
-  double e[E], d[H];
-#pragma unroll
-  for (int b = 0; b < H; b++) {
-    e[b] = v[b] + v[N - b];
-    d[b] = v[b] - v[N - b];
-  }
-  if constexpr (Eo<N>::M == 1) e[H] = v[H];
-  double s[E];
-#pragma unroll
-  for (int a = 0; a < E; a++) {
-    s[a] = 0.0;
-#pragma unroll
-    for (int b = 0; b < E; b++) s[a] = fma(A.cf[a * E + b], e[b], s[a]);
-  }
-  double en = 0.0, od = 0.0;
-#pragma unroll
-  for (int a = 0; a < H; a++) {
-    double t = 0.0;
-#pragma unroll
-    for (int b = 0; b < H; b++) t = fma(A.cf[E * E + a * H + b], d[b], t);
-    o[a] = s[a] + t;
-    o[N - a] = s[a] - t;
-    // v_a o_a + v_{N-a} o_{N-a} = s e_a + t d_a
-    en = fma(s[a], e[a], en);
-    od = fma(t, d[a], od);
-  }
-  if constexpr (Eo<N>::M == 1) {
-    o[H] = s[H];
-    en = fma(s[H], e[H], en);
-  }
-  return en + od;
 }
 
 template <int NV>
@@ -561,7 +511,7 @@ __global__ void __launch_bounds__(kPT, 1) cg_patch_kernel(const __grid_constant_
         double v[N + 1], o[N + 1];
 #pragma unroll
         for (int k = 0; k <= N; k++) v[k] = u[k];
-        const double en = kh_product<N>(A, v, o);
+        const double en = eo_product<N, true>(A.cf, v, o);
         acc[0] = fma(ex_row[j], en, acc[0]);
         if (e == 0 && edge_out[0]) put(edge_out[0] + j, o[0], seq);
         if (e == nex - 1 && edge_out[1]) put(edge_out[1] + j, o[N], seq);
@@ -575,7 +525,7 @@ __global__ void __launch_bounds__(kPT, 1) cg_patch_kernel(const __grid_constant_
         double v[N + 1], o[N + 1];
 #pragma unroll
         for (int k = 0; k <= N; k++) v[k] = u[k * pitch];
-        const double en = kh_product<N>(A, v, o);
+        const double en = eo_product<N, true>(A.cf, v, o);
         acc[0] = fma(ey_col[i], en, acc[0]);
         if (e == 0 && edge_out[2]) put(edge_out[2] + i, o[0], seq);
         if (e == ney - 1 && edge_out[3]) put(edge_out[3] + i, o[N], seq);
@@ -716,21 +666,14 @@ size_t patch_smem(int N, int nex, int ney, bool regs) {
 
 template <int N>
 cudaError_t launch_n(const PatchLaunch& L, cudaStream_t s) {
-  constexpr int H = Eo<N>::H, E = Eo<N>::E, n = N + 1;
+  constexpr int n = N + 1;
   PatchArgs<N> A;
   std::memset(&A, 0, sizeof(A));
   if (L.one) A.one = *L.one;
   A.solves = L.solves;
   A.cta_solve = L.cta_solve;
   A.res = L.res;
-  auto sym = [&](int a, int b) {  // the two mirrored entries averaged
-    return 0.5L * ((long double)L.Kh[a * n + b] + (long double)L.Kh[(N - a) * n + (N - b)]);
-  };
-  for (int a = 0; a < E; a++)
-    for (int b = 0; b < E; b++)
-      A.cf[a * E + b] = (double)(b < H ? 0.5L * (sym(a, b) + sym(a, N - b)) : sym(a, b));
-  for (int a = 0; a < H; a++)
-    for (int b = 0; b < H; b++) A.cf[E * E + a * H + b] = (double)(0.5L * (sym(a, b) - sym(a, N - b)));
+  eo_coefs<N>(L.Kh, 1.0, A.cf);
   for (int a = 0; a < n; a++) {
     A.w[a] = L.w[a];
     A.kd[a] = L.Kh[a * n + a];

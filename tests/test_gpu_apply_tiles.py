@@ -1,0 +1,105 @@
+"""The operator apply at the edges of its tiles, every order, against the
+tensor-product operator assembled from the mesh's own GLL tables in FP64.
+
+Meshes of one tile, one element more or less than whole tiles, several tiles
+with interior ones, and sizes on both sides of every staging rule: rows of an
+odd, even and multiple-of-four number of unknowns, first columns at every
+offset from an 8-byte boundary, tiles that end the array, x off alignment.
+
+Tolerances: the sums run over at most 4N + 8 products, so FP64 results are
+within 64 rounding errors (64 * 2^-53, about 7e-15) of the row's sum of
+magnitudes, FP32 arithmetic within 64 * 2^-24 (about 4e-6).
+"""
+import numpy as np
+import pytest
+
+pytestmark = pytest.mark.gpu
+
+P, CH, BOX = (True, True), (True, False), (False, False)
+WALLS = {P: (False,) * 4, CH: (True, True, False, False), BOX: (True,) * 4, "nat": (False,) * 4}
+
+
+def dense_1d(ne, N, w, Kh, periodic, lo, hi):
+    nv = ne * N + 1
+    K, W = np.zeros((nv, nv)), np.zeros(nv)
+    for e in range(ne):
+        s = slice(e * N, e * N + N + 1)
+        K[s, s] += Kh
+        W[s] += w
+    if periodic:
+        K[0] += K[-1]
+        K[:, 0] += K[:, -1]
+        W[0] += W[-1]
+    return K[lo:hi, lo:hi], W[lo:hi]
+
+
+def system(S, nx, ny, N, per, walls):
+    m = S.Mesh("m", [nx, ny], "legendre", N, [0.0, 0.0], [1.0, 0.7], list(per))
+    b = S.BCs(*walls, m)
+    u = S.Field("u", m, 1, b)
+    ls = S.HelmholtzEqn(u, None, -3.0, -1.0, 0.5, 0, S.solver_opts(mode=S.MODE_EXACT))
+    x, w, D = m.gll()
+    Kh = D.T @ np.diag(w) @ D
+    bot, top, left, right = walls
+    X = (int(left), nx * N + (0 if per[0] or right else 1))
+    Y = (int(bot), ny * N + (0 if per[1] or top else 1))
+    Kx, Wx = dense_1d(nx, N, w, Kh, per[0], *X)
+    Ky, Wy = dense_1d(ny, N, w, Kh, per[1], *Y)
+    hx, hy = 1.0 / nx, 0.7 / ny
+    al, bx, by = -3.0 * hx * hy / 4, -0.5 * hy / hx, -0.5 * hx / hy
+
+    def apply(v, mag=False):
+        f = np.abs if mag else (lambda z: z)
+        v = f(v.reshape(len(Wy), len(Wx)))
+        return (f(al) * Wy[:, None] * Wx * v + f(bx) * Wy[:, None] * (v @ f(Kx).T)
+                + f(by) * Wx * (f(Ky) @ v)).ravel()
+
+    return (m, b, u), ls, apply, len(Wx) * len(Wy)
+
+
+def sizes(N):
+    ex = 64 // N  # elements of a tile row; a tile has four element rows
+    return [(2, 2), (ex, 4), (ex + 1, 5), (max(2, ex - 1), 3), (3 * ex, 12), (3 * ex + 2, 13)]
+
+
+KINDS = [(P, WALLS[P]), (CH, WALLS[CH]), (BOX, WALLS[BOX]), (BOX, WALLS["nat"]),
+         (BOX, (False, True, True, False))]
+
+
+@pytest.mark.parametrize("N", range(2, 13))
+@pytest.mark.parametrize("kind", range(len(KINDS)))
+def test_fp64(segpu, N, kind):
+    import torch
+    for nx, ny in sizes(N):
+        keep, ls, apply, n = system(segpu, nx, ny, N, *KINDS[kind])
+        assert ls.vecSize == n
+        x = np.random.default_rng(nx * 100 + ny).standard_normal(n)
+        xd = torch.tensor(np.concatenate([[0.0], x]), device="cuda")
+        y = torch.full((n + 2,), 7.0, device="cuda", dtype=torch.float64)
+        ls.apply(xd.data_ptr() + 8, y.data_ptr() + 8)
+        torch.cuda.synchronize()
+        got = y.cpu().numpy()
+        assert got[0] == 7.0 and got[-1] == 7.0
+        assert (np.abs(got[1:-1] - apply(x)) <= 64 * 2.0 ** -53 * apply(x, True)).all(), (nx, ny)
+
+
+@pytest.mark.parametrize("N", range(2, 13))
+@pytest.mark.parametrize("kind", range(len(KINDS)))
+@pytest.mark.parametrize("half", [False, True])
+def test_reduced_precision(segpu, N, kind, half):
+    import torch
+    dt = torch.float16 if half else torch.bfloat16
+    for k, (nx, ny) in enumerate(sizes(N) + [(3 * (64 // N) + 1, 12), (3 * (64 // N) + 3, 12)]):
+        keep, ls, apply, n = system(segpu, nx, ny, N, *KINDS[kind])
+        x = torch.tensor(np.random.default_rng(nx * 100 + ny).standard_normal(n)).to(dt)
+        off = k % 5  # 2-byte steps off alignment
+        xd = torch.zeros(n + 8, device="cuda", dtype=dt)
+        xd[off:off + n] = x.cuda()
+        y = torch.full((n + 2,), 7.0, device="cuda", dtype=torch.float32)
+        ls.apply_low(xd.data_ptr() + 2 * off, y.data_ptr() + 4,
+                     segpu.PREC_FP16 if half else segpu.PREC_BF16)
+        torch.cuda.synchronize()
+        got = y.cpu().numpy().astype(np.float64)
+        assert got[0] == 7.0 and got[-1] == 7.0
+        xr = x.double().numpy()
+        assert (np.abs(got[1:-1] - apply(xr)) <= 64 * 2.0 ** -24 * apply(xr, True)).all(), (nx, ny)
