@@ -308,7 +308,7 @@ def run_gpu(args, rank, world):
             torch.cuda.synchronize()
             sl_ms.append(e0.elapsed_time(e1))
         log("FDM inverse timing")
-        # the dense FDM transform (four fdm_dgemm_kernel launches) on a mesh
+        # the dense FDM inverse (folded directions, four products) on a mesh
         # whose element count is not a power of two (63 x 64 elements, p = 8:
         # 504 x 512 unknowns), the path of walled and general meshes, CUDA
         # events on the library's stream, L2 flushed before each call
@@ -490,28 +490,29 @@ SL_FLOPS_PER_VERTEX = (2 * 9 * 5 + 2 * 81 * 2 + 2 * 9 * 2) + (2 * 9 * 5 + 2 * 81
 SL_TRAFFIC_BYTES = 6.358016e6
 # DRAM traffic of one fdm_dgemm_kernel launch (M = N = K = 512), from one ncu
 # capture of that kernel on this workload (cold caches: read 4.21 MB, write 0).
-FDM_GEMM_TRAFFIC_BYTES = 4.211968e6
 
 
 def dense_fdm_roofline(r):
-    """The dense FDM product kernel (fdm_dgemm_kernel, four launches per
-    inverse; the path of meshes whose element counts are not powers of two
-    and of walled directions), timed live as one inverse of a 63 x 64
-    element, p = 8 system (504 x 512 unknowns): achieved = the four
-    products' algorithmic FLOPs (2 M N K each) / the inverse's time, against
-    the FP64 DGEMM rate measured in the same run (MEASURED_PEAKS.json holds
-    no FP64 figure). DRAM traffic per launch from one ncu capture of the
-    512^3 product."""
+    """The dense FDM inverse (the path of meshes whose element counts are not
+    powers of two and of walled directions), timed live on a 63 x 64 element,
+    p = 8 system (504 x 512 unknowns): a fold, four fdm_dgemm_ksplit_kernel
+    launches on the even and odd halves of both directions, an unfold.
+    Achieved = the four products' algorithmic FLOPs on the halves / the whole
+    inverse's time, against the FP64 DGEMM rate measured in the same run
+    (MEASURED_PEAKS.json holds no FP64 figure)."""
     gx, gy = r["dense_gx"], r["dense_gy"]
-    flops = 2 * (2.0 * gy * gx * gx) + 2 * (2.0 * gy * gx * gy)
+
+    def halves(g):  # a periodic direction: g/2 + 1 even modes, the rest odd
+        return (g // 2 + 1) ** 2 + (g - g // 2 - 1) ** 2
+
+    flops = 2 * (2.0 * gy * halves(gx)) + 2 * (2.0 * gx * halves(gy))
     t = r["dense_fdm_ms"] * 1e-3
     achieved = flops / t / 1e12
-    return {"kernel": "fdm_dgemm_kernel (FP64 DMMA, 32x32 tiles), 4 launches, 504x512 unknowns",
+    return {"kernel": "fold, 4 x fdm_dgemm_ksplit_kernel (FP64 DMMA, 32-row tiles), unfold, 504x512 unknowns",
             "bound": "tensor", "achieved": achieved, "peak": r["fp64_tflops"], "unit": "TFLOP/s",
             "frac": achieved / r["fp64_tflops"],
             "peak_source": "FP64 DGEMM (torch.matmul float64 8192^3) measured in this run",
-            "inverse_ms": r["dense_fdm_ms"], "launch_ms": r["dense_fdm_ms"] / 4,
-            "algorithmic_flops_per_inverse": flops, "traffic": FDM_GEMM_TRAFFIC_BYTES}
+            "inverse_ms": r["dense_fdm_ms"], "algorithmic_flops_per_inverse": flops}
 
 
 def bloch_roofline(r):

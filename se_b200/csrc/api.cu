@@ -238,6 +238,9 @@ struct se_advector {
   unsigned* err;  // device error bits of this advector's SL kernels
   bool record;
 };
+namespace {
+struct Eig1D;
+}
 struct se_linsys {
   se_field *sol, *rhs;
   bool poisson;
@@ -276,8 +279,8 @@ struct se_linsys {
   void *Sx_lo, *Sy_lo, *SxT_lo, *SyT_lo;  // low-precision copies (cached, shared)
   int fdm_lbuf_prec;          // precision the L2, L3 buffers were sized for
   double *X1, *X2, *ax;       // FP64 work: two transform buffers, A x
-  double* zlow;               // FP64 inverse: the low spectral block [lowk][lowk]
-  int lowk;
+  double* zlow;               // FP64 inverse: the low modes' block [kFdmLow][kFdmLow]
+  const Eig1D *eigx, *eigy;   // FP64 inverse: the directions' folded blocks (cached, shared)
   // FP64 inverse of a doubly periodic system with 2^k elements per
   // direction: Bloch form (bloch.cu) with its complex spectral work array
   bool bloch;
@@ -1057,15 +1060,13 @@ int refine_eig(int n, const std::vector<double>& K, const std::vector<double>& W
   return SE_OK;
 }
 
-// Generalised eigenvectors S (S^T K S = diag(lam), S^T W S = I) of one
-// direction, on the device: eigenvectors of W^-1/2 K W^-1/2 by cuSOLVER
+// Generalised eigenvectors E (E^T K E = diag(lam), E^T W E = I; column-major)
+// of one symmetric pair of size n: eigenvectors of W^-1/2 K W^-1/2 by cuSOLVER
 // syevd (setup only), scaled by W^-1/2, then refined (refine_eig).
-int eig_1d(const Dir& d, const double* Kh, const double* w, double** S_dev, double** ST_dev,
-           double** lam_dev, std::vector<double>& S_host) {
-  std::vector<double> K, W;
-  assemble_1d(d, Kh, w, K, W);
-  const int n = d.hi - d.lo;
-  std::vector<double> A((size_t)n * n);
+int eig_pair(int n, const std::vector<double>& K, const std::vector<double>& W,
+             std::vector<double>& A, std::vector<double>& lam) {
+  A.resize((size_t)n * n);
+  lam.resize(n);
   for (int i = 0; i < n; i++)
     for (int j = 0; j < n; j++) A[(size_t)j * n + i] = K[(size_t)i * n + j] / std::sqrt(W[i] * W[j]);
   double *dA = nullptr, *dlam = nullptr, *work = nullptr;
@@ -1088,45 +1089,118 @@ int eig_1d(const Dir& d, const double* Kh, const double* w, double** S_dev, doub
                               work, lwork, info) == CUSOLVER_STATUS_SUCCESS;
   ok = ok && cudaMemcpy(&hinfo, info, sizeof(int), cudaMemcpyDeviceToHost) == cudaSuccess && hinfo == 0;
   ok = ok && cudaMemcpy(A.data(), dA, sizeof(double) * A.size(), cudaMemcpyDeviceToHost) == cudaSuccess;
+  ok = ok && cudaMemcpy(lam.data(), dlam, sizeof(double) * n, cudaMemcpyDeviceToHost) == cudaSuccess;
   if (h) cusolverDnDestroy(h);
   dfree(work);
   dfree(info);
-  if (!ok) {
-    dfree(dA);
-    dfree(dlam);
-    return fail(SE_ERR_CUDA, "eigendecomposition of the 1-D operator failed (n=%d)", n);
-  }
+  dfree(dA);
+  dfree(dlam);
+  if (!ok) return fail(SE_ERR_CUDA, "eigendecomposition of the 1-D operator failed (n=%d)", n);
   for (int j = 0; j < n; j++)
     for (int i = 0; i < n; i++) A[(size_t)j * n + i] /= std::sqrt(W[i]);
-  {
-    std::vector<double> lam(n);
-    if (cudaMemcpy(lam.data(), dlam, sizeof(double) * n, cudaMemcpyDeviceToHost) != cudaSuccess) {
-      dfree(dA);
-      dfree(dlam);
-      return fail(SE_ERR_CUDA, "eigenvalue download failed (n=%d)", n);
+  return refine_eig(n, K, W, A, lam);
+}
+
+// A direction is its own mirror image when it is periodic or both its ends
+// are of one kind: all elements are equal and the GLL nodes symmetric.
+FoldDir fold_of(const Dir& d) {
+  FoldDir f;
+  f.n = d.hi - d.lo;
+  f.periodic = d.periodic != 0;
+  f.on = f.n > 1 && (d.periodic || d.lo == d.nV - d.hi);
+  f.ge = !f.on ? f.n : f.periodic ? f.n / 2 + 1 : (f.n + 1) / 2;
+  f.go = f.n - f.ge;
+  f.os = (f.ge + 1) & ~1;
+  f.len = f.os + ((f.go + 1) & ~1);
+  return f;
+}
+int fold_mirror(const FoldDir& f, int i) {
+  return f.periodic ? (i == 0 ? 0 : f.n - i) : f.n - 1 - i;
+}
+
+// The eigenpairs of one direction: full eigenvectors E (column-major,
+// ascending eigenvalues lam) and, folded (FoldDir), the even then the odd
+// modes' blocks on the half direction, FE row-major (entry (i, m)), FT their
+// transposes (rows at the pitch FoldDir gives), lamF their eigenvalues by slot. A folded block is the pair's own
+// eigenproblem on the sums (differences) of mirrored unknowns: K and W summed
+// over the mirrored entries (with the odd part's signs), which has no
+// degenerate pairs (a periodic direction's sine and cosine modes fall into
+// different blocks) and an eighth of the work each.
+int eig_1d(const Dir& d, const double* Kh, const double* w, std::vector<double>& E,
+           std::vector<double>& lam, std::vector<double>& FE, std::vector<double>& FT,
+           std::vector<double>& lamF) {
+  std::vector<double> K, W;
+  assemble_1d(d, Kh, w, K, W);
+  const FoldDir f = fold_of(d);
+  const int n = f.n;
+  FE.clear();
+  FT.clear();
+  lamF.clear();
+  auto append = [&](int m, const std::vector<double>& A, const std::vector<double>& l) {
+    for (int i = 0; i < m; i++) {
+      for (int j = 0; j < m; j++) FE.push_back(A[(size_t)j * m + i]);
+      FT.insert(FT.end(), A.begin() + (size_t)i * m, A.begin() + (size_t)(i + 1) * m);
+      if (m & 1) {
+        FE.push_back(0.0);
+        FT.push_back(0.0);
+      }
     }
-    if (int rc2 = refine_eig(n, K, W, A, lam)) {
-      dfree(dA);
-      dfree(dlam);
-      return rc2;
+    lamF.insert(lamF.end(), l.begin(), l.end());
+    if (m & 1) lamF.push_back(1.0);  // an empty slot
+  };
+  if (!f.on) {
+    if (int rc = eig_pair(n, K, W, E, lam)) return rc;
+    append(n, E, lam);
+    return SE_OK;
+  }
+  std::vector<std::pair<double, int>> order;  // eigenvalue, mode (even then odd)
+  std::vector<double> full((size_t)n * n, 0.0);
+  for (int part = 0; part < 2; part++) {
+    const int first = part && f.periodic ? 1 : 0, m = part ? n - f.ge : f.ge;
+    if (m == 0) continue;
+    const double sg = part ? -1.0 : 1.0;
+    std::vector<double> Kp((size_t)m * m), Wp(m), A, l;
+    for (int a = 0; a < m; a++) {
+      const int i = a + first, im = fold_mirror(f, i);
+      Wp[a] = im != i ? W[i] + W[im] : W[i];
+      for (int b = 0; b < m; b++) {
+        const int j = b + first, jm = fold_mirror(f, j);
+        double v = K[(size_t)i * n + j];
+        if (jm != j) v += sg * K[(size_t)i * n + jm];
+        if (im != i) {
+          double u = K[(size_t)im * n + j];
+          if (jm != j) u += sg * K[(size_t)im * n + jm];
+          v += sg * u;
+        }
+        Kp[(size_t)a * m + b] = v;
+      }
     }
-    CK(upload_now(dlam, lam.data(), sizeof(double) * n));
+    for (int a = 0; a < m; a++)
+      for (int b = 0; b < a; b++) {  // symmetric to the last bit
+        const double v = 0.5 * (Kp[(size_t)a * m + b] + Kp[(size_t)b * m + a]);
+        Kp[(size_t)a * m + b] = Kp[(size_t)b * m + a] = v;
+      }
+    if (int rc = eig_pair(m, Kp, Wp, A, l)) return rc;
+    append(m, A, l);
+    for (int k = 0; k < m; k++) {
+      const int mode = (part ? f.ge : 0) + k;
+      order.push_back({l[k], mode});
+      for (int a = 0; a < m; a++) {
+        const int i = a + first, im = fold_mirror(f, i);
+        full[(size_t)mode * n + i] = A[(size_t)k * m + a];
+        if (im != i) full[(size_t)mode * n + im] = sg * A[(size_t)k * m + a];
+      }
+    }
   }
-  S_host = A;
-  CK(upload_now(dA, A.data(), sizeof(double) * A.size()));
-  std::vector<double> T((size_t)n * n);
-  for (int j = 0; j < n; j++)
-    for (int i = 0; i < n; i++) T[(size_t)i * n + j] = A[(size_t)j * n + i];
-  double* dT = nullptr;
-  if (int rc2 = dalloc(&dT, (size_t)n * n)) {
-    dfree(dA);
-    dfree(dlam);
-    return rc2;
+  std::stable_sort(order.begin(), order.end(),
+                   [](const auto& a, const auto& b) { return a.first < b.first; });
+  E.resize((size_t)n * n);
+  lam.resize(n);
+  for (int k = 0; k < n; k++) {
+    lam[k] = order[k].first;
+    std::copy(full.begin() + (size_t)order[k].second * n,
+              full.begin() + (size_t)(order[k].second + 1) * n, E.begin() + (size_t)k * n);
   }
-  CK(upload_now(dT, T.data(), sizeof(double) * T.size()));
-  *S_dev = dA;
-  *ST_dev = dT;
-  *lam_dev = dlam;
   return SE_OK;
 }
 
@@ -1161,6 +1235,11 @@ struct Eig1D {
   double* ST = nullptr;   // row-major E
   double* lam = nullptr;  // eigenvalues
   double lmax = 0.0;
+  // FP64 inverse: the folded direction's blocks, their eigenvalues and the
+  // low modes' eigenvectors [n][kFdmLow]
+  FoldDir fold;
+  double *FE = nullptr, *FT = nullptr, *lamF = nullptr, *low8 = nullptr;
+  FdmLowMap lowmap;
   void* low[3] = {nullptr, nullptr, nullptr};   // [1] FP32, [2] BF16 copies of S
   void* lowT[3] = {nullptr, nullptr, nullptr};  // and of ST
   // TF32 hi/lo pairs for the tcgen05 products, rows padded to tc_pitch:
@@ -1182,15 +1261,41 @@ int eig_get(const Dir& d, const double* Kh, const double* w, int prec, Eig1D** o
   std::vector<double> Sh;
   if (!e) {
     Eig1D* ne = new Eig1D();
-    ne->n = d.hi - d.lo;
-    if (int rc = eig_1d(d, Kh, w, &ne->S, &ne->ST, &ne->lam, Sh)) {
+    const int n = ne->n = d.hi - d.lo;
+    std::vector<double> lam, FE, FT, lamF;
+    int rc = eig_1d(d, Kh, w, Sh, lam, FE, FT, lamF);
+    if (!rc) {
+      for (double v : lam) ne->lmax = std::max(ne->lmax, std::fabs(v));
+      const FoldDir f = ne->fold = fold_of(d);
+      ne->lowmap = f.on ? FdmLowMap{std::min(kFdmLow / 2, f.ge), std::min(kFdmLow / 2, f.go), f.os}
+                        : FdmLowMap{std::min(kFdmLow, n), 0, f.os};
+      std::vector<double> T((size_t)n * n), low((size_t)n * kFdmLow, 0.0);
+      for (int j = 0; j < n; j++)
+        for (int i = 0; i < n; i++) T[(size_t)i * n + j] = Sh[(size_t)j * n + i];
+      const FdmLowMap& lm = ne->lowmap;
+      for (int k = 0; k < lm.even; k++)
+        for (int i = 0; i < f.ge; i++) low[(size_t)i * kFdmLow + k] = FE[(size_t)i * f.os + k];
+      const int go = f.go;
+      for (int k = 0; k < lm.odd; k++)
+        for (int a = 0; a < go; a++)
+          low[(size_t)(a + (f.periodic ? 1 : 0)) * kFdmLow + kFdmLow / 2 + k] =
+              FE[(size_t)f.ge * f.os + (size_t)a * (f.len - f.os) + k];
+      auto up = [&](double** dst, const std::vector<double>& v) -> int {
+        if (int r = dalloc(dst, v.size())) return r;
+        CK(upload_now(*dst, v.data(), sizeof(double) * v.size()));
+        return SE_OK;
+      };
+      (void)((rc = up(&ne->S, Sh)) || (rc = up(&ne->ST, T)) || (rc = up(&ne->lam, lam)) ||
+             (rc = up(&ne->FE, FE)) || (rc = up(&ne->FT, FT)) || (rc = up(&ne->lamF, lamF)) ||
+             (rc = up(&ne->low8, low)));
+    }
+    if (rc) {
+      for (double* p : {ne->S, ne->ST, ne->lam, ne->FE, ne->FT, ne->lamF, ne->low8})
+        if (p) cudaFree(p);
       delete ne;
       g_eig[dev].erase(key);
       return rc;
     }
-    std::vector<double> lam(ne->n);
-    CK(cudaMemcpy(lam.data(), ne->lam, sizeof(double) * ne->n, cudaMemcpyDeviceToHost));
-    for (double v : lam) ne->lmax = std::max(ne->lmax, std::fabs(v));
     e = ne;
   }
   if (prec == 2 && !e->low[prec]) {
@@ -1383,6 +1488,8 @@ int fdm_setup(se_linsys* ls, int prec) {
   ls->SyT = ey->ST;
   ls->lx = ex->lam;
   ls->ly = ey->lam;
+  ls->eigx = ex;
+  ls->eigy = ey;
   ls->lmax[0] = ex->lmax;
   ls->lmax[1] = ey->lmax;
   ls->Sx_lo = prec ? ex->low[prec] : nullptr;
@@ -1391,10 +1498,11 @@ int fdm_setup(se_linsys* ls, int prec) {
   ls->SyT_lo = prec ? ey->lowT[prec] : nullptr;
   if (!ls->X1) {
     ls->fpart_n = std::max(kFdmPartials, std::max(residual_blocks(op), residual_partial_blocks(op)));
-    if ((rc = dalloc(&ls->X1, n)) || (rc = dalloc(&ls->X2, n)) || (rc = dalloc(&ls->ax, n)) ||
-        (rc = dalloc(&ls->zlow, 64)) || (rc = dalloc(&ls->fpart, 2 * (size_t)ls->fpart_n + 16)))
+    const size_t nf = (size_t)ex->fold.len * ey->fold.len;
+    if ((rc = dalloc(&ls->X1, nf)) || (rc = dalloc(&ls->X2, nf)) || (rc = dalloc(&ls->ax, n)) ||
+        (rc = dalloc(&ls->zlow, kFdmLow * kFdmLow)) || (rc = dalloc(&ls->fpart, 2 * (size_t)ls->fpart_n + 16)))
       return rc;
-    ls->lowk = std::min(8, std::min(op.G[0], op.G[1]));
+    CK(cudaMemsetAsync(ls->zlow, 0, sizeof(double) * kFdmLow * kFdmLow, g_stream));
     if (bloch_ok(op.d[0]) && bloch_ok(op.d[1])) {
       Bloch1D *bx = nullptr, *by = nullptr;
       if ((rc = bloch_get(op.d[0], op.Kh, op.w, &bx)) || (rc = bloch_get(op.d[1], op.Kh, op.w, &by)))
@@ -1458,18 +1566,20 @@ double null_tol(const se_linsys* ls) {
 }
 // out (= or +=) A^{-1} in by four FP64 products on the row-major
 // G_y x G_x unknown arrays F:  Ey^T (F Ex), spectral divide, then
-// Ey ((.) Ex^T), the divide fused into the second product's epilogue and the
-// accumulation into the fourth's (gemm.cu). The lowest lowk x lowk spectral
-// block skips the backward products: the divide moves it to zlow and the
-// fourth product adds Ey[:, <k] (zlow Ex[:, <k]^T) in double-double. For a
-// smooth solution that block holds the largest coefficients, so the FP64
-// rounding of the backward products no longer sets the first step's
-// residual (with refined eigenvectors one step reaches about 3e-11 of the
-// right-hand side in the Jacobi-preconditioned norm at 64x64 elements,
-// p = 8, where plain FP64 products leave about 1e-9).
+// Ey ((.) Ex^T), the divide fused into the second product's epilogue. The
+// array is folded first (launch_fdm_fold), so that a mirror-symmetric
+// direction's factors are two blocks of half the size, and unfolded into the
+// output. The low modes of both directions skip the backward products: the
+// divide moves them to zlow and the unfolding adds them in double-double. For
+// a smooth solution they hold the largest coefficients, so the FP64 rounding
+// of the backward products does not set the first step's residual (with
+// refined eigenvectors one step reaches about 3e-11 of the right-hand side in
+// the Jacobi-preconditioned norm at 64x64 elements, p = 8, where plain FP64
+// products leave about 1e-9). Measured, 768 x 383 unknowns (128x64 elements,
+// p = 6, walls in y): 68 us against 78 with the full factors; a solve at 110x90
+// elements, p = 7, walls all round, 160 us against 257.
 int fdm_apply64(se_linsys* ls, const double* in, double* out, bool accumulate,
                 const FdmState* gate = nullptr) {
-  const int gx = ls->op.G[0], gy = ls->op.G[1];
   const OpDev& op = ls->op;
   const double nt = null_tol(ls);
   if (ls->bloch) {
@@ -1477,16 +1587,36 @@ int fdm_apply64(se_linsys* ls, const double* in, double* out, bool accumulate,
                             accumulate, ls->xh, gate, g_stream));
     return SE_OK;
   }
-  const FdmLow low{ls->zlow, ls->SxT, gx, ls->lowk};
-  CK(launch_fdm_gemm(0, 0, in, 1, ls->SxT, ls->X1, 1, gy, gx, gx, gx, gx, gx, nullptr, nullptr,
-                     nullptr, nullptr, 0, 0, 0, 0, g_stream, nullptr,
-                     gate ? &gate->reason : nullptr));
-  CK(launch_fdm_gemm(0, 1, ls->Sy, 1, ls->X1, ls->X2, 1, gy, gx, gy, gy, gx, gx, nullptr, nullptr,
-                     ls->lx, ls->ly, op.alpha, op.beta[0], op.beta[1], nt, g_stream, &low));
-  CK(launch_fdm_gemm(0, 0, ls->X2, 1, ls->Sx, ls->X1, 1, gy, gx, gx, gx, gx, gx, nullptr, nullptr,
-                     nullptr, nullptr, 0, 0, 0, 0, g_stream));
-  CK(launch_fdm_gemm(0, accumulate ? 2 : 0, ls->SyT, 1, ls->X1, out, 1, gy, gx, gy, gy, gx, gx,
-                     nullptr, nullptr, nullptr, nullptr, 0, 0, 0, 0, g_stream, &low));
+  const Eig1D &ex = *ls->eigx, &ey = *ls->eigy;
+  FdmProduct p;
+  std::memset(&p, 0, sizeof(p));
+  p.x = ex.fold;
+  p.y = ey.fold;
+  auto product = [&](int which, const double* A, const double* B, double* C) {
+    p.which = which;
+    p.A = A;
+    p.B = B;
+    p.C = C;
+    return launch_fdm_dgemm(p, g_stream);
+  };
+  CK(launch_fdm_fold(ex.fold, ey.fold, in, ls->X2, gate ? &gate->reason : nullptr, g_stream));
+  CK(product(FDM_FACTOR_B, ls->X2, ex.FE, ls->X1));
+  p.lx = ex.lamF;
+  p.ly = ey.lamF;
+  p.alpha = op.alpha;
+  p.bx = op.beta[0];
+  p.by = op.beta[1];
+  p.null_tol = nt;
+  p.zlow = ls->zlow;
+  p.low_c = ex.lowmap;
+  p.low_r = ey.lowmap;
+  CK(product(FDM_FACTOR_A, ey.FT, ls->X1, ls->X2));
+  p.lx = p.ly = nullptr;
+  p.zlow = nullptr;
+  CK(product(FDM_FACTOR_B, ls->X2, ex.FT, ls->X1));
+  CK(product(FDM_FACTOR_A, ey.FE, ls->X1, ls->X2));
+  CK(launch_fdm_unfold(ex.fold, ey.fold, ls->X2, out, accumulate, ls->zlow, ex.low8, ey.low8,
+                       g_stream));
   return SE_OK;
 }
 

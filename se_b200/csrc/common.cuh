@@ -401,13 +401,6 @@ cudaError_t launch_tc_split(const double* x, int rows, int cols, int ld, float* 
 // (|divisor| <= null_tol gives 0), 2 accumulate into FP64 C scaled by *cmax
 // (cmax == nullptr: 1). a_fp64: A is FP64 (scaled by 1/*amax when amax is
 // given) whatever prec; c_fp64: C is FP64 (required for epi 2).
-//
-// low (FP64 only, k in 1..8): the lowest k x k block of spectral coefficients
-// carried apart from the backward transform. With epi 1 the block of C
-// (rows and columns < k) is moved into zlow[k][k] and left 0 in C; with
-// epi 0 or 2 the product's outputs get sum_a A[r][a] U[a][c] added, U[a][c] =
-// sum_b zlow[a][b] ex[c * ldex + b], in double-double (with the old value
-// for epi 2), rounded once.
 // One periodic direction of nel = 2^logn equal elements of order p in Bloch
 // form (bloch.cu): V [nel][p][p] complex, row i column k, the W-orthonormal
 // eigenvectors of wavenumber m; mu [nel][p] their eigenvalues; tw [nel/2]
@@ -429,17 +422,56 @@ cudaError_t launch_bloch_inverse(const BlochDir& bx, const BlochDir& by, double 
                                  cudaStream_t s);
 size_t bloch_spectrum_elems(const BlochDir& bx, const BlochDir& by);
 
-struct FdmLow {
-  double* zlow;
-  const double* ex;
-  int ldex, k;
+// A direction of the FP64 dense inverse. Where the direction is its own mirror
+// image (periodic, or two ends of the same kind) every eigenvector is even or
+// odd about the reflection i -> n-1-i (periodic: n-i mod n): `on`. A folded
+// vector holds the ge sums over mirrored pairs (and the fixed points) in slots
+// [0, ge), then the go differences in [os, os + go); the eigenvector matrix
+// becomes an even block of ge modes and an odd one of go, half the
+// multiplications. os and len (the folded length) are even, so that rows of
+// folded arrays and of the blocks start on 16-byte boundaries.
+struct FoldDir {
+  int n, ge, go, os, len, on, periodic;
 };
+// A direction's square factor in an FP64 product: the even block (ge x ge,
+// pitch os) and after it the odd block (go x go, pitch len - os).
+enum { FDM_FACTOR_B = 1, FDM_FACTOR_A = 2 };
+// The low modes of a direction that the FP64 inverse carries apart from the
+// backward products: slots [0, even) and [split, split + odd).
+constexpr int kFdmLow = 8;
+struct FdmLowMap {
+  int even, odd, split;
+};
+// C = A B on folded arrays ([y.len][x.len]) in FP64, one operand the factor of
+// a direction (`which`: B that of x, or A that of y); with lx the spectral
+// divide by alpha + bx lx[col] + by ly[row] (|divisor| <= null_tol gives 0)
+// and, with zlow, the low modes moved into zlow[8][8] (0 left in C).
+struct FdmProduct {
+  const double *A, *B;
+  double* C;
+  FoldDir x, y;
+  int which;
+  const double *lx, *ly;
+  double alpha, bx, by, null_tol;
+  double* zlow;
+  FdmLowMap low_r, low_c;
+};
+cudaError_t launch_fdm_dgemm(const FdmProduct& p, cudaStream_t s);
+// out ([dy.len][dx.len]) = in ([dy.n][dx.n]) folded along both directions (a
+// direction that is not `on` stays as it is); zeros when *gate != 0 (fdm.cu).
+cudaError_t launch_fdm_fold(const FoldDir& dx, const FoldDir& dy, const double* in, double* out,
+                            const int* gate, cudaStream_t s);
+// out (= or +=) the unfolded `in` plus the low modes: sum_ab ly[row][a]
+// zlow[a][b] lx[col][b], ly and lx the low modes' eigenvectors ([n][8]), the
+// sums in double-double, rounded once.
+cudaError_t launch_fdm_unfold(const FoldDir& dx, const FoldDir& dy, const double* in, double* out,
+                              bool accumulate, const double* zlow, const double* lx,
+                              const double* ly, cudaStream_t s);
 cudaError_t launch_fdm_gemm(int prec, int epi, const void* A, int a_fp64, const void* B, void* C,
                             int c_fp64, int M, int N, int K, int lda, int ldb, int ldc,
                             const double* amax, const double* cmax, const double* lx,
                             const double* ly, double alpha, double bx, double by, double null_tol,
-                            cudaStream_t s, const FdmLow* low = nullptr,
-                            const int* gate = nullptr);
+                            cudaStream_t s);
 
 // Fast-diagonalization pieces (fdm.cu). prec: 0 FP64, 1 FP32, 2 BF16.
 cudaError_t launch_spectral_divide(int prec, void* v, int gx, int gy, const double* lx,

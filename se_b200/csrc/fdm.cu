@@ -260,7 +260,147 @@ int blocks_for(size_t n) {
   return (int)(b < 1184 ? (b < 1 ? 1 : b) : 1184);
 }
 
+// ---- folding (FP64 dense inverse) ----
+// Mirror image of i, and the slot of its pair's difference (the sum's is i
+// itself); the odd part skips the fixed point 0 of a periodic direction.
+__device__ __forceinline__ int mirror(const FoldDir& d, int i) {
+  if (!d.on) return i;
+  return d.periodic ? (i == 0 ? 0 : d.n - i) : d.n - 1 - i;
+}
+__device__ __forceinline__ int odd_slot(const FoldDir& d, int i) {
+  return d.os + i - (d.periodic ? 1 : 0);
+}
+
+// Thread = one orbit of the reflections (up to four entries).
+__global__ void __launch_bounds__(256) fdm_fold_kernel(const FoldDir dx, const FoldDir dy,
+                                                       const double* __restrict__ in,
+                                                       double* __restrict__ out,
+                                                       const int* gate) {
+  const int i = blockIdx.x * 32 + (threadIdx.x & 31), j = blockIdx.y * 8 + (threadIdx.x >> 5);
+  if (i >= dx.ge || j >= dy.ge) return;
+  const bool closed = gate && *(volatile const int*)gate != 0;
+  const int im = mirror(dx, i), jm = mirror(dy, j);
+  const size_t n = dx.n;
+  const double a = in[j * n + i], b = in[j * n + im], c = in[jm * n + i], d = in[jm * n + im];
+  const bool px = im != i, py = jm != j;
+  const double se = px ? a + b : a, so = a - b, te = px ? c + d : c, to = c - d;
+  const int oi = odd_slot(dx, i), oj = odd_slot(dy, j);
+  const size_t ld = dx.len;
+  out[j * ld + i] = closed ? 0.0 : py ? se + te : se;
+  if (px) out[j * ld + oi] = closed ? 0.0 : py ? so + to : so;
+  if (py) out[oj * ld + i] = closed ? 0.0 : se - te;
+  if (px && py) out[oj * ld + oi] = closed ? 0.0 : so - to;
+}
+
+// 32 orbit columns x 8 orbit rows a block, one orbit a thread. Every load
+// first; then U = zlow Lx^T per column in double-double, its even and odd x
+// modes apart; then the orbit's four outputs. Bound by latency: the double-
+// double chains, and the passes over arrays that fit L2.
+__global__ void __launch_bounds__(256) fdm_unfold_kernel(const FoldDir dx, const FoldDir dy,
+                                                         const double* __restrict__ in,
+                                                         double* __restrict__ out, int accumulate,
+                                                         const double* __restrict__ zlow,
+                                                         const double* __restrict__ lx,
+                                                         const double* __restrict__ ly) {
+  constexpr int L = kFdmLow, LH = kFdmLow / 2;
+  __shared__ double uh[2][L][32], ul[2][L][32];
+  const int c = threadIdx.x & 31, w = threadIdx.x >> 5;
+  const int i = blockIdx.x * 32 + c, j = blockIdx.y * 8 + w;
+  const bool here = i < dx.ge && j < dy.ge;
+  const int im = mirror(dx, i), oi = odd_slot(dx, i), jm = mirror(dy, j), oj = odd_slot(dy, j);
+  const bool px = im != i, py = jm != j;
+  const size_t n = dx.n, ld = dx.len;
+  // [y parity][x parity]: the products' part v; old: the outputs' old values
+  double v[2][2] = {{0.0, 0.0}, {0.0, 0.0}}, old[4] = {0.0, 0.0, 0.0, 0.0}, e[L];
+  if (here) {
+    v[0][0] = in[j * ld + i];
+    if (px) v[0][1] = in[j * ld + oi];
+    if (py) v[1][0] = in[oj * ld + i];
+    if (px && py) v[1][1] = in[oj * ld + oi];
+    if (accumulate) {
+      old[0] = out[j * n + i];
+      if (px) old[1] = out[j * n + im];
+      if (py) old[2] = out[jm * n + i];
+      if (px && py) old[3] = out[jm * n + im];
+    }
+#pragma unroll
+    for (int a = 0; a < L; a++) e[a] = ly[(size_t)j * L + a];
+  }
+  // a direction that is not folded keeps its low modes in one list: all of
+  // them count as even
+  {
+    double h[2] = {0.0, 0.0}, l[2] = {0.0, 0.0};
+    if (i < dx.ge)
+#pragma unroll
+      for (int b = 0; b < LH; b++) {
+        dd_fma(h[0], l[0], zlow[w * L + b], lx[(size_t)i * L + b]);
+        dd_fma(h[1], l[1], zlow[w * L + LH + b], lx[(size_t)i * L + LH + b]);
+      }
+    if (!dx.on) {
+      dd_add(h[0], l[0], h[1]);
+      l[0] += l[1];
+      h[1] = l[1] = 0.0;
+    }
+#pragma unroll
+    for (int o = 0; o < 2; o++) {
+      uh[o][w][c] = h[o];
+      ul[o][w][c] = l[o];
+    }
+  }
+  __syncthreads();
+  if (!here) return;
+  double h[2][2] = {{0.0, 0.0}, {0.0, 0.0}}, l[2][2] = {{0.0, 0.0}, {0.0, 0.0}};
+#pragma unroll
+  for (int a = 0; a < LH; a++)
+#pragma unroll
+    for (int y = 0; y < 2; y++)
+#pragma unroll
+      for (int x = 0; x < 2; x++) {
+        const int k = a + y * LH;
+        dd_fma(h[y][x], l[y][x], e[k], uh[x][k][c]);
+        l[y][x] = fma(e[k], ul[x][k][c], l[y][x]);
+      }
+  if (!dy.on) {
+#pragma unroll
+    for (int x = 0; x < 2; x++) {
+      dd_add(h[0][x], l[0][x], h[1][x]);
+      l[0][x] += l[1][x];
+      h[1][x] = l[1][x] = 0.0;
+    }
+  }
+#pragma unroll
+  for (int q = 0; q < 4; q++) {
+    const bool my = q & 2, mx = q & 1;
+    if ((my && !py) || (mx && !px)) continue;
+    double s = old[q], r = 0.0;
+#pragma unroll
+    for (int y = 0; y < 2; y++)
+#pragma unroll
+      for (int x = 0; x < 2; x++) {
+        const bool neg = (y && my) != (x && mx);
+        dd_add(s, r, neg ? -h[y][x] : h[y][x]);
+        r += neg ? -l[y][x] : l[y][x];
+        dd_add(s, r, neg ? -v[y][x] : v[y][x]);
+      }
+    out[(size_t)(my ? jm : j) * n + (mx ? im : i)] = s + r;
+  }
+}
+
 }  // namespace
+
+cudaError_t launch_fdm_fold(const FoldDir& dx, const FoldDir& dy, const double* in, double* out,
+                            const int* gate, cudaStream_t s) {
+  const dim3 grid((dx.ge + 31) / 32, (dy.ge + 7) / 8);
+  fdm_fold_kernel<<<grid, 256, 0, s>>>(dx, dy, in, out, gate);
+  return cudaGetLastError();
+}
+cudaError_t launch_fdm_unfold(const FoldDir& dx, const FoldDir& dy, const double* in, double* out,
+                              bool accumulate, const double* zlow, const double* lx,
+                              const double* ly, cudaStream_t s) {
+  const dim3 grid((dx.ge + 31) / 32, (dy.ge + 7) / 8);
+  fdm_unfold_kernel<<<grid, 256, 0, s>>>(dx, dy, in, out, accumulate ? 1 : 0, zlow, lx, ly);
+  return cudaGetLastError();
+}
 
 cudaError_t launch_spectral_divide(int prec, void* v, int gx, int gy, const double* lx,
                                    const double* ly, double alpha, double bx, double by,

@@ -20,13 +20,16 @@
 // Epilogues: store; store after the spectral divide
 // C[l][k] /= alpha + bx lx[k] + by ly[l] (entries whose divisor is below
 // null_tol in magnitude — the null mode — become 0); accumulate into an FP64
-// C with an optional scale read from device memory. The FP64 products can
-// carry the lowest k x k spectral block (k <= 8) apart from the backward
-// transform: the divide moves it out of C into zlow, and the transform's
-// last product adds sum_a A[r][a] U[a][c], U[a][c] = sum_b zlow[a][b]
-// ex[c][b], to its outputs in double-double (the block holds the largest
-// coefficients of a smooth solution, whose FP64 product rounding would
-// otherwise dominate the solve's first residual).
+// C with an optional scale read from device memory (low precisions).
+//
+// FP64 products with a folded direction (FdmBlocks, fdm.cu): the square
+// factor is block-diagonal, an even and an odd block stored one after the
+// other, so the product is two of half the depth in one launch; a block of
+// threads works inside one of them. The divide can move the lowest modes of
+// both directions out of C into zlow (8 x 8), leaving zeros: a smooth
+// solution's largest coefficients, which the unfolding adds back in
+// double-double so that the products' rounding of them does not dominate the
+// solve's first residual.
 #include <cuda_bf16.h>
 
 #include "common.cuh"
@@ -122,15 +125,20 @@ struct GemmArgs {
   const double* cmax;  // accumulate scale, nullptr: 1
   const double *lx, *ly;
   double alpha, bx, by, null_tol;
-  // FP64 only: the low spectral block carried apart (FdmLow, common.cuh);
-  // lowk = 0: none
+  // FP64 only: the folded directions, which operand is a direction's factor,
+  // the low modes
+  FoldDir x, y;
+  int which;
   double* zlow;
-  const double* ex;
-  int ldex, lowk;
-  // FP64 plain stores: when *gate != 0 (a refinement loop that has already
-  // decided) the product is stored as zero; nullptr: no gate
-  const int* gate;
+  FdmLowMap low_r, low_c;
 };
+
+// Place of mode m among the low modes carried apart (-1: not one).
+__device__ __forceinline__ int low_mode(const FdmLowMap& l, int m) {
+  if (m < l.even) return m;
+  const int o = m - l.split;
+  return o >= 0 && o < l.odd ? kFdmLow / 2 + o : -1;
+}
 
 enum { EPI_STORE = 0, EPI_DIVIDE = 1, EPI_ACCUM = 2 };
 
@@ -294,18 +302,10 @@ __global__ void __launch_bounds__(kThreads) fdm_gemm_kernel(const GemmArgs<TA, T
 }
 
 // ---------------------------------------------------------------------------
-// FP64 products: multi-stage cp.async pipeline (8-byte copies with zero fill,
-// so any leading dimension and any edge), BM x BN block tile of WM x WN
-// warps, each warp (BM/WM) x (BN/WN) in m16n8 MMA tiles.
-//
-constexpr int kLowMax = 8;
-// Shared-memory doubles of the low block of a BM x BN output tile: zlow
-// (8 x 8), the tile's rows of A's first 8 columns, U (8 x BN) as hi and lo.
-template <int BM, int BN>
-struct LowSm {
-  static constexpr int SIZE = kLowMax * kLowMax + BM * kLowMax + 2 * kLowMax * BN;
-};
-
+// FP64 products: multi-stage cp.async pipeline (16-byte copies with zero fill;
+// 8-byte ones, which any leading dimension would need, held the products at
+// a third of the FP64 rate), BM x BN block tile of WM x WN warps, each warp
+// (BM/WM) x (BN/WN) in m16n8 MMA tiles.
 template <int BM_, int BN_, int WM_, int WN_, int ST_, int BK_ = 16>
 struct DCfg {
   static constexpr int BM = BM_, BN = BN_, WM = WM_, WN = WN_, ST = ST_;
@@ -314,13 +314,12 @@ struct DCfg {
   static constexpr int MT = BM / WM / 16, NT = BN / WN / 8;
   static constexpr int A_ELEMS = BM * AS, B_ELEMS = BK * BS;
   static constexpr size_t SMEM = (size_t)ST * (A_ELEMS + B_ELEMS) * sizeof(double);
-  static_assert(ST * (A_ELEMS + B_ELEMS) >= LowSm<BM, BN>::SIZE, "low block exceeds the pipeline");
 };
 
-__device__ __forceinline__ void cp_async8(void* smem, const void* gmem, bool valid) {
+// Copies n (0, 1 or 2) doubles and zeros for the rest of 16 bytes.
+__device__ __forceinline__ void cp_async16(void* smem, const void* gmem, int n) {
   const unsigned sa = (unsigned)__cvta_generic_to_shared(smem);
-  asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(sa), "l"(gmem),
-               "r"(valid ? 8 : 0));
+  asm volatile("cp.async.cg.shared.global [%0], [%1], 16, %2;\n" ::"r"(sa), "l"(gmem), "r"(8 * n));
 }
 __device__ __forceinline__ void cp_async_commit() { asm volatile("cp.async.commit_group;\n" ::); }
 template <int N>
@@ -328,86 +327,71 @@ __device__ __forceinline__ void cp_async_wait() {
   asm volatile("cp.async.wait_group %0;\n" ::"n"(N));
 }
 
-// The low block's global operands of one thread, loaded into registers when
-// the kernel starts (they do not depend on the product), so their latency
-// hides behind the main loop: one zlow entry, this thread's share of A's
-// first 8 columns over the tile's rows, and the 8 leading entries of the
-// ex row of the output column whose U entries this thread forms (entries
-// tid, tid + THREADS, ... of the 8 x BN block, all in column tid % BN).
-template <int BM, int BN, int THREADS>
-struct LowRegs {
-  static_assert(THREADS % BN == 0 && THREADS >= kLowMax * kLowMax, "low block thread map");
-  static constexpr int AL = (BM * kLowMax + THREADS - 1) / THREADS;
-  static constexpr int UE = kLowMax * BN / THREADS;
-  double z, al[AL], ex[kLowMax];
+// The output tile of a block and the operands it multiplies: A[row * lda + k]
+// and B[k * ldb + column] for k < K, rows below m_end, columns below n_end; a
+// block of threads works inside one part (even or odd) of either direction.
+struct DTile {
+  const double *A, *B;
+  int m0, n0, m_end, n_end, K, lda, ldb;
 };
-
-template <int BM, int BN, int THREADS>
-__device__ __forceinline__ void low_prefetch(const GemmArgs<double, double, double>& g, int m0,
-                                             int n0, int tid, LowRegs<BM, BN, THREADS>& L) {
-  const int lk = g.lowk;
-  {
-    const int a = tid / kLowMax, b = tid % kLowMax;  // zlow entry (a, b) as an 8 x 8 block
-    L.z = (tid < kLowMax * kLowMax && a < lk && b < lk) ? g.zlow[a * lk + b] : 0.0;
+template <int BM, int BN>
+__device__ __forceinline__ DTile tile_of(const GemmArgs<double, double, double>& g) {
+  const FoldDir &x = g.x, &y = g.y;
+  const int nt = (x.ge + BN - 1) / BN, mt = (y.ge + BM - 1) / BM;
+  const bool xo = (int)blockIdx.x >= nt, yo = (int)blockIdx.y >= mt;
+  DTile t;
+  t.n0 = xo ? x.os + ((int)blockIdx.x - nt) * BN : (int)blockIdx.x * BN;
+  t.m0 = yo ? y.os + ((int)blockIdx.y - mt) * BM : (int)blockIdx.y * BM;
+  t.n_end = xo ? x.os + x.go : x.ge;
+  t.m_end = yo ? y.os + y.go : y.ge;
+  t.lda = t.ldb = x.len;
+  t.A = g.A;
+  t.B = g.B;
+  if (g.which == FDM_FACTOR_B) {
+    t.K = xo ? x.go : x.ge;
+    t.ldb = xo ? x.len - x.os : x.os;
+    if (xo) {
+      t.A += x.os;
+      t.B += (ptrdiff_t)x.ge * x.os - x.os;
+    }
+  } else {
+    t.K = yo ? y.go : y.ge;
+    t.lda = yo ? y.len - y.os : y.os;
+    if (yo) {
+      t.A += (ptrdiff_t)y.ge * y.os - (ptrdiff_t)y.os * t.lda;
+      t.B += (ptrdiff_t)y.os * t.ldb;
+    }
   }
-#pragma unroll
-  for (int q = 0; q < LowRegs<BM, BN, THREADS>::AL; q++) {
-    const int e = tid + q * THREADS, r = e / kLowMax, a = e % kLowMax, gr = m0 + r;
-    L.al[q] = (e < BM * kLowMax && a < lk && gr < g.M) ? g.A[(size_t)gr * g.lda + a] : 0.0;
-  }
-  const int gc = n0 + tid % BN;
-#pragma unroll
-  for (int b = 0; b < kLowMax; b++)
-    L.ex[b] = (b < lk && gc < g.N) ? g.ex[(size_t)gc * g.ldex + b] : 0.0;
+  return t;
+}
+template <int BM, int BN>
+dim3 tile_grid(const GemmArgs<double, double, double>& g) {
+  auto cut = [](const FoldDir& d, int b) { return (d.ge + b - 1) / b + (d.go + b - 1) / b; };
+  return dim3(cut(g.x, BN), cut(g.y, BM));
 }
 
-// Writes the prefetched operands to sm (LowSm layout: zlow as 8 x 8 padded
-// with zeros, A's rows, U hi and lo) and forms U there; ends with the block
-// synchronised.
-template <int BM, int BN, int THREADS>
-__device__ __forceinline__ void low_stage(double* sm, int tid, const LowRegs<BM, BN, THREADS>& L) {
-  double* zl = sm;
-  double* al = zl + kLowMax * kLowMax;
-  double* uh = al + BM * kLowMax;
-  double* ul = uh + kLowMax * BN;
-  if (tid < kLowMax * kLowMax) zl[tid] = L.z;
+// A stage's operands in 16-byte copies (two values; one and a zero at an odd
+// end, zeros beyond).
+template <class C>
+__device__ __forceinline__ void load_stage(const GemmArgs<double, double, double>& g,
+                                           const DTile& t, int k0, double* as, double* bs) {
+  constexpr int AC = C::BK / 2, BC = C::BN / 2;
+  static_assert(C::BM * AC % C::THREADS == 0 && C::BK * BC % C::THREADS == 0 && C::AS % 2 == 0 &&
+                    C::BS % 2 == 0, "stage copies");
 #pragma unroll
-  for (int q = 0; q < LowRegs<BM, BN, THREADS>::AL; q++) {
-    const int e = tid + q * THREADS;
-    if (e < BM * kLowMax) al[e] = L.al[q];
+  for (int e = 0; e < C::BM * AC / C::THREADS; e++) {
+    const int q = threadIdx.x + e * C::THREADS, row = q / AC, col = q % AC * 2;
+    const int gr = t.m0 + row, gc = k0 + col;
+    const int n = gr < t.m_end ? min(2, t.K - gc) : 0;
+    cp_async16(as + row * C::AS + col, n > 0 ? t.A + (ptrdiff_t)gr * t.lda + gc : g.A, max(n, 0));
   }
-  __syncthreads();
-  const int c = tid % BN;
 #pragma unroll
-  for (int q = 0; q < LowRegs<BM, BN, THREADS>::UE; q++) {
-    const int a = (tid + q * THREADS) / BN;
-    double h = 0.0, l = 0.0;
-#pragma unroll
-    for (int b = 0; b < kLowMax; b++) dd_fma(h, l, zl[a * kLowMax + b], L.ex[b]);
-    uh[a * BN + c] = h;
-    ul[a * BN + c] = l;
+  for (int e = 0; e < C::BK * BC / C::THREADS; e++) {
+    const int q = threadIdx.x + e * C::THREADS, row = q / BC, col = q % BC * 2;
+    const int gr = k0 + row, gc = t.n0 + col;
+    const int n = gr < t.K ? min(2, t.n_end - gc) : 0;
+    cp_async16(bs + row * C::BS + col, n > 0 ? t.B + (ptrdiff_t)gr * t.ldb + gc : g.B, max(n, 0));
   }
-  __syncthreads();
-}
-
-// v (the product's FP64 output at tile row r, column c) plus the low block,
-// plus the old value when accumulating, rounded once. Entries beyond lowk
-// are zero in sm, so the sums run over all 8.
-template <int BM, int BN, int EPI>
-__device__ __forceinline__ double low_add(const double* sm, int r, int c, double v,
-                                          const double* dst) {
-  const double* al = sm + kLowMax * kLowMax + r * kLowMax;
-  const double* uh = sm + kLowMax * kLowMax + BM * kLowMax;
-  const double* ul = uh + kLowMax * BN;
-  double h = 0.0, l = 0.0;
-#pragma unroll
-  for (int a = 0; a < kLowMax; a++) {
-    dd_fma(h, l, al[a], uh[a * BN + c]);
-    l = fma(al[a], ul[a * BN + c], l);
-  }
-  dd_add(h, l, v);
-  if constexpr (EPI == EPI_ACCUM) dd_add(h, l, *dst);
-  return h + l;
 }
 
 template <class C, int EPI>
@@ -415,35 +399,15 @@ __global__ void __launch_bounds__(C::THREADS) fdm_dgemm_kernel(const GemmArgs<do
   extern __shared__ __align__(16) double dsm[];
   double* As = dsm;
   double* Bs = dsm + C::ST * C::A_ELEMS;
-  const bool closed = EPI == EPI_STORE && g.gate && *g.gate != 0;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int gq = lane >> 2, tq = lane & 3;
   const int wm = (warp / C::WN) * (C::BM / C::WM), wn = (warp % C::WN) * (C::BN / C::WN);
-  const int m0 = blockIdx.y * C::BM, n0 = blockIdx.x * C::BN;
-  const int nkt = (g.K + C::BK - 1) / C::BK;
-  LowRegs<C::BM, C::BN, C::THREADS> LR;
-  if constexpr (EPI != EPI_DIVIDE) {
-    if (g.lowk) low_prefetch<C::BM, C::BN, C::THREADS>(g, m0, n0, tid, LR);
-  }
+  const DTile t = tile_of<C::BM, C::BN>(g);
+  const int m0 = t.m0, n0 = t.n0;
+  const int nkt = (t.K + C::BK - 1) / C::BK;
 
   auto issue = [&](int i) {
-    const int k0 = i * C::BK;
-    double* as = As + (i % C::ST) * C::A_ELEMS;
-    double* bs = Bs + (i % C::ST) * C::B_ELEMS;
-#pragma unroll
-    for (int e = tid; e < C::BM * C::BK; e += C::THREADS) {
-      const int row = e / C::BK, col = e % C::BK;
-      const int gr = m0 + row, gc = k0 + col;
-      const bool ok = gr < g.M && gc < g.K;
-      cp_async8(as + row * C::AS + col, ok ? g.A + (size_t)gr * g.lda + gc : g.A, ok);
-    }
-#pragma unroll
-    for (int e = tid; e < C::BK * C::BN; e += C::THREADS) {
-      const int row = e / C::BN, col = e % C::BN;
-      const int gr = k0 + row, gc = n0 + col;
-      const bool ok = gr < g.K && gc < g.N;
-      cp_async8(bs + row * C::BS + col, ok ? g.B + (size_t)gr * g.ldb + gc : g.B, ok);
-    }
+    load_stage<C>(g, t, i * C::BK, As + (i % C::ST) * C::A_ELEMS, Bs + (i % C::ST) * C::B_ELEMS);
   };
 
   double acc[C::MT][C::NT][4];
@@ -490,14 +454,6 @@ __global__ void __launch_bounds__(C::THREADS) fdm_dgemm_kernel(const GemmArgs<do
     }
   }
   cp_async_wait<0>();
-  const int lk = g.lowk;
-  if constexpr (EPI != EPI_DIVIDE) {
-    if (lk) {
-      __syncthreads();  // the pipeline's shared memory is free from here
-      low_stage<C::BM, C::BN, C::THREADS>(dsm, tid, LR);
-    }
-  }
-
 #pragma unroll
   for (int mt = 0; mt < C::MT; mt++)
 #pragma unroll
@@ -505,37 +461,30 @@ __global__ void __launch_bounds__(C::THREADS) fdm_dgemm_kernel(const GemmArgs<do
 #pragma unroll
       for (int h = 0; h < 2; h++) {
         const int r = m0 + wm + mt * 16 + gq + 8 * h;
-        if (r >= g.M) continue;
+        if (r >= t.m_end) continue;
 #pragma unroll
         for (int q = 0; q < 2; q++) {
           const int c = n0 + wn + nt * 8 + 2 * tq + q;
-          if (c >= g.N) continue;
+          if (c >= t.n_end) continue;
           double v = acc[mt][nt][2 * h + q];
           double* dst = g.C + (size_t)r * g.ldc + c;
           if constexpr (EPI == EPI_DIVIDE) {
             const double d = g.alpha + g.bx * g.lx[c] + g.by * g.ly[r];
             v = fabs(d) <= g.null_tol ? 0.0 : v / d;
-            if (r < lk && c < lk) {
-              g.zlow[r * lk + c] = v;
+            const int lr = low_mode(g.low_r, r), lc = low_mode(g.low_c, c);
+            if (g.zlow && lr >= 0 && lc >= 0) {
+              g.zlow[lr * kFdmLow + lc] = v;
               v = 0.0;
             }
-          } else {
-            if (lk) {
-              *dst = low_add<C::BM, C::BN, EPI>(dsm, r - m0, c - n0, v, dst);
-              continue;
-            }
           }
-          if constexpr (EPI == EPI_ACCUM)
-            *dst += v;
-          else
-            *dst = closed ? 0.0 : v;
+          *dst = v;
         }
       }
 }
 
 template <class C, int EPI>
 cudaError_t run_d(const GemmArgs<double, double, double>& g, cudaStream_t s) {
-  if (g.M <= 0 || g.N <= 0 || g.K <= 0) return cudaErrorInvalidValue;
+  if (g.M <= 0 || g.N <= 0) return cudaErrorInvalidValue;
   if (C::SMEM > 48 * 1024) {
     static bool attr[64] = {};  // per kernel instantiation and device
     int dev = 0;
@@ -549,8 +498,7 @@ cudaError_t run_d(const GemmArgs<double, double, double>& g, cudaStream_t s) {
       attr[dev] = true;
     }
   }
-  const dim3 grid((g.N + C::BN - 1) / C::BN, (g.M + C::BM - 1) / C::BM);
-  fdm_dgemm_kernel<C, EPI><<<grid, C::THREADS, C::SMEM, s>>>(g);
+  fdm_dgemm_kernel<C, EPI><<<tile_grid<C::BM, C::BN>(g), C::THREADS, C::SMEM, s>>>(g);
   return cudaGetLastError();
 }
 
@@ -560,16 +508,15 @@ cudaError_t run_d(const GemmArgs<double, double, double>& g, cudaStream_t s) {
 // 8 accumulator fragments (8 independent MMA chains) and runs 8 KW MMAs
 // between barriers. At the end the W partial tiles are summed through shared
 // memory in warp order (deterministic) and the epilogue is applied.
-template <int W_, int ST_, int KW_ = 1>
+template <int BN_, int W_, int ST_, int KW_ = 1>
 struct KCfg {
   static constexpr int W = W_, ST = ST_, KW = KW_;
-  static constexpr int BM = 32, BN = 32, BK = 8 * W * KW;
+  static constexpr int BM = 32, BN = BN_, NT = BN / 8, BK = 8 * W * KW;
   static constexpr int AS = BK + 4, BS = BN + 4, RS = BN + 1;
   static constexpr int THREADS = 32 * W;
   static constexpr int A_ELEMS = BM * AS, B_ELEMS = BK * BS;
   static constexpr int PIPE = ST * (A_ELEMS + B_ELEMS), RED = W * BM * RS;
-  static constexpr int LOW = RED + LowSm<BM, BN>::SIZE;  // partial tiles, then the low block
-  static constexpr size_t SMEM = sizeof(double) * (size_t)(PIPE > LOW ? PIPE : LOW);
+  static constexpr size_t SMEM = sizeof(double) * (size_t)(PIPE > RED ? PIPE : RED);
 };
 
 template <class C, int EPI>
@@ -578,41 +525,21 @@ __global__ void __launch_bounds__(C::THREADS) fdm_dgemm_ksplit_kernel(
   extern __shared__ __align__(16) double dsm[];
   double* As = dsm;
   double* Bs = dsm + C::ST * C::A_ELEMS;
-  const bool closed = EPI == EPI_STORE && g.gate && *g.gate != 0;
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int gq = lane >> 2, tq = lane & 3;
-  const int m0 = blockIdx.y * C::BM, n0 = blockIdx.x * C::BN;
-  const int nkt = (g.K + C::BK - 1) / C::BK;
-  LowRegs<C::BM, C::BN, C::THREADS> LR;
-  if constexpr (EPI != EPI_DIVIDE) {
-    if (g.lowk) low_prefetch<C::BM, C::BN, C::THREADS>(g, m0, n0, tid, LR);
-  }
+  const DTile t = tile_of<C::BM, C::BN>(g);
+  const int m0 = t.m0, n0 = t.n0;
+  const int nkt = (t.K + C::BK - 1) / C::BK;
 
   auto issue = [&](int i) {
-    const int k0 = i * C::BK;
-    double* as = As + (i % C::ST) * C::A_ELEMS;
-    double* bs = Bs + (i % C::ST) * C::B_ELEMS;
-#pragma unroll
-    for (int e = tid; e < C::BM * C::BK; e += C::THREADS) {
-      const int row = e / C::BK, col = e % C::BK;
-      const int gr = m0 + row, gc = k0 + col;
-      const bool ok = gr < g.M && gc < g.K;
-      cp_async8(as + row * C::AS + col, ok ? g.A + (size_t)gr * g.lda + gc : g.A, ok);
-    }
-#pragma unroll
-    for (int e = tid; e < C::BK * C::BN; e += C::THREADS) {
-      const int row = e / C::BN, col = e % C::BN;
-      const int gr = k0 + row, gc = n0 + col;
-      const bool ok = gr < g.K && gc < g.N;
-      cp_async8(bs + row * C::BS + col, ok ? g.B + (size_t)gr * g.ldb + gc : g.B, ok);
-    }
+    load_stage<C>(g, t, i * C::BK, As + (i % C::ST) * C::A_ELEMS, Bs + (i % C::ST) * C::B_ELEMS);
   };
 
-  double acc[2][4][4];
+  double acc[2][C::NT][4];
 #pragma unroll
   for (int i = 0; i < 2; i++)
 #pragma unroll
-    for (int j = 0; j < 4; j++)
+    for (int j = 0; j < C::NT; j++)
 #pragma unroll
       for (int q = 0; q < 4; q++) acc[i][j][q] = 0.0;
 
@@ -631,7 +558,7 @@ __global__ void __launch_bounds__(C::THREADS) fdm_dgemm_ksplit_kernel(
 #pragma unroll
     for (int ks = 0; ks < C::KW; ks++) {
       const int kk = (warp * C::KW + ks) * 8;
-      double a[2][4], b[4][2];
+      double a[2][4], b[C::NT][2];
 #pragma unroll
       for (int mt = 0; mt < 2; mt++) {
         const int r0 = mt * 16 + gq;
@@ -641,7 +568,7 @@ __global__ void __launch_bounds__(C::THREADS) fdm_dgemm_ksplit_kernel(
         a[mt][3] = as[(r0 + 8) * C::AS + kk + tq + 4];
       }
 #pragma unroll
-      for (int nt = 0; nt < 4; nt++) {
+      for (int nt = 0; nt < C::NT; nt++) {
         const int c0 = nt * 8 + gq;
         b[nt][0] = bs[(kk + tq) * C::BS + c0];
         b[nt][1] = bs[(kk + tq + 4) * C::BS + c0];
@@ -649,7 +576,7 @@ __global__ void __launch_bounds__(C::THREADS) fdm_dgemm_ksplit_kernel(
 #pragma unroll
       for (int mt = 0; mt < 2; mt++)
 #pragma unroll
-        for (int nt = 0; nt < 4; nt++) mma_f64(acc[mt][nt], a[mt], b[nt]);
+        for (int nt = 0; nt < C::NT; nt++) mma_f64(acc[mt][nt], a[mt], b[nt]);
     }
   }
   cp_async_wait<0>();
@@ -660,21 +587,17 @@ __global__ void __launch_bounds__(C::THREADS) fdm_dgemm_ksplit_kernel(
 #pragma unroll
   for (int mt = 0; mt < 2; mt++)
 #pragma unroll
-    for (int nt = 0; nt < 4; nt++)
+    for (int nt = 0; nt < C::NT; nt++)
 #pragma unroll
       for (int q = 0; q < 4; q++) {
         const int r = mt * 16 + gq + (q >> 1) * 8, c = nt * 8 + 2 * tq + (q & 1);
         red[(warp * C::BM + r) * C::RS + c] = acc[mt][nt][q];
       }
-  const int lk = g.lowk;
-  if constexpr (EPI != EPI_DIVIDE) {
-    if (lk) low_stage<C::BM, C::BN, C::THREADS>(dsm + C::RED, tid, LR);
-  }
   __syncthreads();
   for (int e = tid; e < C::BM * C::BN; e += C::THREADS) {
     const int r = e / C::BN, c = e % C::BN;
     const int gr = m0 + r, gc = n0 + c;
-    if (gr >= g.M || gc >= g.N) continue;
+    if (gr >= t.m_end || gc >= t.n_end) continue;
     double v = red[r * C::RS + c];
 #pragma unroll
     for (int w = 1; w < C::W; w++) v += red[(w * C::BM + r) * C::RS + c];
@@ -682,26 +605,19 @@ __global__ void __launch_bounds__(C::THREADS) fdm_dgemm_ksplit_kernel(
     if constexpr (EPI == EPI_DIVIDE) {
       const double d = g.alpha + g.bx * g.lx[gc] + g.by * g.ly[gr];
       v = fabs(d) <= g.null_tol ? 0.0 : v / d;
-      if (gr < lk && gc < lk) {
-        g.zlow[gr * lk + gc] = v;
+      const int lr = low_mode(g.low_r, gr), lc = low_mode(g.low_c, gc);
+      if (g.zlow && lr >= 0 && lc >= 0) {
+        g.zlow[lr * kFdmLow + lc] = v;
         v = 0.0;
       }
-    } else {
-      if (lk) {
-        *dst = low_add<C::BM, C::BN, EPI>(dsm + C::RED, r, c, v, dst);
-        continue;
-      }
     }
-    if constexpr (EPI == EPI_ACCUM)
-      *dst += v;
-    else
-      *dst = closed ? 0.0 : v;
+    *dst = v;
   }
 }
 
 template <class C, int EPI>
 cudaError_t run_k(const GemmArgs<double, double, double>& g, cudaStream_t s) {
-  if (g.M <= 0 || g.N <= 0 || g.K <= 0) return cudaErrorInvalidValue;
+  if (g.M <= 0 || g.N <= 0) return cudaErrorInvalidValue;
   if (C::SMEM > 48 * 1024) {
     static bool attr[64] = {};  // per kernel instantiation and device
     int dev = 0;
@@ -715,8 +631,7 @@ cudaError_t run_k(const GemmArgs<double, double, double>& g, cudaStream_t s) {
       attr[dev] = true;
     }
   }
-  const dim3 grid((g.N + C::BN - 1) / C::BN, (g.M + C::BM - 1) / C::BM);
-  fdm_dgemm_ksplit_kernel<C, EPI><<<grid, C::THREADS, C::SMEM, s>>>(g);
+  fdm_dgemm_ksplit_kernel<C, EPI><<<tile_grid<C::BM, C::BN>(g), C::THREADS, C::SMEM, s>>>(g);
   return cudaGetLastError();
 }
 
@@ -727,19 +642,14 @@ inline bool small_tiles(int M, int N) { return ((M + 63) / 64) * ((N + 63) / 64)
 template <int P, class TA, class TB, class TC, int EPI>
 cudaError_t run(const GemmArgs<TA, TB, TC>& g, cudaStream_t s) {
   if (g.M <= 0 || g.N <= 0 || g.K <= 0) return cudaErrorInvalidValue;
-  if constexpr (P == 0) {
-    if (small_tiles(g.M, g.N)) return run_k<KCfg<4, 3>, EPI>(g, s);
-    return run_d<DCfg<64, 64, 2, 2, 3>, EPI>(g, s);
+  if (small_tiles(g.M, g.N)) {
+    const dim3 grid((g.N + 31) / 32, (g.M + 31) / 32);
+    fdm_gemm_kernel<P, 32, 32, TA, TB, TC, EPI><<<grid, kThreads, 0, s>>>(g);
   } else {
-    if (small_tiles(g.M, g.N)) {
-      const dim3 grid((g.N + 31) / 32, (g.M + 31) / 32);
-      fdm_gemm_kernel<P, 32, 32, TA, TB, TC, EPI><<<grid, kThreads, 0, s>>>(g);
-    } else {
-      const dim3 grid((g.N + 63) / 64, (g.M + 63) / 64);
-      fdm_gemm_kernel<P, 64, 64, TA, TB, TC, EPI><<<grid, kThreads, 0, s>>>(g);
-    }
-    return cudaGetLastError();
+    const dim3 grid((g.N + 63) / 64, (g.M + 63) / 64);
+    fdm_gemm_kernel<P, 64, 64, TA, TB, TC, EPI><<<grid, kThreads, 0, s>>>(g);
   }
+  return cudaGetLastError();
 }
 
 }  // namespace
@@ -752,25 +662,11 @@ cudaError_t launch_fdm_gemm(int prec, int epi, const void* A, int a_fp64, const 
                             int c_fp64, int M, int N, int K, int lda, int ldb, int ldc,
                             const double* amax, const double* cmax, const double* lx,
                             const double* ly, double alpha, double bx, double by, double null_tol,
-                            cudaStream_t s, const FdmLow* low, const int* gate) {
+                            cudaStream_t s) {
 #define SE_GEMM_ARGS(TA, TB, TC)                                                              \
   GemmArgs<TA, TB, TC> g{(const TA*)A, (const TB*)B, (TC*)C, M, N, K, lda, ldb, ldc, amax, cmax, \
-                         lx, ly, alpha, bx, by, null_tol, nullptr, nullptr, 0, 0, nullptr}
-  if (prec == 0) {
-    SE_GEMM_ARGS(double, double, double);
-    g.gate = gate;
-    if (low && low->k > 0) {
-      if (low->k > kLowMax || !low->zlow || (epi != EPI_DIVIDE && !low->ex))
-        return cudaErrorInvalidValue;
-      g.zlow = low->zlow;
-      g.ex = low->ex;
-      g.ldex = low->ldex;
-      g.lowk = low->k;
-    }
-    if (epi == EPI_DIVIDE) return run<0, double, double, double, EPI_DIVIDE>(g, s);
-    if (epi == EPI_ACCUM) return run<0, double, double, double, EPI_ACCUM>(g, s);
-    return run<0, double, double, double, EPI_STORE>(g, s);
-  }
+                         lx, ly, alpha, bx, by, null_tol, {}, {}, 0, nullptr, {}, {}}
+  if (prec == 0) return cudaErrorInvalidValue;  // launch_fdm_dgemm
   if (prec == 1) {
     if (a_fp64) {
       SE_GEMM_ARGS(double, float, float);
@@ -797,6 +693,35 @@ cudaError_t launch_fdm_gemm(int prec, int epi, const void* A, int a_fp64, const 
   if (epi == EPI_DIVIDE) return run<2, bf, bf, bf, EPI_DIVIDE>(g, s);
   return run<2, bf, bf, bf, EPI_STORE>(g, s);
 #undef SE_GEMM_ARGS
+}
+
+cudaError_t launch_fdm_dgemm(const FdmProduct& p, cudaStream_t s) {
+  GemmArgs<double, double, double> g{p.A, p.B, p.C, p.y.len, p.x.len, 0, 0, 0, p.x.len, nullptr,
+                                     nullptr, p.lx, p.ly, p.alpha, p.bx, p.by, p.null_tol, p.x, p.y,
+                                     p.which, p.zlow, p.low_r, p.low_c};
+  if (!small_tiles(p.y.len, p.x.len))
+    return p.lx ? run_d<DCfg<64, 64, 2, 2, 3>, EPI_DIVIDE>(g, s)
+                : run_d<DCfg<64, 64, 2, 2, 3>, EPI_STORE>(g, s);
+  // The tile width whose fullest SM multiplies least: a direction's two parts
+  // end in partial tiles, and a 301st tile on 148 SMs costs as much as 144
+  // more (768 x 383 unknowns, 300 tiles
+  // of 32 x 32 20.6 us an x product, 396 of 32 x 24 16.1). The 4 stand for a
+  // tile's own cost.
+  auto load = [&](int bn) {
+    const int tiles = ((p.y.ge + 31) / 32 + (p.y.go + 31) / 32) *
+                      ((p.x.ge + bn - 1) / bn + (p.x.go + bn - 1) / bn);
+    return (tiles + 147) / 148 * (bn + 4);
+  };
+  int bn = 32;
+  for (int c : {24, 40})
+    if (load(c) < load(bn)) bn = c;
+#define SE_KCFG(c)                                              \
+  return p.lx ? run_k<KCfg<c, 4, 3>, EPI_DIVIDE>(g, s) \
+              : run_k<KCfg<c, 4, 3>, EPI_STORE>(g, s)
+  if (bn == 24) SE_KCFG(24);
+  if (bn == 40) SE_KCFG(40);
+  SE_KCFG(32);
+#undef SE_KCFG
 }
 
 }  // namespace seg
