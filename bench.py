@@ -488,8 +488,6 @@ SL_FLOPS_PER_VERTEX = (2 * 9 * 5 + 2 * 81 * 2 + 2 * 9 * 2) + (2 * 9 * 5 + 2 * 81
 # DRAM traffic of one SL launch (dram__bytes_read.sum + dram__bytes_write.sum)
 # from one ncu capture of that kernel on this workload.
 SL_TRAFFIC_BYTES = 6.358016e6
-# DRAM traffic of one fdm_dgemm_kernel launch (M = N = K = 512), from one ncu
-# capture of that kernel on this workload (cold caches: read 4.21 MB, write 0).
 
 
 def dense_fdm_roofline(r):

@@ -610,7 +610,7 @@ int linsys_alloc(se_linsys* ls) {
   if (grid <= 0) return fail(SE_ERR_CUDA, "cannot size the cooperative CG launch");
   int sms = 0;
   CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-  ls->patch = patch_plan(ls->op, sms, &ls->pplan);
+  ls->patch = patch_plan_single(ls->op, sms, &ls->pplan);
   Schedule S = make_schedule({&ls->op}, grid);
   ls->grid = (int)S.block_begin.size() - 1;
   ls->nseg = S.nseg;
@@ -710,6 +710,7 @@ int run_cg_patch(se_linsys* ls, const double* b, double* x, double rtol, double 
   PatchLaunch L = patch_launch(ls->op, ls->pplan.gx * ls->pplan.gy, ls->pplan.in_registers,
                                ls->pplan.smem, ls->d_pres);
   L.one = &ps;
+  L.cluster = ls->pplan.cluster;
   if (!ls->ev[0]) {
     CK(cudaEventCreate(&ls->ev[0]));
     CK(cudaEventCreate(&ls->ev[1]));
@@ -3550,7 +3551,7 @@ extern "C" int se_helmholtz_solve_noalloc(const int nEls[2], int N, const double
   int sms = 0;
   CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
   PatchPlan plan;
-  if (patch_plan(op, sms, &plan) && sizeof(PatchPkt) * patch_packets(plan) <= sizeof(double) * 4 * vn) {
+  if (patch_plan_single(op, sms, &plan) && sizeof(PatchPkt) * patch_packets(plan) <= sizeof(double) * 4 * vn) {
     cudaStream_t st = g_stream;
     PatchPkt* pk = reinterpret_cast<PatchPkt*>(z);
     PatchResult* d_res = reinterpret_cast<PatchResult*>(d_solve);
@@ -3558,6 +3559,7 @@ extern "C" int se_helmholtz_solve_noalloc(const int nEls[2], int N, const double
                                      remove_null_space, plan, pk, 1);
     PatchLaunch L = patch_launch(op, plan.gx * plan.gy, plan.in_registers, plan.smem, d_res);
     L.one = &ps;
+    L.cluster = plan.cluster;
     CK(cudaMemsetAsync(pk, 0, sizeof(PatchPkt) * patch_packets(plan), st));
     CK(cudaMemsetAsync(d_res, 0, sizeof(PatchResult), st));
     CK(launch_lift(op, md, sol_dev, lift, st));

@@ -29,11 +29,15 @@
 //      packets, x += a p, r -= a A p, z = D^-1 r, norms; reduction 2.
 // With the constant null space removed, the mean of z is a third reduction.
 //
+// A small solve's blocks form one thread-block cluster and exchange the same
+// values through distributed shared memory instead (CL).
+//
 // What bounds it: latency. At 64x64 elements, p = 8 (262,144 unknowns, 143
-// patches) an iteration takes 6.3 us: about 1.5 us for each of the two
+// patches) an iteration takes 6.4 us: about 1.5 us for each of the two
 // reductions (store to L2, poll), 0.8 us for the stiffness products, 1 us for
 // the node updates, the rest block sums and scalars; the streaming kernel
-// took 20.4 us. At 16x16 elements, p = 6 (64 patches) 4.1 us against 11.4 us.
+// took 20.4 us. At 16x16 elements, p = 6: 2.6 us as a cluster of 16 blocks,
+// 4.1 us as 64 blocks through L2, 11.4 us with the streaming kernel.
 // Several solves of one order share a launch as independent teams of blocks
 // that never wait for one another.
 //
@@ -83,6 +87,66 @@ __device__ __forceinline__ bool get(const PatchPkt* p, unsigned long long seq, d
       : "memory");
   v = __longlong_as_double(b);
   return s == seq;
+}
+
+// ---- cluster form: stores into the other blocks' shared memory ----
+__device__ __forceinline__ unsigned peer_address(const void* p, int rank) {
+  unsigned a = (unsigned)__cvta_generic_to_shared(p), r;
+  asm volatile("mapa.shared::cluster.u32 %0, %1, %2;" : "=r"(r) : "r"(a), "r"(rank));
+  return r;
+}
+// (st.async: the bytes count on the receiving block's mbarrier when they have
+// landed, so that neither side needs a fence; a cluster barrier over plain
+// stores took about 1100 cycles, this about 300)
+__device__ __forceinline__ void store_peer(unsigned at, double v, unsigned bar) {
+  asm volatile("st.async.shared::cluster.mbarrier::complete_tx::bytes.b64 [%0], %1, [%2];" ::"r"(at),
+               "l"(__double_as_longlong(v)), "r"(bar)
+               : "memory");
+}
+__device__ __forceinline__ void put_peer(double2* p, int rank, double a, double b,
+                                         unsigned long long* bar) {
+  asm volatile(
+      "st.async.shared::cluster.mbarrier::complete_tx::bytes.v2.b64 [%0], {%1, %2}, [%3];" ::"r"(
+          peer_address(p, rank)),
+      "l"(__double_as_longlong(a)), "l"(__double_as_longlong(b)), "r"(peer_address(bar, rank))
+      : "memory");
+}
+__device__ __forceinline__ void expect_bytes(unsigned long long* bar, unsigned bytes) {
+  asm volatile("mbarrier.arrive.expect_tx.shared::cta.b64 _, [%0], %1;" ::"r"(
+                   (unsigned)__cvta_generic_to_shared(bar)),
+               "r"(bytes)
+               : "memory");
+}
+__device__ __forceinline__ bool wait_bytes(unsigned long long* bar, unsigned parity) {
+  for (int k = 0; k < kPatchPolls; k++) {
+    unsigned ok;
+    asm volatile(
+        "{\n .reg .pred p;\n mbarrier.try_wait.parity.acquire.cluster.shared::cta.b64 p, [%1], "
+        "%2;\n selp.u32 %0, 1, 0, p;\n}\n"
+        : "=r"(ok)
+        : "r"((unsigned)__cvta_generic_to_shared(bar)), "r"(parity)
+        : "memory");
+    if (ok) return true;
+  }
+  return false;
+}
+__device__ __forceinline__ void cluster_sync() {
+  __syncwarp();
+  asm volatile("barrier.cluster.arrive.release.aligned;\n barrier.cluster.wait.acquire.aligned;"
+               ::: "memory");
+}
+// Sum of the blocks' values in the inbox, by one warp, in a fixed order.
+template <int NV>
+__device__ __forceinline__ void sum_inbox(const double2* in, int G, double* out) {
+  const int l = threadIdx.x & 31;
+  const double2 v = l < G ? in[l] : make_double2(0.0, 0.0);
+#pragma unroll
+  for (int q = 0; q < NV; q++) {
+    double s = q ? v.y : v.x;
+#pragma unroll
+    for (int o = kPatchMaxCluster / 2; o > 0; o >>= 1) s += __shfl_xor_sync(0xffffffffu, s, o);
+    out[q] = s;
+  }
 }
 
 // Sum over a solve's blocks of NV values, by one warp, in a fixed order; the
@@ -187,7 +251,13 @@ __device__ __forceinline__ void block_sum(double (&v)[NV], double2* red2) {
 // K: nodes per thread at most. Up to kPatchRegs of them keep x, the Jacobi
 // inverse, p and the mass coefficient in registers beside r; more keep those
 // in shared memory.
-template <int N, int K>
+//
+// CL: the solve's blocks are one thread-block cluster (at most 16). The edge
+// sums are then stored straight into the neighbour's shared memory and the
+// dot products into every block's inbox, each with its bytes counted on the
+// receiver's mbarrier, in place of the packets; the argument for reusing them
+// is the same.
+template <int N, int K, bool CL>
 __global__ void __launch_bounds__(kPT, 1) cg_patch_kernel(const __grid_constant__ PatchArgs<N> A) {
   constexpr bool REG = K <= kPatchRegs;
   extern __shared__ double sm[];
@@ -200,6 +270,12 @@ __global__ void __launch_bounds__(kPT, 1) cg_patch_kernel(const __grid_constant_
     int its, reason, done, ok;
   } c;
   __shared__ PatchPkt *edge_out[4], *edge_in[4];
+  // CL: where this block's edge sums go (shared address in the neighbour, 0:
+  // the mesh ends here; doubles from one to the next), the sums that arrive
+  __shared__ unsigned edge_at[4], edge_bar[4];
+  __shared__ int edge_step[4];
+  __shared__ unsigned long long arrived[3];  // of the sums A (with the edges), B, M
+  __shared__ double2 inbox[3][kPatchMaxCluster];
   const int tid = threadIdx.x, warp = tid >> 5;
   const int si = A.cta_solve ? A.cta_solve[blockIdx.x] : 0;
   {
@@ -247,8 +323,30 @@ __global__ void __launch_bounds__(kPT, 1) cg_patch_kernel(const __grid_constant_
     else
       nb = at > 0 ? rank - step : (periodic ? rank + last * step : -1);
     const size_t EM = S.edge_stride;
-    edge_out[side] = nb >= 0 ? S.edges + ((size_t)rank * 4 + side) * EM : nullptr;
-    edge_in[side] = nb >= 0 ? S.edges + ((size_t)nb * 4 + (side ^ 1)) * EM : nullptr;
+    if constexpr (CL) {
+      // the neighbour's arrays (its patch may be one element wider or higher)
+      unsigned at = 0;
+      int st = 1;
+      if (nb >= 0) {
+        const int nx = nb % S.gx, ny = nb / S.gx;
+        const int bx = dx.nE * (nx + 1) / S.gx - dx.nE * nx / S.gx;
+        const int by = dy.nE * (ny + 1) / S.gy - dy.nE * ny / S.gy;
+        const int qx = bx * N + 1, qy = by * N + 1, qp = qx | 1, a = qy * qp;
+        const int rx = (REG ? 3 : 5) * a;  // P, KX, KY (DI, X), then RX, RY
+        const int off = side == 0   ? a + bx * N
+                        : side == 1 ? rx
+                        : side == 2 ? 2 * a + by * N * qp
+                                    : rx + (bx + 1) * qy;
+        st = side == 0 ? qp : 1;
+        at = peer_address(sm + off, nb);
+        edge_bar[side] = peer_address(&arrived[0], nb);
+      }
+      edge_at[side] = at;
+      edge_step[side] = st;
+    } else {
+      edge_out[side] = nb >= 0 ? S.edges + ((size_t)rank * 4 + side) * EM : nullptr;
+      edge_in[side] = nb >= 0 ? S.edges + ((size_t)nb * 4 + (side ^ 1)) * EM : nullptr;
+    }
   }
 
   // tables
@@ -274,7 +372,17 @@ __global__ void __launch_bounds__(kPT, 1) cg_patch_kernel(const __grid_constant_
   for (int t = tid; t < (REG ? 3 : 5) * PY * pitch; t += kPT) P[t] = 0.0;
   for (int t = tid; t < (nex + 1) * PY; t += kPT) RX[t] = 0.0;
   for (int t = tid; t < (ney + 1) * PX; t += kPT) RY[t] = 0.0;
-  __syncthreads();
+  if constexpr (CL) {
+    if (tid == 0) {
+      for (int k = 0; k < 3; k++)
+        asm volatile("mbarrier.init.shared::cta.b64 [%0], 1;" ::"r"(
+            (unsigned)__cvta_generic_to_shared(&arrived[k])) : "memory");
+      asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    }
+    cluster_sync();  // no block stores into another before it has cleared its arrays
+  } else {
+    __syncthreads();
+  }
 
   // per-thread nodes: packed (unknown, own, j, i), residual and (REG) x, D^-1,
   // p, alpha wx wy
@@ -311,24 +419,43 @@ __global__ void __launch_bounds__(kPT, 1) cg_patch_kernel(const __grid_constant_
   }
 
   // sum packets, one line a block
-  auto slotA = [&]() { return S.slots; };
-  auto slotB = [&]() { return S.slots + kLine * S.gx * S.gy; };
-  auto slotM = [&]() { return S.slots + 2 * kLine * S.gx * S.gy; };
+  enum { SUM_A = 0, SUM_B = 1, SUM_M = 2 };
+  auto slot = [&](int k) { return S.slots + k * kLine * S.gx * S.gy; };
   unsigned long long seq = S.seq0;
   const int nt = S.norm_type;
+
+  // CL, warp 0: the block's two values to every block's inbox, then every
+  // block's (and extra bytes: the edge sums) in
+  unsigned parity = 0;  // bit k: of arrived[k]
+  auto exchange = [&](int k, double v0, double v1, unsigned extra) {
+    const int G = S.gx * S.gy;
+    if (tid == 0) expect_bytes(&arrived[k], 16u * (unsigned)G + extra);
+    if (tid < G) put_peer(&inbox[k][rank], tid, v0, v1, &arrived[k]);
+    __syncwarp();
+    const bool ok = wait_bytes(&arrived[k], (parity >> k) & 1u);
+    parity ^= 1u << k;
+    return __all_sync(0xffffffffu, ok) != 0;
+  };
 
   // A block's NV sums out, then (warp 0) every block's in: `then` runs on
   // thread 0 with the totals. Ends with a block barrier; false: gave up.
   double rbeta = 0.0;
-  auto reduce2 = [&](PatchPkt* slots, double v0, double v1, auto&& then) {
+  auto reduce2 = [&](int slots, double v0, double v1, auto&& then) {
     double v[2] = {v0, v1};
     block_sum<2>(v, red);
     if (warp == 0) {
-      if (tid < 2) put(slots + kLine * rank + tid, tid ? v[1] : v[0], seq);
-      // while the packets travel: what the totals will be multiplied by
-      rbeta = 1.0 / c.betaold;
       double t[2];
-      const bool ok = sum_packets<2>(slots, S.gx * S.gy, seq, t);
+      bool ok;
+      if constexpr (CL) {
+        rbeta = 1.0 / c.betaold;
+        ok = exchange(slots, v[0], v[1], 0);
+        sum_inbox<2>(inbox[slots], S.gx * S.gy, t);
+      } else {
+        if (tid < 2) put(slot(slots) + kLine * rank + tid, tid ? v[1] : v[0], seq);
+        // while the packets travel: what the totals will be multiplied by
+        rbeta = 1.0 / c.betaold;
+        ok = sum_packets<2>(slot(slots), S.gx * S.gy, seq, t);
+      }
       if (tid == 0) {
         if (!ok) c.ok = 0;
         then(t[0], t[1]);
@@ -338,13 +465,19 @@ __global__ void __launch_bounds__(kPT, 1) cg_patch_kernel(const __grid_constant_
     seq++;
     return c.ok != 0;
   };
-  auto reduce1 = [&](PatchPkt* slots, double v0, auto&& then) {
+  auto reduce1 = [&](int slots, double v0, auto&& then) {
     double v[1] = {v0};
     block_sum<1>(v, red);
     if (warp == 0) {
-      if (tid == 0) put(slots + kLine * rank, v[0], seq);
       double t[1];
-      const bool ok = sum_packets<1>(slots, S.gx * S.gy, seq, t);
+      bool ok;
+      if constexpr (CL) {
+        ok = exchange(slots, v[0], 0.0, 0);
+        sum_inbox<1>(inbox[slots], S.gx * S.gy, t);
+      } else {
+        if (tid == 0) put(slot(slots) + kLine * rank, v[0], seq);
+        ok = sum_packets<1>(slot(slots), S.gx * S.gy, seq, t);
+      }
       if (tid == 0) {
         if (!ok) c.ok = 0;
         then(t[0]);
@@ -408,7 +541,7 @@ __global__ void __launch_bounds__(kPT, 1) cg_patch_kernel(const __grid_constant_
       s0 += r[k];
       s1 += diag(f);
     }
-    if (!reduce2(slotA(), s0, s1, [&](double t0, double t1) { c.cproj = t0 / t1; })) {
+    if (!reduce2(SUM_A, s0, s1, [&](double t0, double t1) { c.cproj = t0 / t1; })) {
       give_up();
       return;
     }
@@ -446,7 +579,7 @@ __global__ void __launch_bounds__(kPT, 1) cg_patch_kernel(const __grid_constant_
   // z with its mean removed: the sums again
   auto mean_sums = [&]() -> bool {
     const double n = (double)S.n;
-    if (!reduce1(slotM(), s_z, [&](double t) { c.zmean = t / n; })) return false;
+    if (!reduce1(SUM_M, s_z, [&](double t) { c.zmean = t / n; })) return false;
     const double zm = c.zmean;
     s_zr = s_n = 0.0;
 #pragma unroll
@@ -460,7 +593,7 @@ __global__ void __launch_bounds__(kPT, 1) cg_patch_kernel(const __grid_constant_
     return true;
   };
   bool good = S.remove_null ? mean_sums() : true;
-  good = good && reduce2(slotB(), s_zr, s_n, [&](double zr, double nn) {
+  good = good && reduce2(SUM_B, s_zr, s_n, [&](double zr, double nn) {
     converged(0, nt == 2 ? zr : nn);
     c.beta = zr;
     if (!c.done && S.max_it <= 0) {
@@ -476,6 +609,16 @@ __global__ void __launch_bounds__(kPT, 1) cg_patch_kernel(const __grid_constant_
   // this thread's first item of the stiffness passes: x items (row j, element
   // e) from thread 0, y items (column i, element e) from the next whole warp
   const int nxi = nex * PY, nxp = (nxi + 31) & ~31, nit = nxp + ney * PX;
+
+  // this block's part of an edge node's stiffness sum, to the other side
+  auto edge_sum = [&](int side, int at, double v) {
+    if constexpr (CL) {
+      if (edge_at[side])
+        store_peer(edge_at[side] + 8u * (unsigned)(at * edge_step[side]), v, edge_bar[side]);
+    } else {
+      if (edge_out[side]) put(edge_out[side] + at, v, seq);
+    }
+  };
 
   while (good && !c.done) {
     // ---- A: direction, stiffness products, energies ----
@@ -513,8 +656,8 @@ __global__ void __launch_bounds__(kPT, 1) cg_patch_kernel(const __grid_constant_
         for (int k = 0; k <= N; k++) v[k] = u[k];
         const double en = eo_product<N, true>(A.cf, v, o);
         acc[0] = fma(ex_row[j], en, acc[0]);
-        if (e == 0 && edge_out[0]) put(edge_out[0] + j, o[0], seq);
-        if (e == nex - 1 && edge_out[1]) put(edge_out[1] + j, o[N], seq);
+        if (e == 0) edge_sum(0, j, o[0]);
+        if (e == nex - 1) edge_sum(1, j, o[N]);
         double* kx = KX + j * pitch + e * N;
 #pragma unroll
         for (int k = 0; k < N; k++) kx[k] = o[k];
@@ -527,8 +670,8 @@ __global__ void __launch_bounds__(kPT, 1) cg_patch_kernel(const __grid_constant_
         for (int k = 0; k <= N; k++) v[k] = u[k * pitch];
         const double en = eo_product<N, true>(A.cf, v, o);
         acc[0] = fma(ey_col[i], en, acc[0]);
-        if (e == 0 && edge_out[2]) put(edge_out[2] + i, o[0], seq);
-        if (e == ney - 1 && edge_out[3]) put(edge_out[3] + i, o[N], seq);
+        if (e == 0) edge_sum(2, i, o[0]);
+        if (e == ney - 1) edge_sum(3, i, o[N]);
         double* ky = KY + (e * N) * pitch + i;
 #pragma unroll
         for (int k = 0; k < N; k++) ky[k * pitch] = o[k];
@@ -537,9 +680,17 @@ __global__ void __launch_bounds__(kPT, 1) cg_patch_kernel(const __grid_constant_
     }
     block_sum<1>(acc, red);
     if (warp == 0) {
-      if (tid == 0) put(slotA() + kLine * rank, acc[0], seq);
       double t[1];
-      const bool ok = sum_packets<1>(slotA(), S.gx * S.gy, seq, t);
+      bool ok;
+      if constexpr (CL) {
+        const unsigned edges = (edge_at[0] ? PY : 0) + (edge_at[1] ? PY : 0) +
+                               (edge_at[2] ? PX : 0) + (edge_at[3] ? PX : 0);
+        ok = exchange(SUM_A, acc[0], 0.0, 8u * edges);
+        sum_inbox<1>(inbox[SUM_A], S.gx * S.gy, t);
+      } else {
+        if (tid == 0) put(slot(SUM_A) + kLine * rank, acc[0], seq);
+        ok = sum_packets<1>(slot(SUM_A), S.gx * S.gy, seq, t);
+      }
       if (tid == 0) {
         if (!ok) c.ok = 0;
         const double dpi = t[0], old = c.dpi;
@@ -552,7 +703,7 @@ __global__ void __launch_bounds__(kPT, 1) cg_patch_kernel(const __grid_constant_
           c.a = c.beta / dpi;
         }
       }
-    } else {
+    } else if constexpr (!CL) {
       // the other warps collect the edge packets meanwhile
       for (int t = tid - 32; t < 2 * (PX + PY); t += kPT - 32) {
         const int side = t < 2 * PY ? (t < PY ? 0 : 1) : (t < 2 * PY + PX ? 2 : 3);
@@ -612,7 +763,7 @@ __global__ void __launch_bounds__(kPT, 1) cg_patch_kernel(const __grid_constant_
       }
     }
     if (S.remove_null) good = mean_sums();
-    good = good && reduce2(slotB(), s_zr, s_n, [&](double zr, double nn) {
+    good = good && reduce2(SUM_B, s_zr, s_n, [&](double zr, double nn) {
       c.its += 1;
       converged(c.its, nt == 2 ? zr : nn);
       if (!c.done) {
@@ -632,6 +783,7 @@ __global__ void __launch_bounds__(kPT, 1) cg_patch_kernel(const __grid_constant_
       }
     });
   }
+  if constexpr (CL) cluster_sync();  // no block leaves while another may store into it
   if (!c.ok) {
     give_up();
     return;
@@ -664,8 +816,10 @@ size_t patch_smem(int N, int nex, int ney, bool regs) {
          ((regs ? 3 : 5) * PY * pitch + (nex + 1) * PY + (ney + 1) * PX + 4 * (PX + PY));
 }
 
+// clusters (cluster form only): how many of these clusters the device holds,
+// instead of a launch.
 template <int N>
-cudaError_t launch_n(const PatchLaunch& L, cudaStream_t s) {
+cudaError_t launch_n(const PatchLaunch& L, cudaStream_t s, int* clusters) {
   constexpr int n = N + 1;
   PatchArgs<N> A;
   std::memset(&A, 0, sizeof(A));
@@ -678,13 +832,38 @@ cudaError_t launch_n(const PatchLaunch& L, cudaStream_t s) {
     A.w[a] = L.w[a];
     A.kd[a] = L.Kh[a * n + a];
   }
-  const void* f = L.in_registers ? (const void*)cg_patch_kernel<N, kPatchRegs>
-                                 : (const void*)cg_patch_kernel<N, kPatchK>;
+  const void* f =
+      L.cluster ? (L.in_registers ? (const void*)cg_patch_kernel<N, kPatchRegs, true>
+                                  : (const void*)cg_patch_kernel<N, kPatchK, true>)
+                : (L.in_registers ? (const void*)cg_patch_kernel<N, kPatchRegs, false>
+                                  : (const void*)cg_patch_kernel<N, kPatchK, false>);
   cudaError_t e =
       cudaFuncSetAttribute(f, cudaFuncAttributeMaxDynamicSharedMemorySize, kPatchSmemMax);
   if (e != cudaSuccess) return e;
+  cudaLaunchConfig_t cfg;
+  std::memset(&cfg, 0, sizeof(cfg));
+  cfg.gridDim = dim3(L.blocks);
+  cfg.blockDim = dim3(kPT);
+  cfg.dynamicSmemBytes = L.smem;
+  cfg.stream = s;
+  cudaLaunchAttribute at;
+  std::memset(&at, 0, sizeof(at));
+  if (L.cluster) {
+    if ((e = cudaFuncSetAttribute(f, cudaFuncAttributeNonPortableClusterSizeAllowed, 1)) !=
+        cudaSuccess)
+      return e;
+    at.id = cudaLaunchAttributeClusterDimension;
+    at.val.clusterDim.x = L.blocks;
+    at.val.clusterDim.y = at.val.clusterDim.z = 1;
+  } else {
+    at.id = cudaLaunchAttributeCooperative;
+    at.val.cooperative = 1;
+  }
+  cfg.attrs = &at;
+  cfg.numAttrs = 1;
+  if (clusters) return cudaOccupancyMaxActiveClusters(clusters, f, &cfg);
   void* args[] = {&A};
-  return cudaLaunchCooperativeKernel(f, dim3(L.blocks), dim3(kPT), args, L.smem, s);
+  return cudaLaunchKernelExC(&cfg, f, args);
 }
 
 }  // namespace
@@ -713,7 +892,7 @@ void patch_plan_table(const OpDev& op, int max_blocks, PatchPlan* out) {
       const double rounds = std::ceil((items + 31) / kPT);
       const double t = (0.9 + 0.06 * N) * items + 250 * rounds + 0.8 * px * py + 3.0 * gx * gy;
       PatchPlan& p = out[gx * gy];
-      if (t < p.cost) p = {gx, gy, (int)(std::max(px, py) + kLine - 1) / kLine * kLine, regs, sm, t};
+      if (t < p.cost) p = {gx, gy, (int)(std::max(px, py) + kLine - 1) / kLine * kLine, regs, 0, sm, t};
     }
   for (int g = 1; g <= max_blocks; g++)
     if (out[g - 1].cost <= out[g].cost) out[g] = out[g - 1];
@@ -724,28 +903,61 @@ size_t patch_smem_bytes(const OpDev& op, const PatchPlan& p, bool in_registers) 
                     in_registers);
 }
 
-bool patch_plan(const OpDev& op, int max_blocks, PatchPlan* out) {
+namespace {
+cudaError_t dispatch(const PatchLaunch& L, cudaStream_t s, int* clusters) {
+  switch (L.N) {
+    case 2: return launch_n<2>(L, s, clusters);
+    case 3: return launch_n<3>(L, s, clusters);
+    case 4: return launch_n<4>(L, s, clusters);
+    case 5: return launch_n<5>(L, s, clusters);
+    case 6: return launch_n<6>(L, s, clusters);
+    case 7: return launch_n<7>(L, s, clusters);
+    case 8: return launch_n<8>(L, s, clusters);
+    case 9: return launch_n<9>(L, s, clusters);
+    case 10: return launch_n<10>(L, s, clusters);
+    case 11: return launch_n<11>(L, s, clusters);
+    case 12: return launch_n<12>(L, s, clusters);
+    default: return cudaErrorInvalidValue;
+  }
+}
+}  // namespace
+
+cudaError_t launch_cg_patch(const PatchLaunch& L, cudaStream_t s) { return dispatch(L, s, nullptr); }
+
+// The cost model's cycles count work; times 1.8 and with 6700 cycles of
+// latency (reductions through L2, block sums, scalars) they matched 16x16
+// p = 6 over 64 blocks (7900) and 64x64 p = 8 over 143 (12000); inside a
+// cluster the latency is about 3100 (16x16 p = 6 over 16 blocks: 5000). So
+// systems up to about 25,000 unknowns run as a cluster.
+bool patch_plan_single(const OpDev& op, int max_blocks, PatchPlan* out) {
   std::vector<PatchPlan> t((size_t)max_blocks + 1);
   patch_plan_table(op, max_blocks, t.data());
   *out = t.back();
-  return out->gx > 0;
-}
-
-cudaError_t launch_cg_patch(const PatchLaunch& L, cudaStream_t s) {
-  switch (L.N) {
-    case 2: return launch_n<2>(L, s);
-    case 3: return launch_n<3>(L, s);
-    case 4: return launch_n<4>(L, s);
-    case 5: return launch_n<5>(L, s);
-    case 6: return launch_n<6>(L, s);
-    case 7: return launch_n<7>(L, s);
-    case 8: return launch_n<8>(L, s);
-    case 9: return launch_n<9>(L, s);
-    case 10: return launch_n<10>(L, s);
-    case 11: return launch_n<11>(L, s);
-    case 12: return launch_n<12>(L, s);
-    default: return cudaErrorInvalidValue;
+  if (out->gx == 0) return false;
+  const double grid = 1.8 * out->cost + 6700.0;
+  // t improves with the block count: the largest cluster first
+  for (int g = std::min(kPatchMaxCluster, max_blocks); g > 0; g--) {
+    PatchPlan p = t[g];
+    if (p.gx == 0 || 1.8 * p.cost + 3100.0 >= grid) break;
+    if (p.gx * p.gy != g) continue;  // the same cut as a smaller count's
+    p.cluster = 1;
+    PatchLaunch L;
+    std::memset(&L, 0, sizeof(L));
+    L.N = op.d[0].N;
+    L.blocks = g;
+    L.in_registers = p.in_registers;
+    L.cluster = true;
+    L.smem = p.smem;
+    L.Kh = op.Kh;
+    L.w = op.w;
+    int held = 0;
+    if (dispatch(L, 0, &held) == cudaSuccess && held > 0) {
+      *out = p;
+      break;
+    }
+    cudaGetLastError();
   }
+  return true;
 }
 
 }  // namespace seg

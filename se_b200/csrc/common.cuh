@@ -301,12 +301,13 @@ struct PatchResult {
 struct PatchPlan {
   int gx, gy, edge_stride;
   bool in_registers;  // every block's nodes fit the kernel form with all state in registers
+  int cluster;        // the blocks are one thread-block cluster
   size_t smem;
   double cost;  // modelled cycles of an iteration's work
 };
 struct PatchLaunch {
   int N, blocks;
-  bool in_registers;
+  bool in_registers, cluster;
   size_t smem;
   const PatchSolve* one;     // host: the solve of a single-solve launch
   const PatchSolve* solves;  // device: a batch's solves (then one is null)
@@ -317,11 +318,13 @@ struct PatchLaunch {
 };
 constexpr int kPatchThreads = 512;
 constexpr int kPatchMaxBlocks = 160;
+constexpr int kPatchMaxCluster = 16;
 constexpr int kPatchLine = 8;  // packets of a 128-byte line
 constexpr int kPatchSmemMax = 224 * 1024;
-// The cut of an operator over at most max_blocks blocks; false: it does not
-// fit on the chip (or has an SVV term).
-bool patch_plan(const OpDev& op, int max_blocks, PatchPlan* out);
+// The cut of a solve of its own over at most max_blocks blocks, as one cluster
+// where that is estimated faster; false: it does not fit on the chip (or has
+// an SVV term).
+bool patch_plan_single(const OpDev& op, int max_blocks, PatchPlan* out);
 // The best cut for every block count 0..max_blocks (gx == 0: it does not fit).
 void patch_plan_table(const OpDev& op, int max_blocks, PatchPlan* out);
 // Shared memory of a plan's blocks in one of the two kernel forms.
