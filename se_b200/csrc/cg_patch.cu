@@ -439,7 +439,6 @@ __global__ void __launch_bounds__(kPT, 1) cg_patch_kernel(const __grid_constant_
 
   // A block's NV sums out, then (warp 0) every block's in: `then` runs on
   // thread 0 with the totals. Ends with a block barrier; false: gave up.
-  double rbeta = 0.0;
   auto reduce2 = [&](int slots, double v0, double v1, auto&& then) {
     double v[2] = {v0, v1};
     block_sum<2>(v, red);
@@ -447,13 +446,10 @@ __global__ void __launch_bounds__(kPT, 1) cg_patch_kernel(const __grid_constant_
       double t[2];
       bool ok;
       if constexpr (CL) {
-        rbeta = 1.0 / c.betaold;
         ok = exchange(slots, v[0], v[1], 0);
         sum_inbox<2>(inbox[slots], S.gx * S.gy, t);
       } else {
         if (tid < 2) put(slot(slots) + kLine * rank + tid, tid ? v[1] : v[0], seq);
-        // while the packets travel: what the totals will be multiplied by
-        rbeta = 1.0 / c.betaold;
         ok = sum_packets<2>(slot(slots), S.gx * S.gy, seq, t);
       }
       if (tid == 0) {
@@ -778,7 +774,7 @@ __global__ void __launch_bounds__(kPT, 1) cg_patch_kernel(const __grid_constant_
           c.done = 1;
         } else {
           c.beta = zr;
-          c.b = zr * rbeta;
+          c.b = zr / c.betaold;
         }
       }
     });

@@ -101,3 +101,23 @@ def test_iteration_limits_and_zero_rhs(segpu):
     st = ls.Solve()
     assert st["its"] == 0 and st["reason"] in (2, 3)
     assert not np.any(u.vals)
+
+
+@pytest.mark.parametrize("case", [3, 5])
+@pytest.mark.parametrize("batched", [False, True])
+def test_subnormal_inner_products(segpu, oracle, case, batched):
+    """Data so small that the inner products are subnormal: the solve ends as
+    the oracle's does (the product of successive p . A p underflows, reason
+    -10 after one step) and leaves finite values, not those of an overflowed
+    1 / beta. Single solves run as a cluster, batches through packets."""
+    e = 1e-156
+    om, m, fs, fr, ls, A, f2v, v2f, sol, rhs = build(segpu, oracle, SMALL[case], -3.0, -1.0, 1.0,
+                                                     True, seed=case + 40)
+    fs.vals, fr.vals = sol * e, rhs * e
+    ls.Assemble()
+    ref, st = oracle.helmholtz_solve(om, sol * e, rhs * e, -3.0, -1.0, 1.0, bcs=SMALL[case][6],
+                                     quirk=True, rtol=1e-10, atol=0.0)
+    ls.set_opts(segpu.solver_opts(rtol=1e-10, atol=0.0))
+    out = segpu.solve_batch([ls])[0] if batched else ls.Solve("helm_")
+    assert (out["reason"], out["its"]) == (st["reason"], st["its"]) == (-10, 1)
+    assert np.isfinite(fs.vals).all() and np.isfinite(out["rnorm"])
