@@ -60,9 +60,10 @@ __device__ __forceinline__ double local_coord(const MeshDev& m, int d, double c,
 // Element and local coordinate of c along d: get_topo and local_coord, bit
 // for bit, without their division away from element boundaries. (c - min) /
 // dx and the product q with the rounded reciprocal differ by at most a few
-// units in the last place, so where q is below 2^19 and further than 1e-9
-// from an integer both have the same integer part and the boundary
-// tolerances (1e-12) do not apply; the rest takes the division.
+// units in the last place, so where |q| is below 2^19 (beyond 2^31 the sum's
+// low word would also alias) and further than 1e-9 from an integer both have
+// the same integer part and the boundary tolerances (1e-12) do not apply; the
+// rest takes the division.
 __device__ __forceinline__ int locate(const MeshDev& m, int d, double c, double& l, unsigned* err) {
   const double off = xsub(c, m.min[d]);
   const double q = xmul(off, m.inv_dx[d]);
@@ -70,7 +71,7 @@ __device__ __forceinline__ int locate(const MeshDev& m, int d, double c, double&
   const double t = xadd(q, magic), r = xsub(t, magic);
   const bool below = q < r;
   int topo = __double2loint(t) - (below ? 1 : 0);
-  if (fabs(xsub(q, r)) > 1.0e-9 && q < 524288.0 && (unsigned)topo < (unsigned)m.nEls[d]) {
+  if (fabs(xsub(q, r)) > 1.0e-9 && fabs(q) < 524288.0 && (unsigned)topo < (unsigned)m.nEls[d]) {
     l = xsub(xmul(xsub(off, xmul(below ? xsub(r, 1.0) : r, m.dx[d])), m.two_over_dx[d]), 1.0);
     if (l < -1.0) l = -1.0;
     if (l > +1.0) l = +1.0;

@@ -87,3 +87,44 @@ def test_second_order_both_forms(segpu, oracle, nx, ny, N, per):
     adv2.Advect(dt)
     acc2 = om.advect(u, u, dt, field_prev=up, vel_prev=up, nthreads=8)
     assert np.abs(adv2.fieldSL.vals - acc2).max() <= ACC_TOL * np.abs(acc2).max()
+
+
+@pytest.mark.parametrize("N", [4, 7])
+@pytest.mark.parametrize("far", [2.0 ** 19 + 3.25, 2.0 ** 31 + 3.25, 2.0 ** 32 - 2.25, 2.0 ** 32 + 3.25,
+                                 2.0 ** 33 - 1.75, 2.0 ** 40 + 4.5, 2.0 ** 50 + 2.25])
+@pytest.mark.parametrize("axis", [0, 1])
+@pytest.mark.parametrize("side", [-1.0, 1.0])
+def test_points_far_outside(segpu, N, far, axis, side):
+    """A point billions of elements outside the mesh takes the value of the
+    mesh's edge, as the reference's search clamped to the mesh gives it, and
+    not that of the element its index is congruent to modulo 2^32. (The
+    spacing is a power of two, so both coordinates are exact; the field is
+    linear and the local coordinate clamped to an end node, so is the value.)"""
+    nE = 8
+    m = make(segpu, nE, nE, N, (0.0, 0.0), (2.0, 2.0), (False, False))
+    X = m.verts
+    f = segpu.Field("f", m, 1, None)
+    f.vals = X[:, axis] + 1.0
+    p = np.array([[0.3, 0.3]])
+    p[0, axis] = side * far * 0.25
+    got = f.InterpGlobal(p)[0, 0]
+    el, lc = m.GlobalToLocal(p)
+    end = nE - 1 if side > 0 else 0
+    assert (el[0] % nE, el[0] // nE)[axis] == end and lc[0, axis] == side
+    assert abs(got - (3.0 if side > 0 else 1.0)) <= 1e-12
+
+
+def test_departures_far_outside_are_refused(segpu):
+    """A flow of 2^33 elements a step is an error, not a gather at the element
+    its departure points are congruent to."""
+    m = make(segpu, 8, 8, 5, (0.0, 0.0), (1.1, 0.9), (True, True))
+    f, v = segpu.Field("f", m, 1, None), segpu.Field("v", m, 2, None)
+    f.vals = np.cos(m.verts[:, 0])
+    for c in (2.0 ** 33 + 8, 2.0 ** 33 + 11.3, -(2.0 ** 33) - 9.1):
+        v.vals = np.tile([c * 1.1 / 8, 0.0], (m.nVertsTotal, 1))
+        adv = segpu.Advector(f, v)
+        adv.record_departures()
+        adv.Advect(1.0)
+        with pytest.raises(segpu.SEError) as e:
+            adv.departures()
+        assert e.value.code == segpu.SE_ERR_DOMAIN
