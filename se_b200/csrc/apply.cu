@@ -42,6 +42,7 @@
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 
+#include <algorithm>
 #include <cstdint>
 #include <cstring>
 
@@ -386,11 +387,11 @@ __device__ __forceinline__ void el_passes(const ElArgs<N, A>& op, const A* X, A*
 }
 
 // quads: x in 16 bits with rows a multiple of four long and an 8-byte aligned
-// base.
+// base. y0: the first row of vertices of this launch.
 template <int N, class TI, class A, class TO, int MINB>
 __global__ void __launch_bounds__(kEfThreads, MINB)
     apply_el_kernel(const __grid_constant__ ElArgs<N, A> op, const TI* __restrict__ x,
-                    TO* __restrict__ y, int quads) {
+                    TO* __restrict__ y, int quads, int y0) {
   typedef EfTile<N> T;
   constexpr bool LOW = sizeof(TI) != sizeof(A);
   constexpr int W = LOW ? (T::SW + 3) | 1 : T::W;
@@ -398,7 +399,7 @@ __global__ void __launch_bounds__(kEfThreads, MINB)
   A* X = reinterpret_cast<A*>(el_smem);  // vertices (gx0-N .. gx0+TX) x (gy0-N .. gy0+TY)
   A* OX = X + T::H * W;                  // row-pass results of the tile's vertices
   A* sw = OX + T::TY * T::OXP;           // assembled weights of an element's first N nodes
-  const int gx0 = blockIdx.x * T::TX, gy0 = blockIdx.y * T::TY;
+  const int gx0 = blockIdx.x * T::TX, gy0 = blockIdx.y * T::TY + y0;
   if (threadIdx.x < N)
     sw[threadIdx.x] = threadIdx.x == 0 ? op.w[0] + op.w[N] : op.w[threadIdx.x];
   bool interior = inside(op.dx, gx0 - N, gx0 + T::TX) && inside(op.dy, gy0 - N, gy0 + T::TY);
@@ -460,8 +461,11 @@ cudaError_t launch_el(const OpDev& od, const TI* x, TO* y, cudaStream_t s) {
     }
   }
   const int quads = LOW && od.G[0] % 4 == 0 && (reinterpret_cast<uintptr_t>(x) & 7) == 0;
-  const dim3 grid((od.d[0].hi + T::TX - 1) / T::TX, (od.d[1].hi + T::TY - 1) / T::TY);
-  apply_el_kernel<N, TI, A, TO, MINB><<<grid, kEfThreads, smem, s>>>(op, x, y, quads);
+  const int rows = (od.d[1].hi + T::TY - 1) / T::TY;
+  for (int r = 0; r < rows; r += kGridRows) {
+    const dim3 grid((od.d[0].hi + T::TX - 1) / T::TX, std::min(rows - r, kGridRows));
+    apply_el_kernel<N, TI, A, TO, MINB><<<grid, kEfThreads, smem, s>>>(op, x, y, quads, r * T::TY);
+  }
   return cudaGetLastError();
 }
 

@@ -101,6 +101,9 @@ __device__ __forceinline__ void dd_fma(double& hi, double& lo, double a, double 
   lo += pe;
 }
 
+// Largest y extent of a grid: more rows of blocks take several launches.
+constexpr int kGridRows = 65535;
+
 // ---------------------------------------------------------------------------
 // Host launch wrappers (defined in sl.cu / linsys.cu). All take the stream.
 

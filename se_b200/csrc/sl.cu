@@ -309,10 +309,10 @@ constexpr int kSlX = 8, kSlY = kSlThreads / kSlX;
 // The thread's vertex: eight consecutive lanes (one pass of the L1 data path
 // for 16-byte loads) are a 4 x 2 block of vertices, which seldom falls into
 // more than two elements.
-__device__ __forceinline__ void sl_vertex(int& i, int& j) {
+__device__ __forceinline__ void sl_vertex(int y0, int& i, int& j) {
   const int t = threadIdx.x;
   i = blockIdx.x * kSlX + ((t & 3) | ((t >> 1) & 4));
-  j = blockIdx.y * kSlY + (((t >> 2) & 1) | ((t >> 3) & 2) | ((t >> 5) << 2));
+  j = blockIdx.y * kSlY + y0 + (((t >> 2) & 1) | ((t >> 3) & 2) | ((t >> 5) << 2));
 }
 
 __device__ __forceinline__ bool owned(const MeshDev& m, int i, int j) {
@@ -324,9 +324,9 @@ template <int N, class FSrc>
 __global__ void __launch_bounds__(kSlThreads, 4)
     sl_first_kernel(const MeshDev m, FSrc field, const double2* __restrict__ vel, double dt,
                     double half_dt, double* __restrict__ out, int* __restrict__ dep_el,
-                    double2* __restrict__ dep_xy, unsigned* err) {
+                    double2* __restrict__ dep_xy, unsigned* err, int y0) {
   int i, j;
-  sl_vertex(i, j);
+  sl_vertex(y0, i, j);
   const int nvx = m.nVerts[0], nvy = m.nVerts[1];
   const bool owner = owned(m, i, j);
   if (i >= nvx || j >= nvy || (!owner && !dep_el)) return;
@@ -359,9 +359,9 @@ __global__ void __launch_bounds__(kSlThreads, 4)
                      const double2* __restrict__ vel, const double2* __restrict__ vel_prev,
                      const Half plus_half, const Half minus_half, double dt, double half_dt,
                      double* __restrict__ out, int* __restrict__ dep_el,
-                     double2* __restrict__ dep_xy, unsigned* err) {
+                     double2* __restrict__ dep_xy, unsigned* err, int y0) {
   int i, j;
-  sl_vertex(i, j);
+  sl_vertex(y0, i, j);
   const int nvx = m.nVerts[0], nvy = m.nVerts[1];
   const bool owner = owned(m, i, j);
   if (i >= nvx || j >= nvy || (!owner && !dep_el)) return;
@@ -424,22 +424,24 @@ cudaError_t launch_sl_t(const MeshDev& m, const FSrc field, const FSrc field_pre
   const double2* v = reinterpret_cast<const double2*>(vel);
   const double2* vm = reinterpret_cast<const double2*>(vel_prev);
   double2* dxy = reinterpret_cast<double2*>(dep_xy);
-  const dim3 grid((m.nVerts[0] + kSlX - 1) / kSlX, (m.nVerts[1] + kSlY - 1) / kSlY);
-  if (!second) {
-    sl_first_kernel<N, FSrc><<<grid, kSlThreads, 0, s>>>(m, field, v, dt, half_dt, out, dep_el,
-                                                         dxy, err);
-    return cudaGetLastError();
-  }
   const Vec2Mix plus{v, vm, 1.5, -0.5}, minus{v, vm, 0.5, 0.5};
-  if (mix) {
-    const int nv = m.nVerts[0] * m.nVerts[1];
-    double2* x = reinterpret_cast<double2*>(mix);
-    mix_kernel<<<(nv + 255) / 256, 256, 0, s>>>(nv, plus, minus, x);
-    sl_second_kernel<N, FSrc, Vec2><<<grid, kSlThreads, 0, s>>>(
-        m, field, field_prev, v, vm, Vec2{x}, Vec2{x + nv}, dt, half_dt, out, dep_el, dxy, err);
-  } else {
-    sl_second_kernel<N, FSrc, Vec2Mix><<<grid, kSlThreads, 0, s>>>(
-        m, field, field_prev, v, vm, plus, minus, dt, half_dt, out, dep_el, dxy, err);
+  const int nv = m.nVerts[0] * m.nVerts[1];
+  double2* x = reinterpret_cast<double2*>(mix);
+  if (second && mix) mix_kernel<<<(nv + 255) / 256, 256, 0, s>>>(nv, plus, minus, x);
+  const int rows = (m.nVerts[1] + kSlY - 1) / kSlY;
+  for (int r = 0; r < rows; r += kGridRows) {
+    const dim3 grid((m.nVerts[0] + kSlX - 1) / kSlX, std::min(rows - r, kGridRows));
+    if (!second)
+      sl_first_kernel<N, FSrc><<<grid, kSlThreads, 0, s>>>(m, field, v, dt, half_dt, out, dep_el,
+                                                           dxy, err, r * kSlY);
+    else if (mix)
+      sl_second_kernel<N, FSrc, Vec2><<<grid, kSlThreads, 0, s>>>(
+          m, field, field_prev, v, vm, Vec2{x}, Vec2{x + nv}, dt, half_dt, out, dep_el, dxy, err,
+          r * kSlY);
+    else
+      sl_second_kernel<N, FSrc, Vec2Mix><<<grid, kSlThreads, 0, s>>>(
+          m, field, field_prev, v, vm, plus, minus, dt, half_dt, out, dep_el, dxy, err,
+          r * kSlY);
   }
   return cudaGetLastError();
 }

@@ -103,3 +103,31 @@ def test_reduced_precision(segpu, N, kind, half):
         assert got[0] == 7.0 and got[-1] == 7.0
         xr = x.double().numpy()
         assert (np.abs(got[1:-1] - apply(xr)) <= 64 * 2.0 ** -24 * apply(xr, True)).all(), (nx, ny)
+
+
+@pytest.mark.parametrize("N,ny", [(2, 262142), (3, 262145)])
+def test_tallest_meshes(segpu, N, ny):
+    """More rows of unknowns than a grid's y dimension of tiles covers (65535
+    tiles of 4 N), FP64 and BF16, against the residual's kernel (r = 0 - A x,
+    which steps over its tiles) at the tolerances above, row sums of
+    magnitudes bounded by 4 times the largest element entries."""
+    import torch
+    m = segpu.Mesh("m", [1, ny], "legendre", N, [0.0, 0.0], [1.0, float(ny)], [False, False])
+    u = segpu.Field("u", m, 1, segpu.BCs(False, False, False, False, m))
+    ls = segpu.HelmholtzEqn(u, None, -3.0, -1.0, 0.5, 0, segpu.solver_opts(mode=segpu.MODE_EXACT))
+    n = ls.vecSize
+    xb = torch.randn(n, device="cuda", generator=torch.Generator("cuda").manual_seed(N)).bfloat16()
+    x = xb.double()
+    y, r, zero = (torch.zeros(n, device="cuda", dtype=torch.float64) for _ in range(3))
+    yf = torch.full((n,), float("nan"), device="cuda")
+    ls.residual(x.data_ptr(), zero.data_ptr(), r.data_ptr())
+    y.fill_(float("nan"))
+    torch.cuda.synchronize()
+    ls.apply(x.data_ptr(), y.data_ptr())
+    ls.apply_low(xb.data_ptr(), yf.data_ptr(), segpu.PREC_BF16)
+    segpu.synchronize()
+    gx, gw, D = m.gll()
+    Kh = np.abs(D.T @ np.diag(gw) @ D)
+    scale = float(x.abs().max()) * 4.0 * (3.0 * gw.max() ** 2 / 4 + Kh.sum(1).max() * gw.max())
+    assert float((y + r).abs().max()) <= 64 * 2.0 ** -53 * scale
+    assert float((yf.double() + r).abs().max()) <= 64 * 2.0 ** -24 * scale

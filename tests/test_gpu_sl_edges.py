@@ -128,3 +128,24 @@ def test_departures_far_outside_are_refused(segpu):
         with pytest.raises(segpu.SEError) as e:
             adv.departures()
         assert e.value.code == segpu.SE_ERR_DOMAIN
+
+
+@pytest.mark.parametrize("order", [1, 2])
+def test_tallest_meshes(segpu, order):
+    """More rows of vertices than a grid's y dimension of blocks covers (65535
+    blocks of 16): 349,526 elements of order 3 are 1,048,579. A field linear
+    in y under a uniform flow is moved by the displacement, cut off at the
+    walls; coordinates near 3.5e5 are known to 6e-11."""
+    ny = 349526
+    m = make(segpu, 1, ny, 3, (0.0, 0.0), (1.0, float(ny)), (False, False))
+    y = m.verts[:, 1]
+    f, v = segpu.Field("f", m, 1, None), segpu.Field("v", m, 2, None)
+    f.vals = y
+    v.vals = np.tile([0.0, 0.7], (m.nVertsTotal, 1))
+    if order == 1:
+        adv, want = segpu.Advector(f, v), np.maximum(y - 0.7, 0.0)
+    else:  # 2 f(x1) - f(x2) / 2 with both levels of the field equal
+        adv = segpu.Advector(f, v, f, v)
+        want = 2.0 * np.maximum(y - 0.7, 0.0) - 0.5 * np.maximum(y - 1.4, 0.0)
+    adv.Advect(1.0)
+    assert np.abs(adv.fieldSL.vals - want).max() <= 1e-9
