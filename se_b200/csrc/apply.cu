@@ -17,15 +17,16 @@
 // The stiffness products run by even/odd halves (kh.cuh) with coefficients in
 // the kernel parameters, the beta factors folded in.
 //
-// Almost every tile is interior: all staged vertices are unknowns, nothing
-// wraps, every element and its left and lower neighbours exist. Its path has
-// no conditions: a staged row is one contiguous run of the unknown array (one
-// address a row, copies at fixed offsets from it) and the weights are the
-// element's own. The others take the general path (a neighbour element that
-// does not exist contributes nothing, by a flag and not by the zero fill,
-// because its own node carries a value). Both compute the same sums in the
-// same order, every output by one thread: the result does not depend on
-// scheduling.
+// Almost every tile of a large mesh is interior: all staged vertices are
+// unknowns, nothing wraps, every element and its left and lower neighbours
+// exist. Its path has no conditions: a staged row is one contiguous run of the
+// unknown array (one address a row, copies at fixed offsets from it) and the
+// weights are the element's own. The others take the general path (a
+// neighbour element that does not exist contributes nothing, by a flag and not
+// by the zero fill, because its own node carries a value), each direction's
+// conditions apart: in a mesh not much wider than a tile, where no tile is
+// interior, most have none along y. All compute the same sums in the same
+// order, every output by one thread: the result does not depend on scheduling.
 //
 // Types: FP64 (x, arithmetic, y), staged by 8-byte cp.async; the reduced-
 // precision apply (x in BF16 or FP16, operator and arithmetic in FP32, y in
@@ -38,7 +39,9 @@
 // p = 10, 17.3 us (56 us on the FP64 tensor cores, whose 8-wide steps pad
 // 11-wide elements, with a host wait for its bounded TMA waits); p = 3, 12 and
 // 11: 31, 28 and 25 us against 92, 104 and 138. BF16, 37.7M unknowns, p = 8:
-// 78 us against 117.
+// 78 us against 117. Without interior tiles: 7 x 50,000 elements, p = 5,
+// between walls 47 us (70 with both directions' conditions in every tile),
+// BF16 43 (66).
 #include <cuda_bf16.h>
 #include <cuda_fp16.h>
 
@@ -97,6 +100,14 @@ struct EfTile {
   static_assert(SW > 64 && SW <= 96, "staging columns");
 };
 constexpr int kEfThreads = 256, kEfWarps = kEfThreads / 32;
+
+// The apply's tile: R times four element rows, up to R items a thread and pass.
+template <int N, int R>
+struct ElTile : EfTile<N> {
+  static constexpr int TY = 4 * N * R;
+  static constexpr int H = TY + N + 1;
+  static constexpr int ITEMS = EfTile<N>::EX * TY;
+};
 
 // Whether the staged range of a tile along d lies inside the unknowns and all
 // elements it touches exist.
@@ -160,10 +171,10 @@ struct ElArgs {
 };
 
 // Interior staging, FP64: one address a row, three copies at fixed offsets.
-template <int N>
+template <int N, int R>
 __device__ __forceinline__ void stage_interior(const ElArgs<N, double>& op, const double* x,
                                                double* X, int gx0, int gy0, int) {
-  typedef EfTile<N> T;
+  typedef ElTile<N, R> T;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   const double* src = x + (size_t)(gy0 - N - op.dy.lo + warp) * op.G0 + (gx0 - N - op.dx.lo + lane);
   unsigned dst = (unsigned)__cvta_generic_to_shared(X + warp * T::W + lane);
@@ -204,10 +215,10 @@ __device__ __forceinline__ void unpack4(uint2 q, float (&f)[4], __half) {
 // aligned): loads of four values from the boundary at or before the row's
 // first vertex, quads - 1 values further left. The staged row then starts
 // quads - 1 floats into its pitch.
-template <int N, class TI>
+template <int N, int R, class TI>
 __device__ __forceinline__ void stage_interior(const ElArgs<N, float>& op, const TI* x, float* X,
                                                int gx0, int gy0, int quads) {
-  typedef EfTile<N> T;
+  typedef ElTile<N, R> T;
   constexpr int W = (T::SW + 3) | 1;
   const size_t q0 = (size_t)(gy0 - N - op.dy.lo) * op.G0 + (gx0 - N - op.dx.lo);
   if (quads) {
@@ -243,10 +254,10 @@ __device__ __forceinline__ void stage_interior(const ElArgs<N, float>& op, const
   const TI* src = x + q0 + (size_t)warp * op.G0 + lane;
   float* dst = X + warp * W + lane;
   const size_t step = (size_t)kEfWarps * op.G0;
-  constexpr int R = (T::H + kEfWarps - 1) / kEfWarps;
-  TI v[R][3];
+  constexpr int Q = (T::H + kEfWarps - 1) / kEfWarps;
+  TI v[Q][3];
 #pragma unroll
-  for (int r = 0; r < R; r++) {
+  for (int r = 0; r < Q; r++) {
     if (warp + r * kEfWarps < T::H) {
       v[r][0] = src[0];
       v[r][1] = src[32];
@@ -255,7 +266,7 @@ __device__ __forceinline__ void stage_interior(const ElArgs<N, float>& op, const
     src += step;
   }
 #pragma unroll
-  for (int r = 0; r < R; r++) {
+  for (int r = 0; r < Q; r++) {
     if (warp + r * kEfWarps < T::H) {
       dst[0] = to_a(v[r][0], 0.f);
       dst[32] = to_a(v[r][1], 0.f);
@@ -266,48 +277,97 @@ __device__ __forceinline__ void stage_interior(const ElArgs<N, float>& op, const
 }
 
 // General staging: every vertex mapped, zero where there is no unknown (the
-// loads of a 16-bit tile issued before any is used).
-template <int N>
+// loads of a 16-bit tile issued before any is used). YIN: the staged rows are
+// consecutive rows of unknowns, only the columns need mapping (a mesh not
+// much wider than a tile consists of such tiles).
+template <int N, int R, bool YIN>
 __device__ __forceinline__ void stage_general(const ElArgs<N, double>& op, const double* x,
                                               double* X, int gx0, int gy0) {
-  ef_stage<N>(op.dx, op.dy, op.G0, x, X, gx0, gy0);
+  typedef ElTile<N, R> T;
+  if constexpr (!YIN) {
+    ef_stage<N, T::H>(op.dx, op.dy, op.G0, x, X, gx0, gy0);
+  } else {
+    const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
+    const double* src[3];
+    int bytes[3];
+    const double* row0 = x + (size_t)(gy0 - N - op.dy.lo + warp) * op.G0;
+#pragma unroll
+    for (int q = 0; q < 3; q++) {
+      const int cu = lane + 32 * q < T::SW ? unk(op.dx, gx0 - N + lane + 32 * q) : -1;
+      src[q] = row0 + max(cu, 0);
+      bytes[q] = cu >= 0 ? 8 : 0;
+    }
+    unsigned dst = (unsigned)__cvta_generic_to_shared(X + warp * T::W + lane);
+    const size_t step = (size_t)kEfWarps * op.G0;
+#pragma unroll
+    for (int r = 0; r < (T::H + kEfWarps - 1) / kEfWarps; r++) {
+      if (r < T::H / kEfWarps || warp + r * kEfWarps < T::H) {
+#pragma unroll
+        for (int q = 0; q < 3; q++) {
+          if (lane + 32 * q < T::SW)
+            asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(dst + 256 * q),
+                         "l"(src[q]), "r"(bytes[q]));
+          src[q] += step;
+        }
+      }
+      dst += kEfWarps * T::W * 8;
+    }
+    asm volatile("cp.async.commit_group;\n" ::);
+    asm volatile("cp.async.wait_group 0;\n" ::);
+  }
 }
-template <int N, class TI>
+template <int N, int R, bool YIN, class TI>
 __device__ __forceinline__ void stage_general(const ElArgs<N, float>& op, const TI* x, float* X,
                                               int gx0, int gy0) {
-  typedef EfTile<N> T;
-  constexpr int W = (T::SW + 3) | 1, R = (T::H + kEfWarps - 1) / kEfWarps;
+  typedef ElTile<N, R> T;
+  constexpr int W = (T::SW + 3) | 1, Q = (T::H + kEfWarps - 1) / kEfWarps;
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
   int cu[3];
 #pragma unroll
   for (int q = 0; q < 3; q++)
     cu[q] = lane + 32 * q < T::SW ? unk(op.dx, gx0 - N + lane + 32 * q) : -1;
-  TI v[R][3];
+  const TI* row = x + (YIN ? (size_t)(gy0 - N - op.dy.lo + warp) * op.G0 : 0);
+  const size_t step = (size_t)kEfWarps * op.G0;
+  TI v[Q][3];
 #pragma unroll
-  for (int r = 0; r < R; r++) {
-    const int j = warp + r * kEfWarps, uy = j < T::H ? unk(op.dy, gy0 - N + j) : -1;
-    const TI* row = x + (size_t)(uy < 0 ? 0 : uy) * op.G0;
-#pragma unroll
-    for (int q = 0; q < 3; q++) v[r][q] = uy >= 0 && cu[q] >= 0 ? row[cu[q]] : TI(0.f);
-  }
-#pragma unroll
-  for (int r = 0; r < R; r++) {
+  for (int r = 0; r < Q; r++) {
     const int j = warp + r * kEfWarps;
+    bool in = j < T::H;
+    if constexpr (!YIN) {
+      const int uy = in ? unk(op.dy, gy0 - N + j) : -1;
+      in = uy >= 0;
+      row = x + (size_t)(in ? uy : 0) * op.G0;
+    }
 #pragma unroll
-    for (int q = 0; q < 3; q++)
-      if (j < T::H && lane + 32 * q < T::SW) X[j * W + lane + 32 * q] = to_a(v[r][q], 0.f);
+    for (int q = 0; q < 3; q++) v[r][q] = in && cu[q] >= 0 ? row[cu[q]] : TI(0.f);
+    if constexpr (YIN) row += step;
+  }
+  float* dst = X + warp * W + lane;
+#pragma unroll
+  for (int r = 0; r < Q; r++) {
+    if (warp + r * kEfWarps < T::H) {
+#pragma unroll
+      for (int q = 0; q < 3; q++)
+        if (lane + 32 * q < T::SW) dst[32 * q] = to_a(v[r][q], 0.f);
+    }
+    dst += kEfWarps * W;
   }
 }
 
 // Row and column passes on the staged tile (row j, column i at X[j * W + i]).
-template <int N, class A, class TO, int W, bool INTERIOR>
+// XIN, YIN: along x, y every output is an unknown and every element and its
+// left (lower) neighbour exists.
+template <int N, int R, class A, class TO, int W, bool XIN, bool YIN>
 __device__ __forceinline__ void el_passes(const ElArgs<N, A>& op, const A* X, A* OX, const A* sw,
                                           int gx0, int gy0, TO* __restrict__ y) {
-  typedef EfTile<N> T;
+  typedef ElTile<N, R> T;
   constexpr int OXP = T::OXP, TX = T::TX, TY = T::TY;
   const int tid = threadIdx.x;
-  if (tid < T::ITEMS) {  // item = (element e, row r)
-    const int r = tid % TY, e = tid / TY;
+#pragma unroll
+  for (int q = 0; q < R; q++) {  // item = (element e, row r)
+    const int it = tid + q * kEfThreads, r = it % TY, e = it / TY;
+    // an item past the mesh's end has no output
+    if (it >= T::ITEMS || (!XIN && gx0 + e * N >= op.dx.hi) || (!YIN && gy0 + r >= op.dy.hi)) continue;
     const A* row = X + (r + N) * W + e * N;  // left element's first node
     A l[N], v[N + 1], o[N + 1];
 #pragma unroll
@@ -319,17 +379,21 @@ __device__ __forceinline__ void el_passes(const ElArgs<N, A>& op, const A* X, A*
 #pragma unroll
     for (int k = 0; k < N; k++) t = fma(op.lx[k], l[k], t);
     A wy;
-    if constexpr (INTERIOR) {
+    if constexpr (XIN) {
       o[0] += t;
-      wy = sw[r % N];
     } else {
-      const int ex = gx0 / N + e, ey = gy0 / N + r / N, a = r % N;
+      const int ex = gx0 / N + e;
       const bool own = ex < op.dx.nE, left = ex > 0 || op.dx.periodic;
       if (!own) {
 #pragma unroll
         for (int k = 0; k < N; k++) o[k] = A(0);
       }
       if (left && ex <= op.dx.nE) o[0] += t;
+    }
+    if constexpr (YIN) {
+      wy = sw[r % N];
+    } else {
+      const int ey = gy0 / N + r / N, a = r % N;
       wy = (ey < op.dy.nE ? op.w[a] : A(0)) +
            (a == 0 && (ey > 0 || op.dy.periodic) ? op.w[N] : A(0));
     }
@@ -337,8 +401,12 @@ __device__ __forceinline__ void el_passes(const ElArgs<N, A>& op, const A* X, A*
     for (int a = 0; a < N; a++) OX[r * OXP + e * N + a] = wy * o[a];
   }
   __syncthreads();
-  if (tid < T::ITEMS) {  // item = (element row e, column c), consecutive columns per warp
-    const int c = tid % TX, e = tid / TX;
+#pragma unroll
+  for (int q = 0; q < R; q++) {  // item = (element row e, column c), consecutive columns per warp
+    const int it = tid + q * kEfThreads, c = it % TX, e = it / TX;
+    if (it >= T::ITEMS) continue;
+    if (!XIN && (gx0 + c < op.dx.lo || gx0 + c >= op.dx.hi)) continue;
+    if (!YIN && gy0 + e * N >= op.dy.hi) continue;
     const A* col = X + (e * N) * W + c + N;  // lower element's first node
     A l[N], v[N + 1], o[N + 1];
 #pragma unroll
@@ -351,9 +419,16 @@ __device__ __forceinline__ void el_passes(const ElArgs<N, A>& op, const A* X, A*
     for (int k = 0; k < N; k++) t = fma(op.ly[k], l[k], t);
     const A* oxp = OX + (e * N) * OXP + c;
     // y = wx (alpha wy x + beta_y (Ky x)) + wy beta_x (Kx x)
-    if constexpr (INTERIOR) {
+    A wx;
+    if constexpr (XIN) {
+      wx = sw[c % N];
+    } else {
+      const int gx = gx0 + c, ex = gx / N, b = gx % N;
+      wx = (ex < op.dx.nE ? op.w[b] : A(0)) +
+           (b == 0 && (ex > 0 || op.dx.periodic) ? op.w[N] : A(0));
+    }
+    if constexpr (YIN) {
       o[0] += t;
-      const A wx = sw[c % N];
       const size_t ld = (size_t)op.G0;
       TO* yp = y + (size_t)(gy0 + e * N - op.dy.lo) * ld + (gx0 + c - op.dx.lo);
 #pragma unroll
@@ -363,16 +438,13 @@ __device__ __forceinline__ void el_passes(const ElArgs<N, A>& op, const A* X, A*
         yp += ld;
       }
     } else {
-      const int ey = gy0 / N + e, gx = gx0 + c, ex = gx / N, b = gx % N;
+      const int ey = gy0 / N + e;
       const bool own = ey < op.dy.nE, low = (ey > 0 || op.dy.periodic) && ey <= op.dy.nE;
       if (!own) {
 #pragma unroll
         for (int k = 0; k < N; k++) o[k] = A(0);
       }
       if (low) o[0] += t;
-      if (gx < op.dx.lo || gx >= op.dx.hi) return;
-      const A wx = (ex < op.dx.nE ? op.w[b] : A(0)) +
-                   (b == 0 && (ex > 0 || op.dx.periodic) ? op.w[N] : A(0));
 #pragma unroll
       for (int a = 0; a < N; a++) {
         const int gy = gy0 + e * N + a;
@@ -380,7 +452,7 @@ __device__ __forceinline__ void el_passes(const ElArgs<N, A>& op, const A* X, A*
         if (a == 0) wa = (own ? op.w[0] : A(0)) + (low ? op.w[N] : A(0));
         const A r = fma(wx, fma(op.alpha * wa, v[a], o[a]), oxp[a * OXP]);
         if (gy >= op.dy.lo && gy < op.dy.hi)
-          y[(size_t)(gy - op.dy.lo) * op.G0 + (gx - op.dx.lo)] = (TO)r;
+          y[(size_t)(gy - op.dy.lo) * op.G0 + (gx0 + c - op.dx.lo)] = (TO)r;
       }
     }
   }
@@ -388,11 +460,11 @@ __device__ __forceinline__ void el_passes(const ElArgs<N, A>& op, const A* X, A*
 
 // quads: x in 16 bits with rows a multiple of four long and an 8-byte aligned
 // base. y0: the first row of vertices of this launch.
-template <int N, class TI, class A, class TO, int MINB>
+template <int N, int R, class TI, class A, class TO, int MINB>
 __global__ void __launch_bounds__(kEfThreads, MINB)
     apply_el_kernel(const __grid_constant__ ElArgs<N, A> op, const TI* __restrict__ x,
                     TO* __restrict__ y, int quads, int y0) {
-  typedef EfTile<N> T;
+  typedef ElTile<N, R> T;
   constexpr bool LOW = sizeof(TI) != sizeof(A);
   constexpr int W = LOW ? (T::SW + 3) | 1 : T::W;
   extern __shared__ __align__(16) unsigned char el_smem[];
@@ -412,22 +484,28 @@ __global__ void __launch_bounds__(kEfThreads, MINB)
     if (last + (T::SW + 6) / 4 * 4 > (size_t)op.G0 * op.G1) interior = false;
   }
   if (interior) {
-    stage_interior<N>(op, x, X, gx0, gy0, LOW && quads ? shift + 1 : 0);
+    stage_interior<N, R>(op, x, X, gx0, gy0, LOW && quads ? shift + 1 : 0);
   } else {
     shift = 0;
-    stage_general<N>(op, x, X, gx0, gy0);
+    if (inside(op.dy, gy0 - N, gy0 + T::TY))
+      stage_general<N, R, true>(op, x, X, gx0, gy0);
+    else
+      stage_general<N, R, false>(op, x, X, gx0, gy0);
   }
   __syncthreads();
   // (a tile at a periodic seam has general staging and plain passes)
-  if (all_outputs(op.dx, gx0, T::TX) && all_outputs(op.dy, gy0, T::TY))
-    el_passes<N, A, TO, W, true>(op, X + shift, OX, sw, gx0, gy0, y);
+  const bool xin = all_outputs(op.dx, gx0, T::TX), yin = all_outputs(op.dy, gy0, T::TY);
+  if (xin && yin)
+    el_passes<N, R, A, TO, W, true, true>(op, X + shift, OX, sw, gx0, gy0, y);
+  else if (yin)
+    el_passes<N, R, A, TO, W, false, true>(op, X, OX, sw, gx0, gy0, y);
   else
-    el_passes<N, A, TO, W, false>(op, X, OX, sw, gx0, gy0, y);
+    el_passes<N, R, A, TO, W, false, false>(op, X, OX, sw, gx0, gy0, y);
 }
 
-template <int N, class TI, class A, class TO>
-cudaError_t launch_el(const OpDev& od, const TI* x, TO* y, cudaStream_t s) {
-  typedef EfTile<N> T;
+template <int N, int R, class TI, class A, class TO>
+cudaError_t launch_tile(const OpDev& od, const TI* x, TO* y, cudaStream_t s) {
+  typedef ElTile<N, R> T;
   constexpr bool LOW = sizeof(TI) != sizeof(A);
   constexpr int W = LOW ? (T::SW + 3) | 1 : T::W;
   // blocks per SM: the most without spills and with no kernel slower (bf16,
@@ -454,7 +532,7 @@ cudaError_t launch_el(const OpDev& od, const TI* x, TO* y, cudaStream_t s) {
     if (e != cudaSuccess) return e;
     if (dev < 0 || dev >= 64) return cudaErrorInvalidDevice;
     if (!attr[dev]) {
-      e = cudaFuncSetAttribute(apply_el_kernel<N, TI, A, TO, MINB>,
+      e = cudaFuncSetAttribute(apply_el_kernel<N, R, TI, A, TO, MINB>,
                                cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
       if (e != cudaSuccess) return e;
       attr[dev] = true;
@@ -464,9 +542,23 @@ cudaError_t launch_el(const OpDev& od, const TI* x, TO* y, cudaStream_t s) {
   const int rows = (od.d[1].hi + T::TY - 1) / T::TY;
   for (int r = 0; r < rows; r += kGridRows) {
     const dim3 grid((od.d[0].hi + T::TX - 1) / T::TX, std::min(rows - r, kGridRows));
-    apply_el_kernel<N, TI, A, TO, MINB><<<grid, kEfThreads, smem, s>>>(op, x, y, quads, r * T::TY);
+    apply_el_kernel<N, R, TI, A, TO, MINB><<<grid, kEfThreads, smem, s>>>(op, x, y, quads, r * T::TY);
   }
   return cudaGetLastError();
+}
+
+template <int N, class TI, class A, class TO>
+cudaError_t launch_el(const OpDev& od, const TI* x, TO* y, cudaStream_t s) {
+  // Four times the rows a tile where that leaves a wave of blocks: a 16-bit
+  // tile of a low order has little work beside its fixed costs. Order 2 at
+  // 2000 x 2000 elements 40 us against 60; order 4 in a mesh of one tile's
+  // width, 5 x 30,000 elements, 14.4 us against 20.5.
+  if constexpr (sizeof(TI) != sizeof(A) && N <= 4) {
+    typedef ElTile<N, 1> T;
+    const long tx = (od.d[0].hi + T::TX - 1) / T::TX, ty = (od.d[1].hi + T::TY - 1) / T::TY;
+    if ((N == 2 || tx == 1) && tx * ty > 8 * kSms) return launch_tile<N, 4, TI, A, TO>(od, x, y, s);
+  }
+  return launch_tile<N, 1, TI, A, TO>(od, x, y, s);
 }
 
 // ------------------------------- refinement residual, orders 4 to 8 ----

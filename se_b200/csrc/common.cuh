@@ -101,6 +101,7 @@ __device__ __forceinline__ void dd_fma(double& hi, double& lo, double a, double 
   lo += pe;
 }
 
+constexpr int kSms = 148;  // of a B200
 // Largest y extent of a grid: more rows of blocks take several launches.
 constexpr int kGridRows = 65535;
 

@@ -131,3 +131,41 @@ def test_tallest_meshes(segpu, N, ny):
     scale = float(x.abs().max()) * 4.0 * (3.0 * gw.max() ** 2 / 4 + Kh.sum(1).max() * gw.max())
     assert float((y + r).abs().max()) <= 64 * 2.0 ** -53 * scale
     assert float((yf.double() + r).abs().max()) <= 64 * 2.0 ** -24 * scale
+
+
+# 16-bit tiles of orders 2 to 4 four times as high (from 1184 tiles on; wide
+# meshes of order 2, others one tile wide), the last tile cut short, rows of a
+# multiple of four unknowns and not; order 5 just as narrow on the plain tile
+TALL = [(2, 33, 2370, P), (2, 100, 1187, P), (2, 101, 1186, "nat"), (2, 9, 4799, BOX),
+        (3, 20, 4741, CH), (3, 1, 4745, BOX), (4, 15, 4747, BOX), (4, 16, 4739, P), (5, 7, 4741, CH)]
+
+
+@pytest.mark.parametrize("case", range(len(TALL)))
+def test_tall_tiles(segpu, case):
+    """FP64 and 16-bit applies against the residual's kernel, as above."""
+    import torch
+    N, nx, ny, per = TALL[case]
+    walls = WALLS[per]
+    m = segpu.Mesh("m", [nx, ny], "legendre", N, [0.0, 0.0], [1.0, ny / nx],
+                   list(BOX if per == "nat" else per))
+    u = segpu.Field("u", m, 1, segpu.BCs(*walls, m))
+    ls = segpu.HelmholtzEqn(u, None, -3.0, -1.0, 0.5, 0, segpu.solver_opts(mode=segpu.MODE_EXACT))
+    n = ls.vecSize
+    gx, gw, D = m.gll()
+    Kh = np.abs(D.T @ np.diag(gw) @ D)
+    hx = 1.0 / nx
+    for dt, prec in ((torch.bfloat16, segpu.PREC_BF16), (torch.float16, segpu.PREC_FP16)):
+        xl = torch.randn(n, device="cuda", generator=torch.Generator("cuda").manual_seed(case)).to(dt)
+        x = xl.double()
+        y, r, zero = (torch.zeros(n, device="cuda", dtype=torch.float64) for _ in range(3))
+        y.fill_(float("nan"))
+        yf = torch.full((n + 2,), float("nan"), device="cuda")
+        torch.cuda.synchronize()
+        ls.residual(x.data_ptr(), zero.data_ptr(), r.data_ptr())
+        ls.apply(x.data_ptr(), y.data_ptr())
+        ls.apply_low(xl.data_ptr(), yf.data_ptr() + 4, prec)
+        segpu.synchronize()
+        scale = float(x.abs().max()) * 4.0 * (3.0 * (gw.max() * hx) ** 2 / 4 + Kh.sum(1).max() * gw.max())
+        assert float((y + r).abs().max()) <= 64 * 2.0 ** -53 * scale
+        assert bool(yf[0].isnan()) and bool(yf[-1].isnan())
+        assert float((yf[1:-1].double() + r).abs().max()) <= 64 * 2.0 ** -24 * scale
