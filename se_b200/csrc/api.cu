@@ -239,7 +239,7 @@ struct se_advector {
   bool record;
 };
 namespace {
-struct Eig1D;
+struct EigForm;
 }
 struct se_linsys {
   se_field *sol, *rhs;
@@ -280,7 +280,7 @@ struct se_linsys {
   int fdm_lbuf_prec;          // precision the L2, L3 buffers were sized for
   double *X1, *X2, *ax;       // FP64 work: two transform buffers, A x
   double* zlow;               // FP64 inverse: the low modes' block [kFdmLow][kFdmLow]
-  const Eig1D *eigx, *eigy;   // FP64 inverse: the directions' folded blocks (cached, shared)
+  const EigForm *eigx, *eigy;  // FP64 inverse: the directions' factors (cached, shared)
   // FP64 inverse of a doubly periodic system with 2^k elements per
   // direction: Bloch form (bloch.cu) with its complex spectral work array
   bool bloch;
@@ -1104,11 +1104,11 @@ int eig_pair(int n, const std::vector<double>& K, const std::vector<double>& W,
 
 // A direction is its own mirror image when it is periodic or both its ends
 // are of one kind: all elements are equal and the GLL nodes symmetric.
-FoldDir fold_of(const Dir& d) {
+FoldDir fold_of(const Dir& d, bool fold = true) {
   FoldDir f;
   f.n = d.hi - d.lo;
   f.periodic = d.periodic != 0;
-  f.on = f.n > 1 && (d.periodic || d.lo == d.nV - d.hi);
+  f.on = fold && f.n > 1 && (d.periodic || d.lo == d.nV - d.hi);
   f.ge = !f.on ? f.n : f.periodic ? f.n / 2 + 1 : (f.n + 1) / 2;
   f.go = f.n - f.ge;
   f.os = (f.ge + 1) & ~1;
@@ -1119,25 +1119,14 @@ int fold_mirror(const FoldDir& f, int i) {
   return f.periodic ? (i == 0 ? 0 : f.n - i) : f.n - 1 - i;
 }
 
-// The eigenpairs of one direction: full eigenvectors E (column-major,
-// ascending eigenvalues lam) and, folded (FoldDir), the even then the odd
-// modes' blocks on the half direction, FE row-major (entry (i, m)), FT their
-// transposes (rows at the pitch FoldDir gives), lamF their eigenvalues by slot. A folded block is the pair's own
-// eigenproblem on the sums (differences) of mirrored unknowns: K and W summed
-// over the mirrored entries (with the odd part's signs), which has no
-// degenerate pairs (a periodic direction's sine and cosine modes fall into
-// different blocks) and an eighth of the work each.
-int eig_1d(const Dir& d, const double* Kh, const double* w, std::vector<double>& E,
-           std::vector<double>& lam, std::vector<double>& FE, std::vector<double>& FT,
-           std::vector<double>& lamF) {
-  std::vector<double> K, W;
-  assemble_1d(d, Kh, w, K, W);
-  const FoldDir f = fold_of(d);
-  const int n = f.n;
-  FE.clear();
-  FT.clear();
-  lamF.clear();
-  auto append = [&](int m, const std::vector<double>& A, const std::vector<double>& l) {
+// One direction's factors for the FP64 inverse: the even then the odd modes'
+// blocks on the half direction (or, not folded, the whole matrix), FE
+// row-major (entry (i, m)), FT their transposes, rows at the pitch FoldDir
+// gives, lamF the eigenvalues by slot.
+struct Factors {
+  std::vector<double> FE, FT, lamF;
+  // appends the block of m modes, A column-major, eigenvalues l
+  void append(int m, const std::vector<double>& A, const std::vector<double>& l) {
     for (int i = 0; i < m; i++) {
       for (int j = 0; j < m; j++) FE.push_back(A[(size_t)j * m + i]);
       FT.insert(FT.end(), A.begin() + (size_t)i * m, A.begin() + (size_t)(i + 1) * m);
@@ -1148,10 +1137,23 @@ int eig_1d(const Dir& d, const double* Kh, const double* w, std::vector<double>&
     }
     lamF.insert(lamF.end(), l.begin(), l.end());
     if (m & 1) lamF.push_back(1.0);  // an empty slot
-  };
+  }
+};
+
+// The eigenpairs of one direction: full eigenvectors E (column-major,
+// ascending eigenvalues lam) and the factors of the direction folded as f. A
+// folded block is the pair's own eigenproblem on the sums (differences) of
+// mirrored unknowns: K and W summed over the mirrored entries (with the odd
+// part's signs), which has no degenerate pairs (a periodic direction's sine
+// and cosine modes fall into different blocks) and an eighth of the work each.
+int eig_1d(const Dir& d, const FoldDir& f, const double* Kh, const double* w, std::vector<double>& E,
+           std::vector<double>& lam, Factors& F) {
+  std::vector<double> K, W;
+  assemble_1d(d, Kh, w, K, W);
+  const int n = f.n;
   if (!f.on) {
     if (int rc = eig_pair(n, K, W, E, lam)) return rc;
-    append(n, E, lam);
+    F.append(n, E, lam);
     return SE_OK;
   }
   std::vector<std::pair<double, int>> order;  // eigenvalue, mode (even then odd)
@@ -1182,7 +1184,7 @@ int eig_1d(const Dir& d, const double* Kh, const double* w, std::vector<double>&
         Kp[(size_t)a * m + b] = Kp[(size_t)b * m + a] = v;
       }
     if (int rc = eig_pair(m, Kp, Wp, A, l)) return rc;
-    append(m, A, l);
+    F.append(m, A, l);
     for (int k = 0; k < m; k++) {
       const int mode = (part ? f.ge : 0) + k;
       order.push_back({l[k], mode});
@@ -1230,17 +1232,21 @@ int upload_low(const std::vector<double>& S, int prec, void** out) {
 // and the boundary ends of a direction (not on h, the coefficients or the
 // Laplacian scaling), so every system with the same direction shares one
 // setup; entries live until the process exits.
+struct EigForm {
+  FoldDir fold;
+  FdmLowMap lowmap;
+  // the factors and eigenvalues (Factors) and the low modes' eigenvectors [n][kFdmLow]
+  double *FE = nullptr, *FT = nullptr, *lamF = nullptr, *low8 = nullptr;
+};
 struct Eig1D {
   int n = 0;
   double* S = nullptr;    // W-orthonormal eigenvectors E, column-major (= row-major E^T)
   double* ST = nullptr;   // row-major E
   double* lam = nullptr;  // eigenvalues
   double lmax = 0.0;
-  // FP64 inverse: the folded direction's blocks, their eigenvalues and the
-  // low modes' eigenvectors [n][kFdmLow]
-  FoldDir fold;
-  double *FE = nullptr, *FT = nullptr, *lamF = nullptr, *low8 = nullptr;
-  FdmLowMap lowmap;
+  // FP64 inverse: the direction folded where it can be, and whole where it
+  // cannot or is short (kPlainMax)
+  EigForm folded, plain;
   void* low[3] = {nullptr, nullptr, nullptr};   // [1] FP32, [2] BF16 copies of S
   void* lowT[3] = {nullptr, nullptr, nullptr};  // and of ST
   // TF32 hi/lo pairs for the tcgen05 products, rows padded to tc_pitch:
@@ -1251,6 +1257,31 @@ struct Eig1D {
 typedef std::tuple<int, int, int, int, int, int> EigKey;
 std::mutex g_eig_mu;
 std::map<EigKey, Eig1D*> g_eig[64];
+
+// Longest direction kept whole beside its folded form.
+constexpr int kPlainMax = 256;
+
+int upload_form(EigForm& e, const FoldDir& f, const Factors& F) {
+  e.fold = f;
+  e.lowmap = f.on ? FdmLowMap{std::min(kFdmLow / 2, f.ge), std::min(kFdmLow / 2, f.go), f.os}
+                  : FdmLowMap{std::min(kFdmLow, f.n), 0, f.os};
+  std::vector<double> low((size_t)f.n * kFdmLow, 0.0);
+  for (int k = 0; k < e.lowmap.even; k++)
+    for (int i = 0; i < f.ge; i++) low[(size_t)i * kFdmLow + k] = F.FE[(size_t)i * f.os + k];
+  for (int k = 0; k < e.lowmap.odd; k++)
+    for (int a = 0; a < f.go; a++)
+      low[(size_t)(a + (f.periodic ? 1 : 0)) * kFdmLow + kFdmLow / 2 + k] =
+          F.FE[(size_t)f.ge * f.os + (size_t)a * (f.len - f.os) + k];
+  auto up = [&](double** dst, const std::vector<double>& v) -> int {
+    if (int r = dalloc(dst, v.size())) return r;
+    CK(upload_now(*dst, v.data(), sizeof(double) * v.size()));
+    return SE_OK;
+  };
+  int rc;
+  (void)((rc = up(&e.FE, F.FE)) || (rc = up(&e.FT, F.FT)) || (rc = up(&e.lamF, F.lamF)) ||
+         (rc = up(&e.low8, low)));
+  return rc;
+}
 
 int eig_get(const Dir& d, const double* Kh, const double* w, int prec, Eig1D** out) {
   int dev = 0;
@@ -1263,36 +1294,34 @@ int eig_get(const Dir& d, const double* Kh, const double* w, int prec, Eig1D** o
   if (!e) {
     Eig1D* ne = new Eig1D();
     const int n = ne->n = d.hi - d.lo;
-    std::vector<double> lam, FE, FT, lamF;
-    int rc = eig_1d(d, Kh, w, Sh, lam, FE, FT, lamF);
+    std::vector<double> lam;
+    Factors F;
+    const FoldDir f = fold_of(d);
+    int rc = eig_1d(d, f, Kh, w, Sh, lam, F);
     if (!rc) {
       for (double v : lam) ne->lmax = std::max(ne->lmax, std::fabs(v));
-      const FoldDir f = ne->fold = fold_of(d);
-      ne->lowmap = f.on ? FdmLowMap{std::min(kFdmLow / 2, f.ge), std::min(kFdmLow / 2, f.go), f.os}
-                        : FdmLowMap{std::min(kFdmLow, n), 0, f.os};
-      std::vector<double> T((size_t)n * n), low((size_t)n * kFdmLow, 0.0);
+      std::vector<double> T((size_t)n * n);
       for (int j = 0; j < n; j++)
         for (int i = 0; i < n; i++) T[(size_t)i * n + j] = Sh[(size_t)j * n + i];
-      const FdmLowMap& lm = ne->lowmap;
-      for (int k = 0; k < lm.even; k++)
-        for (int i = 0; i < f.ge; i++) low[(size_t)i * kFdmLow + k] = FE[(size_t)i * f.os + k];
-      const int go = f.go;
-      for (int k = 0; k < lm.odd; k++)
-        for (int a = 0; a < go; a++)
-          low[(size_t)(a + (f.periodic ? 1 : 0)) * kFdmLow + kFdmLow / 2 + k] =
-              FE[(size_t)f.ge * f.os + (size_t)a * (f.len - f.os) + k];
       auto up = [&](double** dst, const std::vector<double>& v) -> int {
         if (int r = dalloc(dst, v.size())) return r;
         CK(upload_now(*dst, v.data(), sizeof(double) * v.size()));
         return SE_OK;
       };
       (void)((rc = up(&ne->S, Sh)) || (rc = up(&ne->ST, T)) || (rc = up(&ne->lam, lam)) ||
-             (rc = up(&ne->FE, FE)) || (rc = up(&ne->FT, FT)) || (rc = up(&ne->lamF, lamF)) ||
-             (rc = up(&ne->low8, low)));
+             (rc = upload_form(f.on ? ne->folded : ne->plain, f, F)));
+      if (!rc && f.on && n <= kPlainMax) {
+        Factors P;
+        P.append(n, Sh, lam);
+        rc = upload_form(ne->plain, fold_of(d, false), P);
+      }
     }
     if (rc) {
-      for (double* p : {ne->S, ne->ST, ne->lam, ne->FE, ne->FT, ne->lamF, ne->low8})
+      for (double* p : {ne->S, ne->ST, ne->lam})
         if (p) cudaFree(p);
+      for (const EigForm& e : {ne->folded, ne->plain})
+        for (double* p : {e.FE, e.FT, e.lamF, e.low8})
+          if (p) cudaFree(p);
       delete ne;
       g_eig[dev].erase(key);
       return rc;
@@ -1473,6 +1502,22 @@ int bloch_get(const Dir& d, const double* Kh, const double* w, Bloch1D** out) {
   return SE_OK;
 }
 
+// Whether the FP64 inverse of two directions folds. Folding halves the
+// products of a direction that is its own mirror image and costs two passes
+// over the array, two launches. Measured, a call of the inverse folded and
+// not: both directions, 3,381 unknowns 27.8 us and 24.7, 5,184 28.3 and 25.6
+// (in a solve's graph 18.6 and 17.8, the solve 67.7 and 69.8), 32,041 35.9
+// and 28.8 (20.8 and 23.0), 600,625 173 and 298; one direction, 22,350 33.9
+// and 28.8 (21.8 and 21.8), 46,440 35.9 and 34.0 (24.1 and 25.8), 601,400 238
+// and 289. Neither: 602,176 unknowns 315 us through the two passes, 291 without.
+constexpr long kFoldBoth = 4096, kFoldOne = 32768;
+bool fdm_folds(const Eig1D& x, const Eig1D& y) {
+  if (!x.plain.FE || !y.plain.FE) return true;
+  const long n = (long)x.n * y.n;
+  const bool fx = x.folded.FE, fy = y.folded.FE;
+  return fx && fy ? n > kFoldBoth : (fx || fy) && n > kFoldOne;
+}
+
 int fdm_setup(se_linsys* ls, int prec) {
   if (ls->svv)
     return fail(SE_ERR_UNSUPPORTED, "the SVV operator needs SE_METHOD_CG (no fast diagonalization)");
@@ -1489,8 +1534,9 @@ int fdm_setup(se_linsys* ls, int prec) {
   ls->SyT = ey->ST;
   ls->lx = ex->lam;
   ls->ly = ey->lam;
-  ls->eigx = ex;
-  ls->eigy = ey;
+  const bool folds = fdm_folds(*ex, *ey);
+  ls->eigx = folds && ex->folded.FE ? &ex->folded : &ex->plain;
+  ls->eigy = folds && ey->folded.FE ? &ey->folded : &ey->plain;
   ls->lmax[0] = ex->lmax;
   ls->lmax[1] = ey->lmax;
   ls->Sx_lo = prec ? ex->low[prec] : nullptr;
@@ -1499,7 +1545,7 @@ int fdm_setup(se_linsys* ls, int prec) {
   ls->SyT_lo = prec ? ey->lowT[prec] : nullptr;
   if (!ls->X1) {
     ls->fpart_n = std::max(kFdmPartials, std::max(residual_blocks(op), residual_partial_blocks(op)));
-    const size_t nf = (size_t)ex->fold.len * ey->fold.len;
+    const size_t nf = (size_t)ls->eigx->fold.len * ls->eigy->fold.len;
     if ((rc = dalloc(&ls->X1, nf)) || (rc = dalloc(&ls->X2, nf)) || (rc = dalloc(&ls->ax, n)) ||
         (rc = dalloc(&ls->zlow, kFdmLow * kFdmLow)) || (rc = dalloc(&ls->fpart, 2 * (size_t)ls->fpart_n + 16)))
       return rc;
@@ -1570,8 +1616,10 @@ double null_tol(const se_linsys* ls) {
 // Ey ((.) Ex^T), the divide fused into the second product's epilogue. The
 // array is folded first (launch_fdm_fold), so that a mirror-symmetric
 // direction's factors are two blocks of half the size, and unfolded into the
-// output. The low modes of both directions skip the backward products: the
-// divide moves them to zlow and the unfolding adds them in double-double. For
+// output; where that does not pay (fdm_folds) the first product reads the
+// input and the last one writes the output. The low modes of both directions
+// skip the backward products: the divide moves them to zlow, and the unfolding
+// or the last product adds them in double-double. For
 // a smooth solution they hold the largest coefficients, so the FP64 rounding
 // of the backward products does not set the first step's residual (with
 // refined eigenvectors one step reaches about 3e-11 of the right-hand side in
@@ -1588,11 +1636,14 @@ int fdm_apply64(se_linsys* ls, const double* in, double* out, bool accumulate,
                             accumulate, ls->xh, gate, g_stream));
     return SE_OK;
   }
-  const Eig1D &ex = *ls->eigx, &ey = *ls->eigy;
+  const EigForm &ex = *ls->eigx, &ey = *ls->eigy;
+  const bool folds = ex.fold.on || ey.fold.on;
+  const int* closed = gate ? &gate->reason : nullptr;
   FdmProduct p;
   std::memset(&p, 0, sizeof(p));
   p.x = ex.fold;
   p.y = ey.fold;
+  p.ldc = ex.fold.len;
   auto product = [&](int which, const double* A, const double* B, double* C) {
     p.which = which;
     p.A = A;
@@ -1600,8 +1651,12 @@ int fdm_apply64(se_linsys* ls, const double* in, double* out, bool accumulate,
     p.C = C;
     return launch_fdm_dgemm(p, g_stream);
   };
-  CK(launch_fdm_fold(ex.fold, ey.fold, in, ls->X2, gate ? &gate->reason : nullptr, g_stream));
-  CK(product(FDM_FACTOR_B, ls->X2, ex.FE, ls->X1));
+  if (folds) CK(launch_fdm_fold(ex.fold, ey.fold, in, ls->X2, closed, g_stream));
+  p.lda = folds ? ex.fold.len : ex.fold.n;
+  p.gate = folds ? nullptr : closed;
+  CK(product(FDM_FACTOR_B, folds ? ls->X2 : in, ex.FE, ls->X1));
+  p.lda = ex.fold.len;
+  p.gate = nullptr;
   p.lx = ex.lamF;
   p.ly = ey.lamF;
   p.alpha = op.alpha;
@@ -1613,8 +1668,15 @@ int fdm_apply64(se_linsys* ls, const double* in, double* out, bool accumulate,
   p.low_r = ey.lowmap;
   CK(product(FDM_FACTOR_A, ey.FT, ls->X1, ls->X2));
   p.lx = p.ly = nullptr;
-  p.zlow = nullptr;
   CK(product(FDM_FACTOR_B, ls->X2, ex.FT, ls->X1));
+  if (!folds) {
+    p.ldc = ex.fold.n;
+    p.low_x = ex.low8;
+    p.low_y = ey.low8;
+    p.accumulate = accumulate;
+    CK(product(FDM_FACTOR_A, ey.FE, ls->X1, out));
+    return SE_OK;
+  }
   CK(product(FDM_FACTOR_A, ey.FE, ls->X1, ls->X2));
   CK(launch_fdm_unfold(ex.fold, ey.fold, ls->X2, out, accumulate, ls->zlow, ex.low8, ey.low8,
                        g_stream));

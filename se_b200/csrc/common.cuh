@@ -452,16 +452,24 @@ struct FdmLowMap {
 // C = A B on folded arrays ([y.len][x.len]) in FP64, one operand the factor of
 // a direction (`which`: B that of x, or A that of y); with lx the spectral
 // divide by alpha + bx lx[col] + by ly[row] (|divisor| <= null_tol gives 0)
-// and, with zlow, the low modes moved into zlow[8][8] (0 left in C).
+// and, with zlow, the low modes moved into zlow[8][8] (0 left in C); zeros
+// when gate && *gate != 0. Where no direction is folded the first product can
+// read the caller's array (lda, any alignment) and the last write it (ldc):
+// with low_y, C (= or +=, accumulate) gets A B + sum_ab low_y[row][a]
+// zlow[a][b] low_x[col][b], the low modes' eigenvectors ([n][8]), in
+// double-double, rounded once.
 struct FdmProduct {
   const double *A, *B;
   double* C;
   FoldDir x, y;
-  int which;
+  int which, lda, ldc;
+  const int* gate;
   const double *lx, *ly;
   double alpha, bx, by, null_tol;
   double* zlow;
   FdmLowMap low_r, low_c;
+  const double *low_x, *low_y;
+  int accumulate;
 };
 cudaError_t launch_fdm_dgemm(const FdmProduct& p, cudaStream_t s);
 // out ([dy.len][dx.len]) = in ([dy.n][dx.n]) folded along both directions (a

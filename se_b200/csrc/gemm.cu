@@ -32,6 +32,8 @@
 // solve's first residual.
 #include <cuda_bf16.h>
 
+#include <cstdint>
+
 #include "common.cuh"
 
 namespace seg {
@@ -125,12 +127,6 @@ struct GemmArgs {
   const double* cmax;  // accumulate scale, nullptr: 1
   const double *lx, *ly;
   double alpha, bx, by, null_tol;
-  // FP64 only: the folded directions, which operand is a direction's factor,
-  // the low modes
-  FoldDir x, y;
-  int which;
-  double* zlow;
-  FdmLowMap low_r, low_c;
 };
 
 // Place of mode m among the low modes carried apart (-1: not one).
@@ -316,6 +312,15 @@ struct DCfg {
   static constexpr size_t SMEM = (size_t)ST * (A_ELEMS + B_ELEMS) * sizeof(double);
 };
 
+// Epilogues of the FP64 products. D_FIRST stores as D_STORE and reads its A
+// (rows of any pitch and alignment) by 8-byte copies.
+enum { D_STORE = 0, D_FIRST, D_DIVIDE, D_FINISH };
+
+__device__ __forceinline__ void cp_async8(void* smem, const void* gmem, bool valid) {
+  const unsigned sa = (unsigned)__cvta_generic_to_shared(smem);
+  asm volatile("cp.async.ca.shared.global [%0], [%1], 8, %2;\n" ::"r"(sa), "l"(gmem),
+               "r"(valid ? 8 : 0));
+}
 // Copies n (0, 1 or 2) doubles and zeros for the rest of 16 bytes.
 __device__ __forceinline__ void cp_async16(void* smem, const void* gmem, int n) {
   const unsigned sa = (unsigned)__cvta_generic_to_shared(smem);
@@ -335,7 +340,7 @@ struct DTile {
   int m0, n0, m_end, n_end, K, lda, ldb;
 };
 template <int BM, int BN>
-__device__ __forceinline__ DTile tile_of(const GemmArgs<double, double, double>& g) {
+__device__ __forceinline__ DTile tile_of(const FdmProduct& g) {
   const FoldDir &x = g.x, &y = g.y;
   const int nt = (x.ge + BN - 1) / BN, mt = (y.ge + BM - 1) / BM;
   const bool xo = (int)blockIdx.x >= nt, yo = (int)blockIdx.y >= mt;
@@ -344,7 +349,8 @@ __device__ __forceinline__ DTile tile_of(const GemmArgs<double, double, double>&
   t.m0 = yo ? y.os + ((int)blockIdx.y - mt) * BM : (int)blockIdx.y * BM;
   t.n_end = xo ? x.os + x.go : x.ge;
   t.m_end = yo ? y.os + y.go : y.ge;
-  t.lda = t.ldb = x.len;
+  t.lda = g.lda;
+  t.ldb = x.len;
   t.A = g.A;
   t.B = g.B;
   if (g.which == FDM_FACTOR_B) {
@@ -365,16 +371,16 @@ __device__ __forceinline__ DTile tile_of(const GemmArgs<double, double, double>&
   return t;
 }
 template <int BM, int BN>
-dim3 tile_grid(const GemmArgs<double, double, double>& g) {
+dim3 tile_grid(const FdmProduct& g) {
   auto cut = [](const FoldDir& d, int b) { return (d.ge + b - 1) / b + (d.go + b - 1) / b; };
   return dim3(cut(g.x, BN), cut(g.y, BM));
 }
 
 // A stage's operands in 16-byte copies (two values; one and a zero at an odd
 // end, zeros beyond).
-template <class C>
-__device__ __forceinline__ void load_stage(const GemmArgs<double, double, double>& g,
-                                           const DTile& t, int k0, double* as, double* bs) {
+template <class C, int EPI>
+__device__ __forceinline__ void load_stage(const FdmProduct& g, const DTile& t, int k0, double* as,
+                                           double* bs) {
   constexpr int AC = C::BK / 2, BC = C::BN / 2;
   static_assert(C::BM * AC % C::THREADS == 0 && C::BK * BC % C::THREADS == 0 && C::AS % 2 == 0 &&
                     C::BS % 2 == 0, "stage copies");
@@ -383,7 +389,13 @@ __device__ __forceinline__ void load_stage(const GemmArgs<double, double, double
     const int q = threadIdx.x + e * C::THREADS, row = q / AC, col = q % AC * 2;
     const int gr = t.m0 + row, gc = k0 + col;
     const int n = gr < t.m_end ? min(2, t.K - gc) : 0;
-    cp_async16(as + row * C::AS + col, n > 0 ? t.A + (ptrdiff_t)gr * t.lda + gc : g.A, max(n, 0));
+    const double* src = t.A + (ptrdiff_t)gr * t.lda + gc;
+    if constexpr (EPI == D_FIRST) {
+      cp_async8(as + row * C::AS + col, n > 0 ? src : g.A, n > 0);
+      cp_async8(as + row * C::AS + col + 1, n > 1 ? src + 1 : g.A, n > 1);
+    } else {
+      cp_async16(as + row * C::AS + col, n > 0 ? src : g.A, max(n, 0));
+    }
   }
 #pragma unroll
   for (int e = 0; e < C::BK * BC / C::THREADS; e++) {
@@ -394,8 +406,87 @@ __device__ __forceinline__ void load_stage(const GemmArgs<double, double, double
   }
 }
 
+// The operands of D_FINISH's low modes that one thread loads, when the kernel
+// starts (they do not depend on the product), so that their latency hides
+// behind the main loop: one zlow entry, its share of the tile's rows of low_y,
+// and low_x of the output column whose entries of U it forms (entries tid,
+// tid + THREADS, ... of the 8 x BN block, all in column tid % BN).
+template <class C>
+struct LowRegs {
+  static constexpr int L = kFdmLow;
+  static_assert(C::THREADS >= L * L && C::BM * L % C::THREADS == 0, "low modes' thread map");
+  static constexpr int AL = C::BM * L / C::THREADS, UE = L * C::BN / C::THREADS;
+  // doubles in shared memory: zlow, low_y's rows, U = zlow low_x^T as hi and lo
+  static constexpr int SIZE = L * L + C::BM * L + 2 * L * C::BN;
+  double z, al[AL], ex[L];
+
+  __device__ __forceinline__ void load(const FdmProduct& g, const DTile& t) {
+    const int tid = threadIdx.x, gc = t.n0 + tid % C::BN;
+    z = tid < L * L ? g.zlow[tid] : 0.0;
+#pragma unroll
+    for (int q = 0; q < AL; q++) {
+      const int e = tid + q * C::THREADS, gr = t.m0 + e / L;
+      al[q] = gr < t.m_end ? g.low_y[(size_t)gr * L + e % L] : 0.0;
+    }
+#pragma unroll
+    for (int b = 0; b < L; b++) ex[b] = gc < t.n_end ? g.low_x[(size_t)gc * L + b] : 0.0;
+  }
+  // To shared memory, and U formed there; ends with the block synchronised.
+  __device__ __forceinline__ void stage(double* sm) const {
+    static_assert(C::THREADS % C::BN == 0, "low modes' thread map");
+    const int tid = threadIdx.x, c = tid % C::BN;
+    double *al_s = sm + L * L, *uh = al_s + C::BM * L, *ul = uh + L * C::BN;
+    if (tid < L * L) sm[tid] = z;
+#pragma unroll
+    for (int q = 0; q < AL; q++) al_s[tid + q * C::THREADS] = al[q];
+    __syncthreads();
+#pragma unroll
+    for (int q = 0; q < UE; q++) {
+      const int a = (tid + q * C::THREADS) / C::BN;
+      double h = 0.0, l = 0.0;
+#pragma unroll
+      for (int b = 0; b < L; b++) dd_fma(h, l, sm[a * L + b], ex[b]);
+      uh[a * C::BN + c] = h;
+      ul[a * C::BN + c] = l;
+    }
+    __syncthreads();
+  }
+  // v, the low modes and the old value (accumulate) at tile row r, column c.
+  static __device__ __forceinline__ double add(const double* sm, int r, int c, double v, double old) {
+    const double *al_s = sm + L * L + r * L, *uh = sm + L * L + C::BM * L, *ul = uh + L * C::BN;
+    double h = 0.0, l = 0.0;
+#pragma unroll
+    for (int a = 0; a < L; a++) {
+      dd_fma(h, l, al_s[a], uh[a * C::BN + c]);
+      l = fma(al_s[a], ul[a * C::BN + c], l);
+    }
+    dd_add(h, l, v);
+    dd_add(h, l, old);
+    return h + l;
+  }
+};
+
+// v, the product's output at (row, column), as the epilogue stores it.
 template <class C, int EPI>
-__global__ void __launch_bounds__(C::THREADS) fdm_dgemm_kernel(const GemmArgs<double, double, double> g) {
+__device__ __forceinline__ void store_out(const FdmProduct& g, const DTile& t, const double* low,
+                                          bool closed, int row, int col, double v) {
+  double* dst = g.C + (size_t)row * g.ldc + col;
+  if constexpr (EPI == D_DIVIDE) {
+    const double d = g.alpha + g.bx * g.lx[col] + g.by * g.ly[row];
+    v = fabs(d) <= g.null_tol ? 0.0 : v / d;
+    const int lr = low_mode(g.low_r, row), lc = low_mode(g.low_c, col);
+    if (lr >= 0 && lc >= 0) {
+      g.zlow[lr * kFdmLow + lc] = v;
+      v = 0.0;
+    }
+  } else if constexpr (EPI == D_FINISH) {
+    v = LowRegs<C>::add(low, row - t.m0, col - t.n0, v, g.accumulate ? *dst : 0.0);
+  }
+  *dst = closed ? 0.0 : v;
+}
+
+template <class C, int EPI>
+__global__ void __launch_bounds__(C::THREADS) fdm_dgemm_kernel(const FdmProduct g) {
   extern __shared__ __align__(16) double dsm[];
   double* As = dsm;
   double* Bs = dsm + C::ST * C::A_ELEMS;
@@ -405,9 +496,12 @@ __global__ void __launch_bounds__(C::THREADS) fdm_dgemm_kernel(const GemmArgs<do
   const DTile t = tile_of<C::BM, C::BN>(g);
   const int m0 = t.m0, n0 = t.n0;
   const int nkt = (t.K + C::BK - 1) / C::BK;
+  const bool closed = (EPI == D_STORE || EPI == D_FIRST) && g.gate && *g.gate != 0;
+  LowRegs<C> low;
+  if constexpr (EPI == D_FINISH) low.load(g, t);
 
   auto issue = [&](int i) {
-    load_stage<C>(g, t, i * C::BK, As + (i % C::ST) * C::A_ELEMS, Bs + (i % C::ST) * C::B_ELEMS);
+    load_stage<C, EPI>(g, t, i * C::BK, As + (i % C::ST) * C::A_ELEMS, Bs + (i % C::ST) * C::B_ELEMS);
   };
 
   double acc[C::MT][C::NT][4];
@@ -454,6 +548,11 @@ __global__ void __launch_bounds__(C::THREADS) fdm_dgemm_kernel(const GemmArgs<do
     }
   }
   cp_async_wait<0>();
+  if constexpr (EPI == D_FINISH) {
+    static_assert(LowRegs<C>::SIZE * sizeof(double) <= C::SMEM, "low modes exceed the pipeline");
+    __syncthreads();  // the pipeline's shared memory is free from here
+    low.stage(dsm);
+  }
 #pragma unroll
   for (int mt = 0; mt < C::MT; mt++)
 #pragma unroll
@@ -465,26 +564,13 @@ __global__ void __launch_bounds__(C::THREADS) fdm_dgemm_kernel(const GemmArgs<do
 #pragma unroll
         for (int q = 0; q < 2; q++) {
           const int c = n0 + wn + nt * 8 + 2 * tq + q;
-          if (c >= t.n_end) continue;
-          double v = acc[mt][nt][2 * h + q];
-          double* dst = g.C + (size_t)r * g.ldc + c;
-          if constexpr (EPI == EPI_DIVIDE) {
-            const double d = g.alpha + g.bx * g.lx[c] + g.by * g.ly[r];
-            v = fabs(d) <= g.null_tol ? 0.0 : v / d;
-            const int lr = low_mode(g.low_r, r), lc = low_mode(g.low_c, c);
-            if (g.zlow && lr >= 0 && lc >= 0) {
-              g.zlow[lr * kFdmLow + lc] = v;
-              v = 0.0;
-            }
-          }
-          *dst = v;
+          if (c < t.n_end) store_out<C, EPI>(g, t, dsm, closed, r, c, acc[mt][nt][2 * h + q]);
         }
       }
 }
 
 template <class C, int EPI>
-cudaError_t run_d(const GemmArgs<double, double, double>& g, cudaStream_t s) {
-  if (g.M <= 0 || g.N <= 0) return cudaErrorInvalidValue;
+cudaError_t run_d(const FdmProduct& g, cudaStream_t s) {
   if (C::SMEM > 48 * 1024) {
     static bool attr[64] = {};  // per kernel instantiation and device
     int dev = 0;
@@ -521,7 +607,7 @@ struct KCfg {
 
 template <class C, int EPI>
 __global__ void __launch_bounds__(C::THREADS) fdm_dgemm_ksplit_kernel(
-    const GemmArgs<double, double, double> g) {
+    const FdmProduct g) {
   extern __shared__ __align__(16) double dsm[];
   double* As = dsm;
   double* Bs = dsm + C::ST * C::A_ELEMS;
@@ -530,9 +616,12 @@ __global__ void __launch_bounds__(C::THREADS) fdm_dgemm_ksplit_kernel(
   const DTile t = tile_of<C::BM, C::BN>(g);
   const int m0 = t.m0, n0 = t.n0;
   const int nkt = (t.K + C::BK - 1) / C::BK;
+  const bool closed = (EPI == D_STORE || EPI == D_FIRST) && g.gate && *g.gate != 0;
+  LowRegs<C> low;
+  if constexpr (EPI == D_FINISH) low.load(g, t);
 
   auto issue = [&](int i) {
-    load_stage<C>(g, t, i * C::BK, As + (i % C::ST) * C::A_ELEMS, Bs + (i % C::ST) * C::B_ELEMS);
+    load_stage<C, EPI>(g, t, i * C::BK, As + (i % C::ST) * C::A_ELEMS, Bs + (i % C::ST) * C::B_ELEMS);
   };
 
   double acc[2][C::NT][4];
@@ -593,31 +682,23 @@ __global__ void __launch_bounds__(C::THREADS) fdm_dgemm_ksplit_kernel(
         const int r = mt * 16 + gq + (q >> 1) * 8, c = nt * 8 + 2 * tq + (q & 1);
         red[(warp * C::BM + r) * C::RS + c] = acc[mt][nt][q];
       }
+  if constexpr (EPI == D_FINISH) {
+    static_assert((C::RED + LowRegs<C>::SIZE) * sizeof(double) <= C::SMEM, "low modes");
+    low.stage(dsm + C::RED);
+  }
   __syncthreads();
   for (int e = tid; e < C::BM * C::BN; e += C::THREADS) {
     const int r = e / C::BN, c = e % C::BN;
-    const int gr = m0 + r, gc = n0 + c;
-    if (gr >= t.m_end || gc >= t.n_end) continue;
+    if (m0 + r >= t.m_end || n0 + c >= t.n_end) continue;
     double v = red[r * C::RS + c];
 #pragma unroll
     for (int w = 1; w < C::W; w++) v += red[(w * C::BM + r) * C::RS + c];
-    double* dst = g.C + (size_t)gr * g.ldc + gc;
-    if constexpr (EPI == EPI_DIVIDE) {
-      const double d = g.alpha + g.bx * g.lx[gc] + g.by * g.ly[gr];
-      v = fabs(d) <= g.null_tol ? 0.0 : v / d;
-      const int lr = low_mode(g.low_r, gr), lc = low_mode(g.low_c, gc);
-      if (g.zlow && lr >= 0 && lc >= 0) {
-        g.zlow[lr * kFdmLow + lc] = v;
-        v = 0.0;
-      }
-    }
-    *dst = v;
+    store_out<C, EPI>(g, t, dsm + C::RED, closed, m0 + r, n0 + c, v);
   }
 }
 
 template <class C, int EPI>
-cudaError_t run_k(const GemmArgs<double, double, double>& g, cudaStream_t s) {
-  if (g.M <= 0 || g.N <= 0) return cudaErrorInvalidValue;
+cudaError_t run_k(const FdmProduct& g, cudaStream_t s) {
   if (C::SMEM > 48 * 1024) {
     static bool attr[64] = {};  // per kernel instantiation and device
     int dev = 0;
@@ -636,8 +717,8 @@ cudaError_t run_k(const GemmArgs<double, double, double>& g, cudaStream_t s) {
 }
 
 // Tile shape by problem size: 32 x 32 tiles (four times the blocks) until
-// the 64 x 64 grid alone covers the GPU's 148 SMs.
-inline bool small_tiles(int M, int N) { return ((M + 63) / 64) * ((N + 63) / 64) < 148; }
+// the 64 x 64 grid alone covers the GPU's SMs.
+inline bool small_tiles(int M, int N) { return ((M + 63) / 64) * ((N + 63) / 64) < kSms; }
 
 template <int P, class TA, class TB, class TC, int EPI>
 cudaError_t run(const GemmArgs<TA, TB, TC>& g, cudaStream_t s) {
@@ -665,7 +746,7 @@ cudaError_t launch_fdm_gemm(int prec, int epi, const void* A, int a_fp64, const 
                             cudaStream_t s) {
 #define SE_GEMM_ARGS(TA, TB, TC)                                                              \
   GemmArgs<TA, TB, TC> g{(const TA*)A, (const TB*)B, (TC*)C, M, N, K, lda, ldb, ldc, amax, cmax, \
-                         lx, ly, alpha, bx, by, null_tol, {}, {}, 0, nullptr, {}, {}}
+                         lx, ly, alpha, bx, by, null_tol}
   if (prec == 0) return cudaErrorInvalidValue;  // launch_fdm_dgemm
   if (prec == 1) {
     if (a_fp64) {
@@ -695,33 +776,47 @@ cudaError_t launch_fdm_gemm(int prec, int epi, const void* A, int a_fp64, const 
 #undef SE_GEMM_ARGS
 }
 
+namespace {
+template <template <class, int> class Run, class C>
+cudaError_t run_epi(const FdmProduct& p, bool wide, cudaStream_t s) {
+  if (p.lx) return Run<C, D_DIVIDE>::run(p, s);
+  return wide ? Run<C, D_STORE>::run(p, s) : Run<C, D_FIRST>::run(p, s);
+}
+template <class C, int EPI>
+struct RunD {
+  static cudaError_t run(const FdmProduct& p, cudaStream_t s) { return run_d<C, EPI>(p, s); }
+};
+template <class C, int EPI>
+struct RunK {
+  static cudaError_t run(const FdmProduct& p, cudaStream_t s) { return run_k<C, EPI>(p, s); }
+};
+}  // namespace
+
 cudaError_t launch_fdm_dgemm(const FdmProduct& p, cudaStream_t s) {
-  GemmArgs<double, double, double> g{p.A, p.B, p.C, p.y.len, p.x.len, 0, 0, 0, p.x.len, nullptr,
-                                     nullptr, p.lx, p.ly, p.alpha, p.bx, p.by, p.null_tol, p.x, p.y,
-                                     p.which, p.zlow, p.low_r, p.low_c};
-  if (!small_tiles(p.y.len, p.x.len))
-    return p.lx ? run_d<DCfg<64, 64, 2, 2, 3>, EPI_DIVIDE>(g, s)
-                : run_d<DCfg<64, 64, 2, 2, 3>, EPI_STORE>(g, s);
+  if (p.x.len <= 0 || p.y.len <= 0 || (p.lx && !p.zlow)) return cudaErrorInvalidValue;
+  // 16-byte copies of A: even rows from an aligned base (folded arrays and
+  // factors always; the caller's array where it happens to have them)
+  const bool wide = p.which == FDM_FACTOR_A ||
+                    (p.lda % 2 == 0 && (reinterpret_cast<uintptr_t>(p.A) & 15) == 0);
+  typedef DCfg<64, 64, 2, 2, 3> D;
+  const bool small = small_tiles(p.y.len, p.x.len);
+  if (p.low_y) return small ? run_k<KCfg<32, 4, 3>, D_FINISH>(p, s) : run_d<D, D_FINISH>(p, s);
+  if (!small) return run_epi<RunD, D>(p, wide, s);
   // The tile width whose fullest SM multiplies least: a direction's two parts
   // end in partial tiles, and a 301st tile on 148 SMs costs as much as 144
-  // more (768 x 383 unknowns, 300 tiles
-  // of 32 x 32 20.6 us an x product, 396 of 32 x 24 16.1). The 4 stand for a
-  // tile's own cost.
+  // more (768 x 383 unknowns, 300 tiles of 32 x 32 20.6 us an x product, 396
+  // of 32 x 24 16.1). The 4 stand for a tile's own cost.
   auto load = [&](int bn) {
     const int tiles = ((p.y.ge + 31) / 32 + (p.y.go + 31) / 32) *
                       ((p.x.ge + bn - 1) / bn + (p.x.go + bn - 1) / bn);
-    return (tiles + 147) / 148 * (bn + 4);
+    return (tiles + kSms - 1) / kSms * (bn + 4);
   };
   int bn = 32;
   for (int c : {24, 40})
     if (load(c) < load(bn)) bn = c;
-#define SE_KCFG(c)                                              \
-  return p.lx ? run_k<KCfg<c, 4, 3>, EPI_DIVIDE>(g, s) \
-              : run_k<KCfg<c, 4, 3>, EPI_STORE>(g, s)
-  if (bn == 24) SE_KCFG(24);
-  if (bn == 40) SE_KCFG(40);
-  SE_KCFG(32);
-#undef SE_KCFG
+  if (bn == 24) return run_epi<RunK, KCfg<24, 4, 3>>(p, wide, s);
+  if (bn == 40) return run_epi<RunK, KCfg<40, 4, 3>>(p, wide, s);
+  return run_epi<RunK, KCfg<32, 4, 3>>(p, wide, s);
 }
 
 }  // namespace seg

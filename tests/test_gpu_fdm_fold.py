@@ -66,3 +66,58 @@ def test_smooth_solve_takes_one_step(segpu, nx, ny, N, per, walls):
                                               method=segpu.METHOD_FDM))
     st = ls.Solve()
     assert st["reason"] == 2 and st["its"] == 1, st
+
+
+# where the inverse folds (from 4,096 unknowns where both directions do, from
+# 32,768 where one does, and with any direction of more than 256), the sizes
+# on either side, and where it does not: odd and even rows
+ROUTES = [
+    (17, 15, 4, P, N4), (17, 16, 4, P, N4),               # 4,080 and 4,352 unknowns
+    (13, 23, 5, P, N4), (11, 13, 6, BOX, ALL), (16, 11, 6, BOX, N4), (13, 10, 7, CH, TB),
+    (51, 1, 5, BOX, ALL), (1, 52, 5, BOX, ALL), (2, 52, 5, CH, N4),  # 254 and 259 long
+    (30, 29, 6, BOX, (True, True, False, True)), (30, 37, 6, BOX, (True, True, False, True)),
+    (31, 36, 6, BOX, (False, True, True, True)), (37, 37, 5, BOX, (False, True, True, True)),
+    (9, 11, 5, BOX, (True, False, True, False)), (10, 11, 4, BOX, (True, False, False, True)),
+    (52, 3, 5, BOX, (False, True, True, False)), (101, 99, 7, BOX, (True, False, True, False)),
+]
+
+
+@pytest.mark.parametrize("case", range(len(ROUTES)))
+@pytest.mark.parametrize("offset", [0, 1])
+def test_routes(segpu, case, offset):
+    """Input on and off a 16-byte boundary, output beside guards."""
+    import torch
+    nx, ny, N, per, walls = ROUTES[case]
+    keep, ls, apply, n = system(segpu, nx, ny, N, per, walls)
+    r = np.random.default_rng(case + 50).standard_normal(n)
+    rd = torch.zeros(n + 1, device="cuda", dtype=torch.float64)
+    rd[offset:n + offset] = torch.tensor(r)
+    x = torch.full((n + 2,), float("nan"), device="cuda", dtype=torch.float64)
+    x[0] = x[-1] = 7.0
+    torch.cuda.synchronize()
+    ls.fdm_apply(rd.data_ptr() + 8 * offset, x.data_ptr() + 8)
+    segpu.synchronize()
+    got = x.cpu().numpy()
+    assert got[0] == 7.0 and got[-1] == 7.0
+    got = got[1:-1]
+    assert (np.abs(apply(got) - r) <= 1e-11 * (apply(got, True) + np.abs(r))).all()
+
+
+@pytest.mark.parametrize("nx,ny,N,per,walls", [(9, 11, 5, BOX, (True, False, True, False)),
+                                               (7, 6, 4, BOX, ALL), (20, 17, 5, BOX, ALL)])
+def test_zero_right_hand_side(segpu, nx, ny, N, per, walls):
+    """A solve that is decided before its first step adds nothing, on either
+    route, also after a solve that left other values in the work arrays."""
+    m = segpu.Mesh("m", [nx, ny], "legendre", N, [0.0, 0.0], [1.0, 1.0], list(per))
+    u, f = segpu.Field("u", m, 1, segpu.BCs(*walls, m)), segpu.Field("f", m, 1, None)
+    ls = segpu.HelmholtzEqn(u, f, -1.0, -1.0, 1.0, 0,
+                            segpu.solver_opts(rtol=1e-10, mode=segpu.MODE_EXACT,
+                                              method=segpu.METHOD_FDM))
+    f.vals = 1.0 + m.verts[:, 0]
+    assert ls.Solve()["reason"] == 2 and np.abs(u.vals).max() > 0
+    f.vals = 0.0
+    st = ls.Solve()
+    assert st["its"] == 0 and st["reason"] in (2, 3)
+    bot, top, left, right = walls
+    g = u.vals.reshape(ny * N + 1, nx * N + 1)
+    assert not g[int(bot):ny * N + 1 - int(top), int(left):nx * N + 1 - int(right)].any()
