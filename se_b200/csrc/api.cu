@@ -273,10 +273,10 @@ struct se_linsys {
   // fast diagonalization (built on the first FDM solve)
   bool fdm_ready;
   int fdm_prec;
-  // eigenvectors E per direction (W-orthonormal; cached, shared): S = row-major
-  // E^T, ST = row-major E; eigenvalues lx, ly
-  double *Sx, *Sy, *SxT, *SyT, *lx, *ly;
-  void *Sx_lo, *Sy_lo, *SxT_lo, *SyT_lo;  // low-precision copies (cached, shared)
+  // per direction (cached, shared): eigenvalues lx, ly of the W-orthonormal
+  // eigenvectors E; in low precision S = row-major E^T, ST = row-major E
+  double *lx, *ly;
+  void *Sx_lo, *Sy_lo, *SxT_lo, *SyT_lo;
   int fdm_lbuf_prec;          // precision the L2, L3 buffers were sized for
   double *X1, *X2, *ax;       // FP64 work: two transform buffers, A x
   double* zlow;               // FP64 inverse: the low modes' block [kFdmLow][kFdmLow]
@@ -1140,6 +1140,33 @@ struct Factors {
   }
 };
 
+// Full eigenvectors E (column-major) and eigenvalues lam, ascending, from the
+// folded factors.
+void expand(const FoldDir& f, const std::vector<double>& FE, const std::vector<double>& lamF,
+            std::vector<double>& E, std::vector<double>& lam) {
+  const int n = f.n;
+  std::vector<std::pair<double, int>> order;  // eigenvalue, slot (even then odd)
+  for (int k = 0; k < f.ge; k++) order.push_back({lamF[k], k});
+  for (int k = 0; k < f.go; k++) order.push_back({lamF[f.os + k], f.os + k});
+  std::stable_sort(order.begin(), order.end(),
+                   [](const auto& a, const auto& b) { return a.first < b.first; });
+  E.assign((size_t)n * n, 0.0);
+  lam.resize(n);
+  for (int c = 0; c < n; c++) {
+    const bool odd = order[c].second >= f.os;
+    const int k = order[c].second - (odd ? f.os : 0), m = odd ? f.go : f.ge;
+    const int pitch = odd ? f.len - f.os : f.os, first = odd && f.periodic ? 1 : 0;
+    const double* B = FE.data() + (odd ? (size_t)f.ge * f.os : 0);
+    lam[c] = order[c].first;
+    for (int a = 0; a < m; a++) {
+      const int i = a + first, im = f.on ? fold_mirror(f, i) : i;
+      const double v = B[(size_t)a * pitch + k];
+      E[(size_t)c * n + i] = v;
+      if (im != i) E[(size_t)c * n + im] = odd ? -v : v;
+    }
+  }
+}
+
 // The eigenpairs of one direction: full eigenvectors E (column-major,
 // ascending eigenvalues lam) and the factors of the direction folded as f. A
 // folded block is the pair's own eigenproblem on the sums (differences) of
@@ -1156,8 +1183,6 @@ int eig_1d(const Dir& d, const FoldDir& f, const double* Kh, const double* w, st
     F.append(n, E, lam);
     return SE_OK;
   }
-  std::vector<std::pair<double, int>> order;  // eigenvalue, mode (even then odd)
-  std::vector<double> full((size_t)n * n, 0.0);
   for (int part = 0; part < 2; part++) {
     const int first = part && f.periodic ? 1 : 0, m = part ? n - f.ge : f.ge;
     if (m == 0) continue;
@@ -1185,25 +1210,8 @@ int eig_1d(const Dir& d, const FoldDir& f, const double* Kh, const double* w, st
       }
     if (int rc = eig_pair(m, Kp, Wp, A, l)) return rc;
     F.append(m, A, l);
-    for (int k = 0; k < m; k++) {
-      const int mode = (part ? f.ge : 0) + k;
-      order.push_back({l[k], mode});
-      for (int a = 0; a < m; a++) {
-        const int i = a + first, im = fold_mirror(f, i);
-        full[(size_t)mode * n + i] = A[(size_t)k * m + a];
-        if (im != i) full[(size_t)mode * n + im] = sg * A[(size_t)k * m + a];
-      }
-    }
   }
-  std::stable_sort(order.begin(), order.end(),
-                   [](const auto& a, const auto& b) { return a.first < b.first; });
-  E.resize((size_t)n * n);
-  lam.resize(n);
-  for (int k = 0; k < n; k++) {
-    lam[k] = order[k].first;
-    std::copy(full.begin() + (size_t)order[k].second * n,
-              full.begin() + (size_t)(order[k].second + 1) * n, E.begin() + (size_t)k * n);
-  }
+  expand(f, F.FE, F.lamF, E, lam);
   return SE_OK;
 }
 
@@ -1240,17 +1248,15 @@ struct EigForm {
 };
 struct Eig1D {
   int n = 0;
-  double* S = nullptr;    // W-orthonormal eigenvectors E, column-major (= row-major E^T)
-  double* ST = nullptr;   // row-major E
-  double* lam = nullptr;  // eigenvalues
+  double* lam = nullptr;  // eigenvalues, ascending
   double lmax = 0.0;
   // FP64 inverse: the direction folded where it can be, and whole where it
   // cannot or is short (kPlainMax)
   EigForm folded, plain;
-  void* low[3] = {nullptr, nullptr, nullptr};   // [1] FP32, [2] BF16 copies of S
-  void* lowT[3] = {nullptr, nullptr, nullptr};  // and of ST
+  void* low[3] = {nullptr, nullptr, nullptr};   // [2] BF16 copy of S = row-major E^T
+  void* lowT[3] = {nullptr, nullptr, nullptr};  // and of ST = row-major E
   // TF32 hi/lo pairs for the tcgen05 products, rows padded to tc_pitch:
-  // tc[0] of S (row-major E^T), tc[1] of ST (row-major E); [.][0] hi, [.][1] lo
+  // tc[0] of S, tc[1] of ST; [.][0] hi, [.][1] lo
   float* tc[2][2] = {{nullptr, nullptr}, {nullptr, nullptr}};
   int tc_pitch = 0;
 };
@@ -1261,6 +1267,11 @@ std::map<EigKey, Eig1D*> g_eig[64];
 // Longest direction kept whole beside its folded form.
 constexpr int kPlainMax = 256;
 
+int upload_doubles(double** dst, const std::vector<double>& v) {
+  if (int rc = dalloc(dst, v.size())) return rc;
+  CK(upload_now(*dst, v.data(), sizeof(double) * v.size()));
+  return SE_OK;
+}
 int upload_form(EigForm& e, const FoldDir& f, const Factors& F) {
   e.fold = f;
   e.lowmap = f.on ? FdmLowMap{std::min(kFdmLow / 2, f.ge), std::min(kFdmLow / 2, f.go), f.os}
@@ -1272,15 +1283,22 @@ int upload_form(EigForm& e, const FoldDir& f, const Factors& F) {
     for (int a = 0; a < f.go; a++)
       low[(size_t)(a + (f.periodic ? 1 : 0)) * kFdmLow + kFdmLow / 2 + k] =
           F.FE[(size_t)f.ge * f.os + (size_t)a * (f.len - f.os) + k];
-  auto up = [&](double** dst, const std::vector<double>& v) -> int {
-    if (int r = dalloc(dst, v.size())) return r;
-    CK(upload_now(*dst, v.data(), sizeof(double) * v.size()));
-    return SE_OK;
-  };
   int rc;
-  (void)((rc = up(&e.FE, F.FE)) || (rc = up(&e.FT, F.FT)) || (rc = up(&e.lamF, F.lamF)) ||
-         (rc = up(&e.low8, low)));
+  (void)((rc = upload_doubles(&e.FE, F.FE)) || (rc = upload_doubles(&e.FT, F.FT)) ||
+         (rc = upload_doubles(&e.lamF, F.lamF)) || (rc = upload_doubles(&e.low8, low)));
   return rc;
+}
+
+// Full eigenvectors (column-major, ascending eigenvalues) from a direction's
+// factors on the device.
+int full_vectors(const Eig1D& e, std::vector<double>& E) {
+  const EigForm& q = e.folded.FE ? e.folded : e.plain;
+  const FoldDir& f = q.fold;
+  std::vector<double> FE((size_t)f.ge * f.os + (size_t)f.go * (f.len - f.os)), lamF(f.len), lam;
+  CK(cudaMemcpy(FE.data(), q.FE, sizeof(double) * FE.size(), cudaMemcpyDeviceToHost));
+  CK(cudaMemcpy(lamF.data(), q.lamF, sizeof(double) * lamF.size(), cudaMemcpyDeviceToHost));
+  expand(f, FE, lamF, E, lam);
+  return SE_OK;
 }
 
 int eig_get(const Dir& d, const double* Kh, const double* w, int prec, Eig1D** out) {
@@ -1300,15 +1318,7 @@ int eig_get(const Dir& d, const double* Kh, const double* w, int prec, Eig1D** o
     int rc = eig_1d(d, f, Kh, w, Sh, lam, F);
     if (!rc) {
       for (double v : lam) ne->lmax = std::max(ne->lmax, std::fabs(v));
-      std::vector<double> T((size_t)n * n);
-      for (int j = 0; j < n; j++)
-        for (int i = 0; i < n; i++) T[(size_t)i * n + j] = Sh[(size_t)j * n + i];
-      auto up = [&](double** dst, const std::vector<double>& v) -> int {
-        if (int r = dalloc(dst, v.size())) return r;
-        CK(upload_now(*dst, v.data(), sizeof(double) * v.size()));
-        return SE_OK;
-      };
-      (void)((rc = up(&ne->S, Sh)) || (rc = up(&ne->ST, T)) || (rc = up(&ne->lam, lam)) ||
+      (void)((rc = upload_doubles(&ne->lam, lam)) ||
              (rc = upload_form(f.on ? ne->folded : ne->plain, f, F)));
       if (!rc && f.on && n <= kPlainMax) {
         Factors P;
@@ -1317,8 +1327,7 @@ int eig_get(const Dir& d, const double* Kh, const double* w, int prec, Eig1D** o
       }
     }
     if (rc) {
-      for (double* p : {ne->S, ne->ST, ne->lam})
-        if (p) cudaFree(p);
+      dfree(ne->lam);
       for (const EigForm& e : {ne->folded, ne->plain})
         for (double* p : {e.FE, e.FT, e.lamF, e.low8})
           if (p) cudaFree(p);
@@ -1329,10 +1338,8 @@ int eig_get(const Dir& d, const double* Kh, const double* w, int prec, Eig1D** o
     e = ne;
   }
   if (prec == 2 && !e->low[prec]) {
-    if (Sh.empty()) {
-      Sh.resize((size_t)e->n * e->n);
-      CK(cudaMemcpy(Sh.data(), e->S, sizeof(double) * Sh.size(), cudaMemcpyDeviceToHost));
-    }
+    if (Sh.empty())
+      if (int rc = full_vectors(*e, Sh)) return rc;
     if (int rc = upload_low(Sh, prec, &e->low[prec])) return rc;
     const int n = e->n;
     std::vector<double> T((size_t)n * n);
@@ -1341,10 +1348,8 @@ int eig_get(const Dir& d, const double* Kh, const double* w, int prec, Eig1D** o
     if (int rc = upload_low(T, prec, &e->lowT[prec])) return rc;
   }
   if (prec == 1 && !e->tc[0][0]) {
-    if (Sh.empty()) {
-      Sh.resize((size_t)e->n * e->n);
-      CK(cudaMemcpy(Sh.data(), e->S, sizeof(double) * Sh.size(), cudaMemcpyDeviceToHost));
-    }
+    if (Sh.empty())
+      if (int rc = full_vectors(*e, Sh)) return rc;
     const int n = e->n, pitch = tc_pitch(n);
     for (int t = 0; t < 2; t++) {
       std::vector<float> hi((size_t)n * pitch, 0.0f), lo((size_t)n * pitch, 0.0f);
@@ -1528,10 +1533,6 @@ int fdm_setup(se_linsys* ls, int prec) {
   Eig1D *ex = nullptr, *ey = nullptr;
   if ((rc = eig_get(op.d[0], op.Kh, op.w, prec, &ex)) || (rc = eig_get(op.d[1], op.Kh, op.w, prec, &ey)))
     return rc;
-  ls->Sx = ex->S;
-  ls->Sy = ey->S;
-  ls->SxT = ex->ST;
-  ls->SyT = ey->ST;
   ls->lx = ex->lam;
   ls->ly = ey->lam;
   const bool folds = fdm_folds(*ex, *ey);

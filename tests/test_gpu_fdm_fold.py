@@ -121,3 +121,52 @@ def test_zero_right_hand_side(segpu, nx, ny, N, per, walls):
     bot, top, left, right = walls
     g = u.vals.reshape(ny * N + 1, nx * N + 1)
     assert not g[int(bot):ny * N + 1 - int(top), int(left):nx * N + 1 - int(right)].any()
+
+
+def test_setup_memory(segpu):
+    """A direction of n unknowns keeps its folded factors, about n^2 doubles,
+    and no full matrix beside them."""
+    import torch
+
+    def solve(nx):
+        m = segpu.Mesh("m", [nx, 2], "legendre", 6, [0.0, 0.0], [1.0, 1.0], [True, False])
+        u, f = segpu.Field("u", m, 1, segpu.BCs(*TB, m)), segpu.Field("f", m, 1, None)
+        f.vals = np.cos(2 * np.pi * m.verts[:, 0])
+        ls = segpu.HelmholtzEqn(u, f, -1.0, -1.0, 1.0, 0,
+                                segpu.solver_opts(rtol=1e-10, mode=segpu.MODE_EXACT,
+                                                  method=segpu.METHOD_FDM))
+        torch.cuda.synchronize()
+        free = torch.cuda.mem_get_info()[0]
+        assert ls.Solve()["reason"] == 2
+        torch.cuda.synchronize()
+        return free - torch.cuda.mem_get_info()[0]
+
+    solve(37)  # cuSOLVER's and the kernels' own memory
+    n = 401 * 6
+    assert solve(401) <= 8 * 1.5 * n * n + (8 << 20)
+
+
+@pytest.mark.parametrize("nx,ny,N,per,walls", [(37, 20, 6, CH, TB), (9, 8, 5, BOX, ALL), (7, 9, 5, P, N4),
+                                               (16, 8, 6, P, N4), (9, 11, 5, BOX, (True, False, True, False))])
+@pytest.mark.parametrize("first", ["fp64", "mixed", "bf16"])
+def test_precisions_in_any_order(segpu, nx, ny, N, per, walls, first):
+    """The low precisions take the eigenvectors from the FP64 factors, whichever
+    precision set a direction up (other element counts per `first`: fresh
+    directions): solutions agree at rtol 1e-11 to 1e-9. (Square elements: BF16
+    refinement does not contract at aspect ratio 4.)"""
+    precs = {"fp64": segpu.PREC_FP64, "mixed": segpu.PREC_MIXED, "bf16": segpu.PREC_BF16}
+    nx += {"fp64": 0, "mixed": 16, "bf16": 32}[first] * (1 if nx != 16 else 0)
+    m = segpu.Mesh("m", [nx, ny], "legendre", N, [0.0, 0.0], [nx / ny, 1.0], list(per))
+    u, f = segpu.Field("u", m, 1, segpu.BCs(*walls, m)), segpu.Field("f", m, 1, None)
+    X = m.verts
+    f.vals = np.cos(2 * np.pi * X[:, 0] * ny / nx) * np.sin(2 * np.pi * X[:, 1]) + 0.5
+    ls = segpu.HelmholtzEqn(u, f, -1.0, -1.0, 1.0, 0)
+    out = []
+    for name in [first] + [k for k in precs if k != first] + ["fp64"]:
+        u.vals = 0.0
+        ls.set_opts(segpu.solver_opts(rtol=1e-11, mode=segpu.MODE_EXACT, method=segpu.METHOD_FDM,
+                                      precision=precs[name], max_it=100))
+        assert ls.Solve()["reason"] == 2, name
+        out.append(u.vals)
+    for v in out[:-1]:
+        assert np.abs(v - out[-1]).max() <= 1e-9 * np.abs(out[-1]).max()
