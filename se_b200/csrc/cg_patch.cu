@@ -483,9 +483,6 @@ __global__ void __launch_bounds__(kPT, 1) cg_patch_kernel(const __grid_constant_
     seq++;
     return c.ok != 0;
   };
-  auto give_up = [&]() {
-    if (tid == 0) atomicExch(&A.res[si].err, S.seq0);
-  };
   // KSPConvergedDefault on the norm at iteration n (thread 0). nn is the
   // squared norm (or its signed form, natural); a square clear of both
   // thresholds decides nothing and spares the root, which is long on the path
@@ -528,6 +525,7 @@ __global__ void __launch_bounds__(kPT, 1) cg_patch_kernel(const __grid_constant_
 
   // right-hand side off the operator's range (remove_null == 2): f -= (sum f
   // / sum d) d
+  bool good = true;
   if (S.remove_null == 2) {
     double s0 = 0.0, s1 = 0.0;
 #pragma unroll
@@ -537,10 +535,7 @@ __global__ void __launch_bounds__(kPT, 1) cg_patch_kernel(const __grid_constant_
       s0 += r[k];
       s1 += diag(f);
     }
-    if (!reduce2(SUM_A, s0, s1, [&](double t0, double t1) { c.cproj = t0 / t1; })) {
-      give_up();
-      return;
-    }
+    good = reduce2(SUM_A, s0, s1, [&](double t0, double t1) { c.cproj = t0 / t1; });
   }
   double s_zr = 0.0, s_n = 0.0, s_z = 0.0;
   {
@@ -588,7 +583,7 @@ __global__ void __launch_bounds__(kPT, 1) cg_patch_kernel(const __grid_constant_
     }
     return true;
   };
-  bool good = S.remove_null ? mean_sums() : true;
+  if (S.remove_null) good = good && mean_sums();
   good = good && reduce2(SUM_B, s_zr, s_n, [&](double zr, double nn) {
     converged(0, nt == 2 ? zr : nn);
     c.beta = zr;
@@ -779,9 +774,11 @@ __global__ void __launch_bounds__(kPT, 1) cg_patch_kernel(const __grid_constant_
       }
     });
   }
-  if constexpr (CL) cluster_sync();  // no block leaves while another may store into it
+  // the only way out, also after a wait that gave up: no block leaves while
+  // another may store into it
+  if constexpr (CL) cluster_sync();
   if (!c.ok) {
-    give_up();
+    if (tid == 0) atomicExch(&A.res[si].err, S.seq0);
     return;
   }
 #pragma unroll

@@ -106,3 +106,29 @@ def test_no_device_fails_loudly(segpu):
     with pytest.raises(segpu.SEError) as e:
         segpu.Field("f", m, 1, None)
     assert e.value.code == segpu.SE_ERR_CUDA
+
+
+def _without_lambdas(src):
+    """src with the body of every lambda cut out."""
+    out, i = [], 0
+    for m in re.finditer(r"\[[&=\w, ]*\]\([^)]*\)\s*(?:->\s*\w+\s*)?\{", src):
+        if m.start() < i:
+            continue
+        out.append(src[i:m.start()])
+        depth, i = 1, m.end()
+        while depth:
+            depth += {"{": 1, "}": -1}.get(src[i], 0)
+            i += 1
+    return "".join(out) + src[i:]
+
+
+def test_on_chip_cg_has_one_way_out_of_a_cluster():
+    """Blocks of a cluster store into one another's shared memory, so none may
+    leave before the closing cluster barrier, whatever gave up."""
+    src = open(os.path.join(ROOT, "se_b200", "csrc", "cg_patch.cu")).read()
+    src = re.sub(r"//[^\n]*", "", src)
+    a = src.index("cg_patch_kernel(const __grid_constant__")
+    kernel = _without_lambdas(src[a:src.index("size_t patch_smem(", a)])
+    loop = kernel.index("while (good && !c.done)")
+    last = kernel.index("if constexpr (CL) cluster_sync();", loop)
+    assert not re.search(r"\breturn\b|\bexit\b", kernel[:last])
