@@ -87,3 +87,39 @@ def test_mixed_batch_and_repeat(segpu):
     for x, y, sa, sb in zip(va, [s[2].vals for s in systems], a, b):
         assert sa["reason"] == 2 and sb["reason"] == 2
         assert np.array_equal(x, y)  # deterministic, autotuned shape reused
+
+
+@pytest.mark.parametrize("odd", ["svv", "large"])
+def test_batch_off_the_chip(segpu, odd):
+    """A CG group with a system that the on-chip kernel does not take (an SVV
+    term, or too many unknowns for the device's blocks) runs as one streaming
+    launch of an autotuned shape: as single solves, and the same bits when the
+    tuned shape is used again."""
+    def one(nx, ny, svv=0, lam=3.0):
+        m = segpu.Mesh("m", [nx, ny], "legendre", 8, [0.0, 0.0], [1.0, 1.0], [True, False])
+        b = segpu.BCs(True, True, False, False, m)
+        X = m.verts
+        u, f = segpu.Field("u", m, 1, b), segpu.Field("f", m, 1, b)
+        f.vals = np.cos(2 * np.pi * X[:, 0]) * np.sin(3 * X[:, 1]) + 0.2
+        ls = segpu.HelmholtzEqn(u, f, -lam, -1.0, 1.0, svv,
+                                segpu.solver_opts(rtol=1e-11, mode=segpu.MODE_EXACT))
+        return u, f, ls
+
+    systems = [one(5, 4), one(9, 7, lam=30.0), one(12, 3)]
+    systems.append(one(6, 5, svv=4) if odd == "svv" else one(96, 97))
+    singles = []
+    for u, f, ls in systems:
+        st = ls.Solve()
+        singles.append((u.vals, st))
+        u.vals = 0.0
+    runs = []
+    for _ in range(2):
+        stats = segpu.solve_batch([s[2] for s in systems])
+        runs.append([s[0].vals for s in systems])
+        for (u, f, ls), (ref, rst), st in zip(systems, singles, stats):
+            assert st["reason"] == rst["reason"] == 2
+            assert abs(st["its"] - rst["its"]) <= 2
+            assert np.abs(u.vals - ref).max() <= 1e-9 * np.abs(ref).max()
+            u.vals = 0.0
+    for a, b in zip(*runs):
+        assert np.array_equal(a, b)

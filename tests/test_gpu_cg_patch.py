@@ -121,3 +121,68 @@ def test_subnormal_inner_products(segpu, oracle, case, batched):
     out = segpu.solve_batch([ls])[0] if batched else ls.Solve("helm_")
     assert (out["reason"], out["its"]) == (st["reason"], st["its"]) == (-10, 1)
     assert np.isfinite(fs.vals).all() and np.isfinite(out["rnorm"])
+
+
+# every form of the kernel: one cluster and a grid, each with all of a block's
+# state in registers (at most 2048 nodes) and in shared memory (at most 4096)
+FORMS = [
+    ((9, 7), 6, P, NONE), ((14, 16), 5, CH, TB),                              # cluster, registers
+    ((20, 20), 9, P, NONE), ((16, 16), 12, CH, TB), ((16, 29), 8, BOX, ALL),  # cluster, shared
+    ((20, 31), 7, P, NONE), ((31, 15), 8, BOX, NONE),
+    ((40, 36), 8, P, NONE), ((35, 44), 7, CH, TB), ((52, 29), 8, BOX, ALL),   # grid, registers
+    ((70, 72), 8, P, NONE), ((66, 61), 9, CH, TB), ((90, 71), 7, BOX, ALL),   # grid, shared
+]
+
+
+def form_system(S, form, method, poisson=False, off=0.0, **kw):
+    ne, p, per, walls = form
+    m = S.Mesh("m", list(ne), "legendre", p, [0, 0], [1, 1], list(per))
+    b = S.BCs(*walls, m)
+    X = m.verts
+    u, f = S.Field("u", m, 1, b), S.Field("f", m, 1, b)
+    f.vals = (np.cos(2 * np.pi * X[:, 0]) * np.sin(4 * np.pi * X[:, 1])
+              + np.cos(6 * np.pi * X[:, 1]) + off)
+    o = S.solver_opts(rtol=1e-11, mode=S.MODE_EXACT, method=method, **kw)
+    ls = S.PoissonEqn(u, f, 1.0, o) if poisson else S.HelmholtzEqn(u, f, -20.0, -1.0, 1.0, 0, o)
+    return m, u, f, ls
+
+
+@pytest.mark.parametrize("form", range(len(FORMS)))
+@pytest.mark.parametrize("norm", [0, 1, 2])
+def test_every_form_and_norm(segpu, form, norm):
+    _, u, _, ls = form_system(segpu, FORMS[form], segpu.METHOD_CG, norm_type=norm)
+    assert ls.Solve()["reason"] == 2
+    _, r, _, lr = form_system(segpu, FORMS[form], segpu.METHOD_FDM)
+    assert lr.Solve()["reason"] == 2
+    assert np.abs(u.vals - r.vals).max() <= 1e-8 * np.abs(r.vals).max()
+
+
+PERIODIC = [0, 2, 5, 7, 10]
+
+
+@pytest.mark.parametrize("form", PERIODIC)
+@pytest.mark.parametrize("project", [False, True])
+def test_null_space_in_every_form(segpu, form, project):
+    """Periodic Poisson: the mean of z as a third reduction, and a right-hand
+    side off the operator's range projected onto it first."""
+    off = 0.3 if project else 0.0
+    out = []
+    for method in (segpu.METHOD_CG, segpu.METHOD_FDM):
+        _, u, _, ls = form_system(segpu, FORMS[form], method, poisson=True, off=off)
+        st = ls.Solve(removeNullSpace=True, projectRHS=project)
+        assert st["reason"] == 2, st
+        out.append(u.vals - u.vals.mean())
+    assert np.abs(out[0] - out[1]).max() <= 1e-8 * np.abs(out[1]).max()
+
+
+def test_batch_with_null_space(segpu):
+    """Teams of one block to many, the constant removed in each."""
+    sizes = [(40, 36), (9, 8), (2, 2), (25, 14), (5, 6), (50, 41)]
+    systems = [form_system(segpu, (s, 8, P, NONE), segpu.METHOD_CG, poisson=True) for s in sizes]
+    stats = segpu.solve_batch([s[3] for s in systems], removeNullSpace=True)
+    for (m, u, f, ls), s, st in zip(systems, sizes, stats):
+        assert st["reason"] == 2
+        _, r, _, lr = form_system(segpu, (s, 8, P, NONE), segpu.METHOD_FDM, poisson=True)
+        assert lr.Solve(removeNullSpace=True)["reason"] == 2
+        got, ref = u.vals - u.vals.mean(), r.vals - r.vals.mean()
+        assert np.abs(got - ref).max() <= 1e-8 * np.abs(ref).max()
