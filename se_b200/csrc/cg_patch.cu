@@ -483,6 +483,16 @@ __global__ void __launch_bounds__(kPT, 1) cg_patch_kernel(const __grid_constant_
     seq++;
     return c.ok != 0;
   };
+  // the last common step of a cluster's blocks, on every way out: none leaves
+  // while another may store into it (one that gave up early waits here for
+  // the others, whose waits for it run out)
+  auto leave = [&]() {
+    if constexpr (CL) cluster_sync();
+  };
+  auto give_up = [&]() {
+    leave();
+    if (tid == 0) atomicExch(&A.res[si].err, S.seq0);
+  };
   // KSPConvergedDefault on the norm at iteration n (thread 0). nn is the
   // squared norm (or its signed form, natural); a square clear of both
   // thresholds decides nothing and spares the root, which is long on the path
@@ -525,7 +535,6 @@ __global__ void __launch_bounds__(kPT, 1) cg_patch_kernel(const __grid_constant_
 
   // right-hand side off the operator's range (remove_null == 2): f -= (sum f
   // / sum d) d
-  bool good = true;
   if (S.remove_null == 2) {
     double s0 = 0.0, s1 = 0.0;
 #pragma unroll
@@ -535,7 +544,10 @@ __global__ void __launch_bounds__(kPT, 1) cg_patch_kernel(const __grid_constant_
       s0 += r[k];
       s1 += diag(f);
     }
-    good = reduce2(SUM_A, s0, s1, [&](double t0, double t1) { c.cproj = t0 / t1; });
+    if (!reduce2(SUM_A, s0, s1, [&](double t0, double t1) { c.cproj = t0 / t1; })) {
+      give_up();
+      return;
+    }
   }
   double s_zr = 0.0, s_n = 0.0, s_z = 0.0;
   {
@@ -583,7 +595,7 @@ __global__ void __launch_bounds__(kPT, 1) cg_patch_kernel(const __grid_constant_
     }
     return true;
   };
-  if (S.remove_null) good = good && mean_sums();
+  bool good = S.remove_null ? mean_sums() : true;
   good = good && reduce2(SUM_B, s_zr, s_n, [&](double zr, double nn) {
     converged(0, nt == 2 ? zr : nn);
     c.beta = zr;
@@ -774,13 +786,11 @@ __global__ void __launch_bounds__(kPT, 1) cg_patch_kernel(const __grid_constant_
       }
     });
   }
-  // the only way out, also after a wait that gave up: no block leaves while
-  // another may store into it
-  if constexpr (CL) cluster_sync();
   if (!c.ok) {
-    if (tid == 0) atomicExch(&A.res[si].err, S.seq0);
+    give_up();
     return;
   }
+  leave();
 #pragma unroll
   for (int k = 0; k < K; k++) {
     const unsigned f = node(k);

@@ -122,13 +122,19 @@ def _without_lambdas(src):
     return "".join(out) + src[i:]
 
 
-def test_on_chip_cg_has_one_way_out_of_a_cluster():
+def test_on_chip_cg_leaves_a_cluster_together():
     """Blocks of a cluster store into one another's shared memory, so none may
-    leave before the closing cluster barrier, whatever gave up."""
+    leave without the closing cluster barrier, whatever gave up: every way out
+    of the kernel runs leave(), which is that barrier."""
     src = open(os.path.join(ROOT, "se_b200", "csrc", "cg_patch.cu")).read()
     src = re.sub(r"//[^\n]*", "", src)
     a = src.index("cg_patch_kernel(const __grid_constant__")
-    kernel = _without_lambdas(src[a:src.index("size_t patch_smem(", a)])
-    loop = kernel.index("while (good && !c.done)")
-    last = kernel.index("if constexpr (CL) cluster_sync();", loop)
-    assert not re.search(r"\breturn\b|\bexit\b", kernel[:last])
+    kernel = src[a:src.index("size_t patch_smem(", a)]
+    assert re.search(r"auto leave = \[&\]\(\) \{\s*if constexpr \(CL\) cluster_sync\(\);\s*\};", kernel)
+    assert re.search(r"auto give_up = \[&\]\(\) \{\s*leave\(\);", kernel)
+    body = _without_lambdas(kernel)
+    loop = body.index("while (good && !c.done)")
+    assert body.rindex("leave();") > loop
+    before = body[:body.rindex("leave();")]
+    for m in re.finditer(r"\breturn\b|\bexit\b", before):
+        assert before[:m.start()].rstrip().endswith("give_up();")
