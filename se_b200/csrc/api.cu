@@ -3499,6 +3499,29 @@ std::mutex g_noalloc_mu;                // guards the host-side tables below
 double* g_noalloc_dev[kMaxDevices];     // device address of the scratch, per device
 CgTile g_noalloc_tiles[kNoAllocMaxTiles];
 int g_noalloc_begin[kNoAllocMaxGrid + 1];
+// on-chip cuts of the systems solved last (a cut depends on these numbers
+// alone: the search takes about 5 us, its occupancy query more)
+struct NoAllocPlan {
+  int dev, N, nE[2];  // N == 0: empty
+  bool fits;
+  PatchPlan plan;
+};
+constexpr int kNoAllocPlans = 8;
+NoAllocPlan g_noalloc_plans[kNoAllocPlans];
+int g_noalloc_next = 0;
+
+const NoAllocPlan& noalloc_plan(int dev, int sms, const OpDev& op) {
+  for (const NoAllocPlan& p : g_noalloc_plans)
+    if (p.N == op.d[0].N && p.dev == dev && p.nE[0] == op.d[0].nE && p.nE[1] == op.d[1].nE) return p;
+  NoAllocPlan& p = g_noalloc_plans[g_noalloc_next];
+  g_noalloc_next = (g_noalloc_next + 1) % kNoAllocPlans;
+  p.dev = dev;
+  p.N = op.d[0].N;
+  p.nE[0] = op.d[0].nE;
+  p.nE[1] = op.d[1].nE;
+  p.fits = patch_plan_single(op, sms, &p.plan);
+  return p;
+}
 }  // namespace
 
 extern "C" int se_helmholtz_solve_noalloc(const int nEls[2], int N, const double min[2],
@@ -3613,8 +3636,9 @@ extern "C" int se_helmholtz_solve_noalloc(const int nEls[2], int N, const double
   // and w, which that solve does not use (zeroed: they may hold anything)
   int sms = 0;
   CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
-  PatchPlan plan;
-  if (patch_plan_single(op, sms, &plan) && sizeof(PatchPkt) * patch_packets(plan) <= sizeof(double) * 4 * vn) {
+  const NoAllocPlan& np = noalloc_plan(dev, sms, op);
+  const PatchPlan& plan = np.plan;
+  if (np.fits && sizeof(PatchPkt) * patch_packets(plan) <= sizeof(double) * 4 * vn) {
     cudaStream_t st = g_stream;
     PatchPkt* pk = reinterpret_cast<PatchPkt*>(z);
     PatchResult* d_res = reinterpret_cast<PatchResult*>(d_solve);

@@ -46,7 +46,6 @@
 #include <algorithm>
 #include <cmath>
 #include <cstring>
-#include <vector>
 
 #include "common.cuh"
 #include "kh.cuh"
@@ -933,9 +932,10 @@ cudaError_t launch_cg_patch(const PatchLaunch& L, cudaStream_t s) { return dispa
 // cluster the latency is about 3100 (16x16 p = 6 over 16 blocks: 5000). So
 // systems up to about 25,000 unknowns run as a cluster.
 bool patch_plan_single(const OpDev& op, int max_blocks, PatchPlan* out) {
-  std::vector<PatchPlan> t((size_t)max_blocks + 1);
-  patch_plan_table(op, max_blocks, t.data());
-  *out = t.back();
+  max_blocks = std::min(max_blocks, kPatchMaxBlocks);
+  PatchPlan t[kPatchMaxBlocks + 1];
+  patch_plan_table(op, max_blocks, t);
+  *out = t[max_blocks];
   if (out->gx == 0) return false;
   const double grid = 1.8 * out->cost + 6700.0;
   // t improves with the block count: the largest cluster first

@@ -167,3 +167,60 @@ def test_noalloc_refuses_other_methods_and_precisions(segpu):
     with pytest.raises(segpu.SEError) as e:
         run_noalloc(segpu, CHANNEL, rhs, sol, -3.0, -1.0, 1.0, opts=opts)
     assert e.value.code == segpu.SE_ERR_ARG
+
+
+SHIM = """
+#include <cstdlib>
+#include <new>
+static long count;
+extern "C" long shim_news() { return count; }
+void* operator new(std::size_t n) { count++; if (void* p = std::malloc(n ? n : 1)) return p; throw std::bad_alloc(); }
+void operator delete(void* p) noexcept { std::free(p); }
+void operator delete(void* p, std::size_t) noexcept { std::free(p); }
+"""
+
+CALLS = """
+import ctypes, sys
+sys.path[:0] = [{tests!r}, {root!r}]
+import test_zz_no_alloc as T
+from se_b200 import segpu as S
+import torch
+news = ctypes.CDLL({shim!r}).shim_news
+news.restype = ctypes.c_long
+S.load_library()
+real = S._lib.se_helmholtz_solve_noalloc
+per_call = []
+def counted(*a):
+    n = news()
+    rc = real(*a)
+    per_call.append(news() - n)
+    return rc
+class Lib:
+    se_helmholtz_solve_noalloc = staticmethod(counted)
+    def __getattr__(self, k): return getattr(S._lib, k)
+lib = Lib()
+S.load_library = lambda: lib
+for case in (T.CHANNEL, T.BOX, T.CHANNEL, T.BOX):
+    rhs, sol = T.fields(case, 1)
+    T.run_noalloc(S, case, rhs, sol, -3.0, -1.0, 1.0)
+print("news", per_call)
+"""
+
+
+def test_noalloc_allocates_nothing_on_the_heap(segpu, tmp_path):
+    """Host tables are on the stack or kept: no operator new in a call (counted
+    by a preloaded one in a process of its own), also not where two systems
+    take turns."""
+    import os
+    import subprocess
+    import sys
+    src, shim = tmp_path / "shim.cpp", tmp_path / "shim.so"
+    src.write_text(SHIM)
+    subprocess.run(["g++", "-shared", "-fPIC", "-O1", "-o", str(shim), str(src)], check=True)
+    here = os.path.dirname(os.path.abspath(__file__))
+    script = CALLS.format(tests=here, root=os.path.dirname(here), shim=str(shim))
+    r = subprocess.run([sys.executable, "-c", script], capture_output=True, text=True, timeout=300,
+                       env=dict(os.environ, LD_PRELOAD=str(shim)))
+    assert r.returncode == 0, r.stderr[-2000:]
+    counts = [int(k) for k in r.stdout.split("news [")[1].split("]")[0].split(",")]
+    assert len(counts) == 4 and counts[2:] == [0, 0], counts
