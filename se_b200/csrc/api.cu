@@ -694,17 +694,27 @@ CgSolve patch_state(const PatchResult& r) {
   return st;
 }
 
-// Run the on-chip CG for A x = b (the system's cut fits); fills stats.
+// The packets of a system's on-chip solves, allocated by the first one.
+int patch_buffers(se_linsys* ls) {
+  if (ls->d_pkts) return SE_OK;
+  const size_t np = patch_packets(ls->pplan);
+  int rc;
+  if (!(rc = dalloc(&ls->d_pres, 1)) && !(rc = dalloc(&ls->d_pkts, np))) {
+    cudaError_t e = cudaMemsetAsync(ls->d_pkts, 0, sizeof(PatchPkt) * np, g_stream);
+    if (e == cudaSuccess) e = cudaMemsetAsync(ls->d_pres, 0, sizeof(PatchResult), g_stream);
+    if (e == cudaSuccess) return SE_OK;
+    rc = cuda_fail(e, "clearing the CG packets");
+  }
+  dfree(ls->d_pres);
+  dfree(ls->d_pkts);
+  return rc;
+}
+
+// Run the on-chip CG for A x = b (the system's cut fits, its packets are
+// there); fills stats.
 int run_cg_patch(se_linsys* ls, const double* b, double* x, double rtol, double atol, double dtol,
                  int max_it, int remove_null, CgSolve* out_state, float* kernel_ms) {
   cudaStream_t s = g_stream;
-  if (!ls->d_pkts) {
-    int rc;
-    const size_t np = patch_packets(ls->pplan);
-    if ((rc = dalloc(&ls->d_pres, 1)) || (rc = dalloc(&ls->d_pkts, np))) return rc;
-    CK(cudaMemsetAsync(ls->d_pkts, 0, sizeof(PatchPkt) * np, s));
-    CK(cudaMemsetAsync(ls->d_pres, 0, sizeof(PatchResult), s));
-  }
   const PatchSolve ps = make_patch(ls->op, b, x, rtol, atol, dtol, max_it, ls->opts.norm_type,
                                    remove_null, ls->pplan, ls->d_pkts, ++ls->patch_seq);
   PatchLaunch L = patch_launch(ls->op, ls->pplan.gx * ls->pplan.gy, ls->pplan.in_registers,
@@ -730,8 +740,13 @@ int run_cg_patch(se_linsys* ls, const double* b, double* x, double rtol, double 
 // Run the persistent CG for A x = b on this system's schedule; fills stats.
 int run_cg(se_linsys* ls, const double* b, double* x, double rtol, double atol, double dtol,
            int max_it, int remove_null, CgSolve* out_state, float* kernel_ms, int lowp = 0) {
-  if (lowp == 0 && ls->patch)
-    return run_cg_patch(ls, b, x, rtol, atol, dtol, max_it, remove_null, out_state, kernel_ms);
+  if (lowp == 0 && ls->patch) {
+    const int rc = patch_buffers(ls);
+    if (!rc)
+      return run_cg_patch(ls, b, x, rtol, atol, dtol, max_it, remove_null, out_state, kernel_ms);
+    if (rc != SE_ERR_OOM) return rc;
+    g_err.clear();  // no room for them: the streaming kernel below needs none
+  }
   CgSolve cs = make_solve(ls, b, x, rtol, atol, dtol, max_it, remove_null);
   cudaStream_t s = g_stream;
   CK(cudaMemcpyAsync(ls->d_solve, &cs, sizeof(cs), cudaMemcpyHostToDevice, s));
@@ -2131,7 +2146,9 @@ int run_cg_batch_once(int dev, std::vector<se_linsys*>& sys, const std::vector<c
 // would finish last (iterations grow with the longer side's element count at
 // equal order, an iteration costs its reductions' latency plus the cut's
 // work). Packing beats giving one solve the whole device: an iteration's two
-// reductions (about 2 us) do not shrink with more blocks.
+// reductions (about 2 us) do not shrink with more blocks. The launches follow
+// one another on the stream, each with sequence numbers of its own, so they
+// share one launch's packets (a few MB at most).
 constexpr double kPatchLatency = 4500.0;  // cycles of an iteration's reductions
 struct PatchWs {
   PatchPkt* pkts = nullptr;
@@ -2142,7 +2159,7 @@ struct PatchWs {
   unsigned long long seq = 0;
 };
 PatchWs g_patch[64];
-// best cut for every block count, by order and element counts
+// best cut for every block count, by order and element counts (of the last few hundred systems)
 std::map<std::tuple<int, int, int, int>, std::vector<PatchPlan>> g_patch_tables;
 
 int run_patch_group(int dev, std::vector<se_linsys*>& sys, int remove_null,
@@ -2150,6 +2167,7 @@ int run_patch_group(int dev, std::vector<se_linsys*>& sys, int remove_null,
   int sms = 0;
   CK(cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev));
   const int cap = std::min(sms, kPatchMaxBlocks), n = (int)sys.size();
+  if (g_patch_tables.size() > 256) g_patch_tables.clear();
   std::vector<const std::vector<PatchPlan>*> tab(n);
   std::vector<int> g(n), order(n);
   auto its = [&](int i) { return (double)std::max(sys[i]->op.d[0].nE, sys[i]->op.d[1].nE); };
@@ -2209,20 +2227,28 @@ int run_patch_group(int dev, std::vector<se_linsys*>& sys, int remove_null,
   PatchWs& W = g_patch[dev];
   cudaStream_t s = g_stream;
   size_t npk = 0;
-  for (int i = 0; i < n; i++) npk += patch_packets((*tab[i])[g[i]]);
+  for (int l = 0; l < nl; l++) {
+    size_t k1 = 0;
+    for (int k = first[l]; k < first[l + 1]; k++) k1 += patch_packets((*tab[order[k]])[g[order[k]]]);
+    npk = std::max(npk, k1);
+  }
   int rc;
   if (W.cap_pkts < npk) {
     if ((rc = grow(&W.pkts, &W.cap_pkts, npk))) return rc;
-    CK(cudaMemsetAsync(W.pkts, 0, sizeof(PatchPkt) * W.cap_pkts, s));
+    const cudaError_t e = cudaMemsetAsync(W.pkts, 0, sizeof(PatchPkt) * W.cap_pkts, s);
+    if (e != cudaSuccess) {
+      W.cap_pkts = 0;  // not cleared: not to be used
+      return cuda_fail(e, "clearing the CG packets");
+    }
   }
-  W.seq++;
   std::vector<PatchSolve> solves(n);
   std::vector<int> cta;
   std::vector<int> cta_first;
-  size_t at = 0;
   for (int l = 0; l < nl; l++) {
     cta_first.push_back((int)cta.size());
     const int base = (int)cta.size();
+    size_t at = 0;
+    W.seq++;
     for (int k = first[l]; k < first[l + 1]; k++) {
       const int i = order[k];
       se_linsys* ls = sys[i];
@@ -2285,7 +2311,11 @@ int solve_cg_group(std::vector<se_linsys*>& sys, int remove_null, std::vector<Cg
   const int N = sys[0]->op.d[0].N;
   bool patch = true;
   for (const se_linsys* ls : sys) patch = patch && ls->patch;
-  if (patch) return run_patch_group(dev, sys, remove_null, out, ms);
+  if (patch) {
+    const int rc = run_patch_group(dev, sys, remove_null, out, ms);
+    if (rc != SE_ERR_OOM) return rc;
+    g_err.clear();  // no room for the packets
+  }
   std::vector<const OpDev*> ops;
   long ntiles = 0;
   for (se_linsys* ls : sys) {

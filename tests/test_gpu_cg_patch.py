@@ -186,3 +186,56 @@ def test_batch_with_null_space(segpu):
         assert lr.Solve(removeNullSpace=True)["reason"] == 2
         got, ref = u.vals - u.vals.mean(), r.vals - r.vals.mean()
         assert np.abs(got - ref).max() <= 1e-8 * np.abs(ref).max()
+
+
+def test_solves_with_no_memory_left(segpu):
+    """A system created before the rest of the program took all device memory
+    still solves, alone and in a batch: without room for its packets the
+    streaming kernel runs on the vectors the system has."""
+    import ctypes
+    import torch
+
+    def make(ne, svv=0):
+        m, u, f, ls = smooth(segpu, ne, 5, 7.0, segpu.METHOD_CG)
+        if svv:
+            ls = segpu.HelmholtzEqn(u, f, -7.0, -1.0, 1.0, svv,
+                                    segpu.solver_opts(rtol=1e-11, mode=segpu.MODE_EXACT))
+        return m, u, f, ls
+
+    # both streaming kernels' code on the device, and the answers
+    warm = [make((9, 8), 2), make((8, 8), 2)]
+    for w in warm:
+        assert w[3].Solve()["reason"] == 2
+    segpu.solve_batch([w[3] for w in warm])
+    ref = [make((9, 8)), make((6, 7))]
+    for r in ref:
+        assert r[3].Solve()["reason"] == 2
+    ref = [r[1].vals for r in ref]
+    systems = [make((9, 8)), make((6, 7))]
+    torch.cuda.synchronize()
+    torch.cuda.empty_cache()
+    rt = ctypes.CDLL("libcudart.so.12")
+    rt.cudaMalloc.argtypes = [ctypes.POINTER(ctypes.c_void_p), ctypes.c_size_t]
+    rt.cudaFree.argtypes = [ctypes.c_void_p]
+    held = []
+    size = torch.cuda.mem_get_info()[0]
+    while size >= 256:
+        p = ctypes.c_void_p()
+        if rt.cudaMalloc(ctypes.byref(p), size) == 0:
+            held.append(p)
+        else:
+            rt.cudaGetLastError()
+            size //= 2
+    try:
+        got = []
+        for s in systems:
+            assert s[3].Solve()["reason"] == 2
+            got.append(s[1].vals)
+            s[1].vals = 0.0
+        assert all(st["reason"] == 2 for st in segpu.solve_batch([s[3] for s in systems]))
+        got += [s[1].vals for s in systems]
+    finally:
+        for p in held:
+            rt.cudaFree(p)
+    for a, b in zip(got, ref + ref):
+        assert np.abs(a - b).max() <= 1e-8 * np.abs(b).max()
