@@ -402,12 +402,6 @@ cudaError_t launch_tc_plan(const TcPlan& p, cudaStream_t s);
 cudaError_t launch_tc_split(const double* x, int rows, int cols, int ld, float* hi, float* lo,
                             int pitch, cudaStream_t s);
 
-// C = A B (row-major, leading dimensions lda/ldb/ldc) on the tensor cores
-// (gemm.cu). prec: 0 FP64, 1 TF32 on FP32 data, 2 BF16. epi: 0 store,
-// 1 store after the spectral divide by alpha + bx lx[col] + by ly[row]
-// (|divisor| <= null_tol gives 0), 2 accumulate into FP64 C scaled by *cmax
-// (cmax == nullptr: 1). a_fp64: A is FP64 (scaled by 1/*amax when amax is
-// given) whatever prec; c_fp64: C is FP64 (required for epi 2).
 // One periodic direction of nel = 2^logn equal elements of order p in Bloch
 // form (bloch.cu): V [nel][p][p] complex, row i column k, the W-orthonormal
 // eigenvectors of wavenumber m; mu [nel][p] their eigenvalues; tw [nel/2]
@@ -482,6 +476,12 @@ cudaError_t launch_fdm_fold(const FoldDir& dx, const FoldDir& dy, const double* 
 cudaError_t launch_fdm_unfold(const FoldDir& dx, const FoldDir& dy, const double* in, double* out,
                               bool accumulate, const double* zlow, const double* lx,
                               const double* ly, cudaStream_t s);
+// C = A B (row-major, leading dimensions lda/ldb/ldc) on the tensor cores
+// (gemm.cu). prec: 1 TF32 on FP32 data, 2 BF16. epi: 0 store,
+// 1 store after the spectral divide by alpha + bx lx[col] + by ly[row]
+// (|divisor| <= null_tol gives 0), 2 accumulate into FP64 C scaled by *cmax
+// (cmax == nullptr: 1). a_fp64: A is FP64 (scaled by 1/*amax when amax is
+// given); c_fp64: C is FP64 (required for epi 2).
 cudaError_t launch_fdm_gemm(int prec, int epi, const void* A, int a_fp64, const void* B, void* C,
                             int c_fp64, int M, int N, int K, int lda, int ldb, int ldc,
                             const double* amax, const double* cmax, const double* lx,

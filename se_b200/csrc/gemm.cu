@@ -5,31 +5,35 @@
 //
 // C (M x N) = A (M x K) * B (K x N), all row-major with leading dimensions,
 // on the tensor cores through warp-level MMA:
-//   P = 0  FP64 data, m16n8k8 f64 MMA (Blackwell's FP64 tensor path; there is
-//          no FP64 kind of the tcgen05 MMA), FP64 accumulation;
+//   FP64 data, m16n8k8 f64 MMA (Blackwell's FP64 tensor path; there is no FP64
+//   kind of the tcgen05 MMA), FP64 accumulation (launch_fdm_dgemm);
 //   P = 1  FP32 data rounded to TF32, m16n8k8 tf32 MMA, FP32 accumulation;
-//   P = 2  BF16 data, m16n8k16 bf16 MMA, FP32 accumulation.
-// While a grid of 64 x 64 tiles would leave SMs idle, 32 x 32 tiles: FP64 by
-// 4 warps that split each K stage and sum their partial tiles in warp order,
-// low precision by 2 x 2 warps; 64 x 64 tiles (2 x 2 warps) above that. FP64
-// operands stream through a multi-stage cp.async pipeline; low-precision ones pass
-// through registers (converted, and the FP64 first operand scaled, on the
-// way) into double-buffered shared memory. Any leading dimension (odd ones
-// included) is accepted.
+//   P = 2  BF16 data, m16n8k16 bf16 MMA, FP32 accumulation (launch_fdm_gemm).
 //
-// Epilogues: store; store after the spectral divide
-// C[l][k] /= alpha + bx lx[k] + by ly[l] (entries whose divisor is below
-// null_tol in magnitude — the null mode — become 0); accumulate into an FP64
-// C with an optional scale read from device memory (low precisions).
+// Low precision: 32 x 32 tiles while a grid of 64 x 64 tiles would leave SMs
+// idle, 64 x 64 above that, 2 x 2 warps; operands pass through registers
+// (converted, and the FP64 first operand scaled, on the way) into
+// double-buffered shared memory, from rows of any length. Epilogues: store;
+// store after the spectral divide C[l][k] /= alpha + bx lx[k] + by ly[l]
+// (entries whose divisor is below null_tol in magnitude -- the null mode --
+// become 0); accumulate into an FP64 C with an optional scale read from device
+// memory.
 //
-// FP64 products with a folded direction (FdmBlocks, fdm.cu): the square
-// factor is block-diagonal, an even and an odd block stored one after the
-// other, so the product is two of half the depth in one launch; a block of
-// threads works inside one of them. The divide can move the lowest modes of
-// both directions out of C into zlow (8 x 8), leaving zeros: a smooth
-// solution's largest coefficients, which the unfolding adds back in
-// double-double so that the products' rounding of them does not dominate the
-// solve's first residual.
+// FP64: one operand is a direction's factor. Where the direction is folded
+// (FoldDir, fdm.cu) that factor is block-diagonal, an even and an odd block
+// stored one after the other, and the product two of half the depth in one
+// launch; a block of threads works inside one of them. Tiles of 32 x 24, 32 or
+// 40 by 4 warps that split each K stage and sum their partial tiles in warp
+// order; 64 x 64 by 2 x 2 warps where an unfolded array of that size covers the
+// SMs with them (a folded one may not: its two parts' partial tiles). Operands
+// stream through a multi-stage pipeline of 16-byte copies, so rows start on
+// even offsets: folded arrays and factors are laid out that way, and only the
+// input of an inverse that does not fold may not be (D_FIRST, 8-byte copies).
+// The divide moves the low modes of both directions out of C into zlow
+// (8 x 8), leaving zeros: a smooth solution's largest coefficients, which the
+// unfolding, or the last product where nothing is folded (D_FINISH), adds back
+// in double-double so that the products' rounding of them does not dominate
+// the solve's first residual.
 #include <cuda_bf16.h>
 
 #include <cstdint>
@@ -44,12 +48,6 @@ constexpr int kThreads = 128;
 template <int P>
 struct Tr;
 template <>
-struct Tr<0> {
-  typedef double S;
-  typedef double Acc;
-  enum { BK = 16, KS = 8, AP = 4, BP = 8 };
-};
-template <>
 struct Tr<1> {
   typedef uint32_t S;  // TF32 bit patterns
   typedef float Acc;
@@ -62,7 +60,6 @@ struct Tr<2> {
   enum { BK = 32, KS = 16, AP = 8, BP = 8 };
 };
 
-__device__ __forceinline__ double as_d(double x) { return x; }
 __device__ __forceinline__ float as_f(float x) { return x; }
 __device__ __forceinline__ float as_f(__nv_bfloat16 x) { return __bfloat162float(x); }
 
@@ -76,19 +73,15 @@ __device__ __forceinline__ uint32_t to_tf32(float f) {
 // multiplies FP64 inputs (the FDM's 1/max|r| normalisation).
 template <int P, class T>
 __device__ __forceinline__ typename Tr<P>::S to_s(T x, double scale) {
-  if constexpr (P == 0) {
-    return as_d(x) * scale;
-  } else {
-    float f;
-    if constexpr (sizeof(T) == 8)
-      f = (float)(as_d(x) * scale);
-    else
-      f = as_f(x);
-    if constexpr (P == 1)
-      return to_tf32(f);
-    else
-      return __float2bfloat16_rn(f);
-  }
+  float f;
+  if constexpr (sizeof(T) == 8)
+    f = (float)(x * scale);
+  else
+    f = as_f(x);
+  if constexpr (P == 1)
+    return to_tf32(f);
+  else
+    return __float2bfloat16_rn(f);
 }
 
 __device__ __forceinline__ void mma_f64(double (&c)[4], const double (&a)[4], const double (&b)[2]) {
@@ -212,7 +205,7 @@ __global__ void __launch_bounds__(kThreads) fdm_gemm_kernel(const GemmArgs<TA, T
     const S* bs = Bs[buf];
 #pragma unroll
     for (int kk = 0; kk < BK; kk += KS) {
-      if constexpr (P == 0 || P == 1) {
+      if constexpr (P == 1) {
         S a[MT][4], b[NT][2];
 #pragma unroll
         for (int mt = 0; mt < MT; mt++) {
@@ -232,10 +225,7 @@ __global__ void __launch_bounds__(kThreads) fdm_gemm_kernel(const GemmArgs<TA, T
         for (int mt = 0; mt < MT; mt++)
 #pragma unroll
           for (int nt = 0; nt < NT; nt++) {
-            if constexpr (P == 0)
-              mma_f64(acc[mt][nt], a[mt], b[nt]);
-            else
-              mma_tf32(acc[mt][nt], a[mt], b[nt]);
+            mma_tf32(acc[mt][nt], a[mt], b[nt]);
           }
       } else {
         uint32_t a[MT][4], b[NT][2];
@@ -299,8 +289,7 @@ __global__ void __launch_bounds__(kThreads) fdm_gemm_kernel(const GemmArgs<TA, T
 
 // ---------------------------------------------------------------------------
 // FP64 products: multi-stage cp.async pipeline (16-byte copies with zero fill;
-// 8-byte ones, which any leading dimension would need, held the products at
-// a third of the FP64 rate), BM x BN block tile of WM x WN warps, each warp
+// 8-byte ones held the products at a third of the FP64 rate), BM x BN block tile of WM x WN warps, each warp
 // (BM/WM) x (BN/WN) in m16n8 MMA tiles.
 template <int BM_, int BN_, int WM_, int WN_, int ST_, int BK_ = 16>
 struct DCfg {
@@ -588,10 +577,10 @@ cudaError_t run_d(const FdmProduct& g, cudaStream_t s) {
   return cudaGetLastError();
 }
 
-// FP64 products split over K inside the block: a 32 x 32 output tile per
+// FP64 products split over K inside the block: a 32 x BN output tile per
 // block of W warps; stage i holds a (8 W KW)-wide slice of K and warp w
 // multiplies its w-th (8 KW)-wide part, so every warp keeps the whole tile's
-// 8 accumulator fragments (8 independent MMA chains) and runs 8 KW MMAs
+// 2 NT accumulator fragments (independent MMA chains) and runs 2 NT KW MMAs
 // between barriers. At the end the W partial tiles are summed through shared
 // memory in warp order (deterministic) and the epilogue is applied.
 template <int BN_, int W_, int ST_, int KW_ = 1>
@@ -735,9 +724,8 @@ cudaError_t run(const GemmArgs<TA, TB, TC>& g, cudaStream_t s) {
 
 }  // namespace
 
-// prec: 0 FP64, 1 TF32 on FP32 data, 2 BF16. Types by role:
-//  in:  FP64 (prec 0, or the normalised first product of prec 1/2 when amax
-//       is given), else the low type;
+// prec: 1 TF32 on FP32 data, 2 BF16. Types by role:
+//  in:  FP64 for the normalised first product (amax given), else the low type;
 //  out: FP64 for accumulate, else the precision's type.
 cudaError_t launch_fdm_gemm(int prec, int epi, const void* A, int a_fp64, const void* B, void* C,
                             int c_fp64, int M, int N, int K, int lda, int ldb, int ldc,
@@ -747,7 +735,7 @@ cudaError_t launch_fdm_gemm(int prec, int epi, const void* A, int a_fp64, const 
 #define SE_GEMM_ARGS(TA, TB, TC)                                                              \
   GemmArgs<TA, TB, TC> g{(const TA*)A, (const TB*)B, (TC*)C, M, N, K, lda, ldb, ldc, amax, cmax, \
                          lx, ly, alpha, bx, by, null_tol}
-  if (prec == 0) return cudaErrorInvalidValue;  // launch_fdm_dgemm
+  if (prec != 1 && prec != 2) return cudaErrorInvalidValue;  // FP64: launch_fdm_dgemm
   if (prec == 1) {
     if (a_fp64) {
       SE_GEMM_ARGS(double, float, float);
