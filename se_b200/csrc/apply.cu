@@ -94,7 +94,6 @@ struct EfTile {
   static constexpr int W = SW | 1;       // staged row pitch (odd)
   static constexpr int OXP = (TX + 1) | 1;  // x-pass output pitch (odd)
   static constexpr int TY = 4 * N;       // output rows per tile
-  static constexpr int H = TY + N + 1;   // staged rows
   static constexpr int ITEMS = EX * TY;  // x-pass (= y-pass) items, one per thread
   static_assert(ITEMS <= 256 && TX * (TY / N) == ITEMS && TY % N == 0, "tile shape");
   static_assert(SW > 64 && SW <= 96, "staging columns");
@@ -124,7 +123,7 @@ __device__ __forceinline__ bool all_outputs(const Dir& d, int first, int n) {
 // Stage the tile's vertices and its N-vertex halo to the left and below into
 // X (zero where a vertex is no unknown): warp w takes rows w, w + 8, ...;
 // lane l columns l, l + 32, l + 64; all copies issued before the wait.
-template <int N, int H = EfTile<N>::H>
+template <int N, int H>
 __device__ __forceinline__ void ef_stage(const Dir& dx, const Dir& dy, int G0,
                                          const double* __restrict__ x, double* X, int gx0,
                                          int gy0) {

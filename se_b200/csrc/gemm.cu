@@ -404,9 +404,9 @@ template <class C>
 struct LowRegs {
   static constexpr int L = kFdmLow;
   static_assert(C::THREADS >= L * L && C::BM * L % C::THREADS == 0, "low modes' thread map");
-  static constexpr int AL = C::BM * L / C::THREADS, UE = L * C::BN / C::THREADS;
+  static constexpr int AL = C::BM * L / C::THREADS;
   // doubles in shared memory: zlow, low_y's rows, U = zlow low_x^T as hi and lo
-  static constexpr int SIZE = L * L + C::BM * L + 2 * L * C::BN;
+  static constexpr int size() { return L * L + C::BM * L + 2 * L * C::BN; }
   double z, al[AL], ex[L];
 
   __device__ __forceinline__ void load(const FdmProduct& g, const DTile& t) {
@@ -430,7 +430,7 @@ struct LowRegs {
     for (int q = 0; q < AL; q++) al_s[tid + q * C::THREADS] = al[q];
     __syncthreads();
 #pragma unroll
-    for (int q = 0; q < UE; q++) {
+    for (int q = 0; q < L * C::BN / C::THREADS; q++) {
       const int a = (tid + q * C::THREADS) / C::BN;
       double h = 0.0, l = 0.0;
 #pragma unroll
@@ -538,7 +538,7 @@ __global__ void __launch_bounds__(C::THREADS) fdm_dgemm_kernel(const FdmProduct 
   }
   cp_async_wait<0>();
   if constexpr (EPI == D_FINISH) {
-    static_assert(LowRegs<C>::SIZE * sizeof(double) <= C::SMEM, "low modes exceed the pipeline");
+    static_assert(LowRegs<C>::size() * sizeof(double) <= C::SMEM, "low modes exceed the pipeline");
     __syncthreads();  // the pipeline's shared memory is free from here
     low.stage(dsm);
   }
@@ -672,7 +672,7 @@ __global__ void __launch_bounds__(C::THREADS) fdm_dgemm_ksplit_kernel(
         red[(warp * C::BM + r) * C::RS + c] = acc[mt][nt][q];
       }
   if constexpr (EPI == D_FINISH) {
-    static_assert((C::RED + LowRegs<C>::SIZE) * sizeof(double) <= C::SMEM, "low modes");
+    static_assert((C::RED + LowRegs<C>::size()) * sizeof(double) <= C::SMEM, "low modes");
     low.stage(dsm + C::RED);
   }
   __syncthreads();
