@@ -1669,10 +1669,8 @@ int fdm_apply64(se_linsys* ls, const double* in, double* out, bool accumulate,
   };
   if (folds) CK(launch_fdm_fold(ex.fold, ey.fold, in, ls->X2, closed, g_stream));
   p.lda = folds ? ex.fold.len : ex.fold.n;
-  p.gate = folds ? nullptr : closed;
   CK(product(FDM_FACTOR_B, folds ? ls->X2 : in, ex.FE, ls->X1));
   p.lda = ex.fold.len;
-  p.gate = nullptr;
   p.lx = ex.lamF;
   p.ly = ey.lamF;
   p.alpha = op.alpha;
@@ -1690,6 +1688,7 @@ int fdm_apply64(se_linsys* ls, const double* in, double* out, bool accumulate,
     p.low_x = ex.low8;
     p.low_y = ey.low8;
     p.accumulate = accumulate;
+    p.gate = closed;
     CK(product(FDM_FACTOR_A, ey.FE, ls->X1, out));
     return SE_OK;
   }

@@ -446,12 +446,12 @@ struct FdmLowMap {
 // C = A B on folded arrays ([y.len][x.len]) in FP64, one operand the factor of
 // a direction (`which`: B that of x, or A that of y); with lx the spectral
 // divide by alpha + bx lx[col] + by ly[row] (|divisor| <= null_tol gives 0)
-// and, with zlow, the low modes moved into zlow[8][8] (0 left in C); zeros
-// when gate && *gate != 0. Where no direction is folded the first product can
-// read the caller's array (lda, any alignment) and the last write it (ldc):
-// with low_y, C (= or +=, accumulate) gets A B + sum_ab low_y[row][a]
-// zlow[a][b] low_x[col][b], the low modes' eigenvectors ([n][8]), in
-// double-double, rounded once.
+// and, with zlow, the low modes moved into zlow[8][8] (0 left in C). Where no
+// direction is folded the first product can read the caller's array (lda, any
+// alignment) and the last write it (ldc): with low_y, C (= or +=, accumulate)
+// gets A B + sum_ab low_y[row][a] zlow[a][b] low_x[col][b], the low modes'
+// eigenvectors ([n][8]), in double-double, rounded once; zeros (or nothing
+// added) when gate && *gate != 0.
 struct FdmProduct {
   const double *A, *B;
   double* C;

@@ -378,12 +378,12 @@ __device__ __forceinline__ void load_stage(const FdmProduct& g, const DTile& t, 
     const int q = threadIdx.x + e * C::THREADS, row = q / AC, col = q % AC * 2;
     const int gr = t.m0 + row, gc = k0 + col;
     const int n = gr < t.m_end ? min(2, t.K - gc) : 0;
-    const double* src = t.A + (ptrdiff_t)gr * t.lda + gc;
     if constexpr (EPI == D_FIRST) {
+      const double* src = t.A + (ptrdiff_t)gr * t.lda + gc;
       cp_async8(as + row * C::AS + col, n > 0 ? src : g.A, n > 0);
       cp_async8(as + row * C::AS + col + 1, n > 1 ? src + 1 : g.A, n > 1);
     } else {
-      cp_async16(as + row * C::AS + col, n > 0 ? src : g.A, max(n, 0));
+      cp_async16(as + row * C::AS + col, n > 0 ? t.A + (ptrdiff_t)gr * t.lda + gc : g.A, max(n, 0));
     }
   }
 #pragma unroll
@@ -406,7 +406,7 @@ struct LowRegs {
   static_assert(C::THREADS >= L * L && C::BM * L % C::THREADS == 0, "low modes' thread map");
   static constexpr int AL = C::BM * L / C::THREADS;
   // doubles in shared memory: zlow, low_y's rows, U = zlow low_x^T as hi and lo
-  static constexpr int size() { return L * L + C::BM * L + 2 * L * C::BN; }
+  enum { SIZE = L * L + C::BM * L + 2 * L * C::BN };
   double z, al[AL], ex[L];
 
   __device__ __forceinline__ void load(const FdmProduct& g, const DTile& t) {
@@ -469,9 +469,10 @@ __device__ __forceinline__ void store_out(const FdmProduct& g, const DTile& t, c
       v = 0.0;
     }
   } else if constexpr (EPI == D_FINISH) {
-    v = LowRegs<C>::add(low, row - t.m0, col - t.n0, v, g.accumulate ? *dst : 0.0);
+    const double old = g.accumulate ? *dst : 0.0;
+    v = closed ? old : LowRegs<C>::add(low, row - t.m0, col - t.n0, v, old);
   }
-  *dst = closed ? 0.0 : v;
+  *dst = v;
 }
 
 template <class C, int EPI>
@@ -485,7 +486,7 @@ __global__ void __launch_bounds__(C::THREADS) fdm_dgemm_kernel(const FdmProduct 
   const DTile t = tile_of<C::BM, C::BN>(g);
   const int m0 = t.m0, n0 = t.n0;
   const int nkt = (t.K + C::BK - 1) / C::BK;
-  const bool closed = (EPI == D_STORE || EPI == D_FIRST) && g.gate && *g.gate != 0;
+  const bool closed = EPI == D_FINISH && g.gate && *g.gate != 0;
   LowRegs<C> low;
   if constexpr (EPI == D_FINISH) low.load(g, t);
 
@@ -538,7 +539,7 @@ __global__ void __launch_bounds__(C::THREADS) fdm_dgemm_kernel(const FdmProduct 
   }
   cp_async_wait<0>();
   if constexpr (EPI == D_FINISH) {
-    static_assert(LowRegs<C>::size() * sizeof(double) <= C::SMEM, "low modes exceed the pipeline");
+    static_assert(LowRegs<C>::SIZE * sizeof(double) <= C::SMEM, "low modes exceed the pipeline");
     __syncthreads();  // the pipeline's shared memory is free from here
     low.stage(dsm);
   }
@@ -605,7 +606,7 @@ __global__ void __launch_bounds__(C::THREADS) fdm_dgemm_ksplit_kernel(
   const DTile t = tile_of<C::BM, C::BN>(g);
   const int m0 = t.m0, n0 = t.n0;
   const int nkt = (t.K + C::BK - 1) / C::BK;
-  const bool closed = (EPI == D_STORE || EPI == D_FIRST) && g.gate && *g.gate != 0;
+  const bool closed = EPI == D_FINISH && g.gate && *g.gate != 0;
   LowRegs<C> low;
   if constexpr (EPI == D_FINISH) low.load(g, t);
 
@@ -672,7 +673,7 @@ __global__ void __launch_bounds__(C::THREADS) fdm_dgemm_ksplit_kernel(
         red[(warp * C::BM + r) * C::RS + c] = acc[mt][nt][q];
       }
   if constexpr (EPI == D_FINISH) {
-    static_assert((C::RED + LowRegs<C>::size()) * sizeof(double) <= C::SMEM, "low modes");
+    static_assert((C::RED + LowRegs<C>::SIZE) * sizeof(double) <= C::SMEM, "low modes");
     low.stage(dsm + C::RED);
   }
   __syncthreads();
