@@ -487,7 +487,7 @@ SL_BYTES_PER_VERTEX = 32.0
 SL_FLOPS_PER_VERTEX = (2 * 9 * 5 + 2 * 81 * 2 + 2 * 9 * 2) + (2 * 9 * 5 + 2 * 81 + 2 * 9)
 # DRAM traffic of one SL launch (dram__bytes_read.sum + dram__bytes_write.sum)
 # from one ncu capture of that kernel on this workload.
-SL_TRAFFIC_BYTES = 6.358016e6
+SL_TRAFFIC_BYTES = 6.367744e6
 
 
 def dense_fdm_roofline(r):
@@ -554,8 +554,8 @@ def sl_roofline(r):
             "traffic": SL_TRAFFIC_BYTES,
             "fp64_tflops_achieved": fp64, "fp64_tflops_peak_measured_dgemm": r["fp64_tflops"],
             "fp64_frac": fp64 / r["fp64_tflops"],
-            "limiter": "latency of the element-block gathers through L1 (ncu: L1 data path "
-                       "72% busy, FP64 pipe 27%, DRAM 1.8%, long-scoreboard stalls)"}
+            "limiter": "the L1 data path, 16-byte element-block gathers (ncu: 74% busy, 5.6 "
+                       "wavefronts a request, FP64 pipe 25%, DRAM 2.2%, long-scoreboard stalls)"}
 
 
 def tc_roofline(r):
@@ -882,8 +882,8 @@ def run_ensemble(count=256, seed=2024):
     """256 independent Helmholtz solves, mesh n x n elements with n uniform in
     8..64, p in {4, 6, 8}, lambda log-uniform in [1e-2, 1e2], RHS a seeded sum
     of 8 Fourier modes; doubly periodic unit square; rtol 1e-10. Timed with
-    the batch call (FDM: graphs overlapped on 8 streams; CG: one persistent
-    launch per order, autotuned)."""
+    the batch call (FDM: graphs overlapped on 8 streams; CG: per
+    order, each solve on a team of blocks of its own)."""
     import torch
     import se_b200 as S
     rng = np.random.default_rng(seed)
@@ -917,7 +917,7 @@ def run_ensemble(count=256, seed=2024):
             systems.append((m, bc, u, rr, ls))
         lss = [s[4] for s in systems]
         ng = sum(ls.vecSize for ls in lss)
-        S.solve_batch(lss)  # setup: eigen cache, graphs, autotuned launch shape
+        S.solve_batch(lss)  # setup: eigen cache, graphs, workspaces
         times = []
         for _ in range(3):
             torch.cuda.synchronize()

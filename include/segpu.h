@@ -279,10 +279,11 @@ int se_linsys_solve(se_linsys* ls, int remove_null_space, se_solve_stats* stats)
  * reference, which solves one system at a time through the same Solve).
  * Systems using SE_METHOD_CG and the same polynomial order run in persistent
  * cooperative launches, each solve on a team of blocks of its own with its
- * whole state on the chip. A group with a system that does not fit (above
- * about 600,000 unknowns) or has an SVV term runs as one launch (up to 256
- * systems) whose shape is chosen by a built-in autotuner on the first batch
- * of a given signature;
+ * whole state on the chip: patches of whole elements, at most 4096 nodes, one
+ * an SM (every system to about 510,000 unknowns, none above about 587,000,
+ * by order and element counts). A group with a system that does not fit or
+ * has an SVV term runs as one launch (up to 256 systems) whose shape is chosen
+ * by a built-in autotuner on the first batch of a given signature;
  * SE_METHOD_FDM systems run their solve graphs overlapped on a pool of 8
  * streams. stats (nullable) gets one entry per system; the return value is
  * SE_ERR_NOT_CONVERGED if any system diverged. The caller's stream is ordered
@@ -301,7 +302,7 @@ int se_linsys_solve_finish(se_linsys* ls, se_solve_stats* stats);
  * aliased), queued on the calling thread's stream. */
 int se_linsys_apply(se_linsys* ls, const double* x_dev, double* y_dev);
 /* No counterpart in the reference: x = A^{-1} r by the fast-diagonalization
- * transforms in FP64 (four tensor-core products; exact up to rounding, the
+ * transforms in FP64 (tensor-core products; exact up to rounding, the
  * null mode of a singular operator set to zero), on the calling thread's
  * stream; device pointers, vec_size entries each, not aliased. A
  * preconditioner for callers that run their own Krylov loop. The first call

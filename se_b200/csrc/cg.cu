@@ -2,8 +2,9 @@
 // Helmholtz/Poisson solves of one polynomial order N, sm_100a.
 //
 // FP64 solves that fit the chip run cg_patch.cu's kernel; this one serves what
-// does not: systems above about 600,000 unknowns, SVV operators, and the
-// reduced-precision apply.
+// does not: systems too large for its patches (above about 510,000 to 587,000
+// unknowns by order and element counts), SVV operators, the reduced-precision
+// apply, and a system without memory for its packets.
 //
 // One cooperative launch runs every iteration of every solve in the batch.
 // The unknown grid of each solve is cut into tiles of kCgTileX x kCgTileY

@@ -4,9 +4,9 @@
     python tests/profile_cases.py apply_bf16 [ne]  # BF16-in, FP32 operator apply
     python tests/profile_cases.py sl [ne]          # first-order SL advection
     python tests/profile_cases.py sl2 [ne]         # second-order SL advection
-    python tests/profile_cases.py cg [ne]          # persistent Jacobi-PCG solve
+    python tests/profile_cases.py cg [ne]          # Jacobi-PCG solve, on the chip where it fits
     python tests/profile_cases.py fdm [ne]         # one FDM solve (a CUDA graph)
-    python tests/profile_cases.py fdm_apply [ne]   # the FDM transform: 4 product kernels
+    python tests/profile_cases.py fdm_apply [ne]   # the FDM inverse: Bloch passes, or products (folded where it pays)
     python tests/profile_cases.py fdm_apply_tc [ne]  # the same on the tcgen05 tensor cores (TF32 hi/lo)
     python tests/profile_cases.py residual [ne]    # the refinement residual r = b - A x (double-double)
 
