@@ -1076,15 +1076,21 @@ int refine_eig(int n, const std::vector<double>& K, const std::vector<double>& W
   return SE_OK;
 }
 
-// Generalised eigenvectors E (E^T K E = diag(lam), E^T W E = I; column-major)
-// of one symmetric pair of size n: eigenvectors of W^-1/2 K W^-1/2 by cuSOLVER
-// syevd (setup only), scaled by W^-1/2, then refined (refine_eig).
-int eig_pair(int n, const std::vector<double>& K, const std::vector<double>& W,
-             std::vector<double>& A, std::vector<double>& lam) {
-  A.resize((size_t)n * n);
+// A cuSOLVER handle for the eigenproblems of one set-up, created by the first
+// (creating and destroying one takes milliseconds, several times a small
+// direction's eigenproblem).
+struct EigSolver {
+  cusolverDnHandle_t h = nullptr;
+  bool ready() { return h || cusolverDnCreate(&h) == CUSOLVER_STATUS_SUCCESS; }
+  ~EigSolver() {
+    if (h) cusolverDnDestroy(h);
+  }
+};
+
+// Eigenvectors (columns of A, column-major, overwriting it) and ascending
+// eigenvalues of a symmetric matrix by cuSOLVER syevd (set-up only).
+int syevd(EigSolver& es, int n, std::vector<double>& A, std::vector<double>& lam) {
   lam.resize(n);
-  for (int i = 0; i < n; i++)
-    for (int j = 0; j < n; j++) A[(size_t)j * n + i] = K[(size_t)i * n + j] / std::sqrt(W[i] * W[j]);
   double *dA = nullptr, *dlam = nullptr, *work = nullptr;
   int* info = nullptr;
   int rc;
@@ -1094,9 +1100,9 @@ int eig_pair(int n, const std::vector<double>& K, const std::vector<double>& W,
     dfree(info);
     return rc;
   }
-  cusolverDnHandle_t h = nullptr;
   int lwork = 0, hinfo = 0;
-  bool ok = cusolverDnCreate(&h) == CUSOLVER_STATUS_SUCCESS;
+  bool ok = es.ready();
+  const cusolverDnHandle_t h = es.h;
   ok = ok && cudaMemcpy(dA, A.data(), sizeof(double) * A.size(), cudaMemcpyHostToDevice) == cudaSuccess;
   ok = ok && cusolverDnDsyevd_bufferSize(h, CUSOLVER_EIG_MODE_VECTOR, CUBLAS_FILL_MODE_LOWER, n, dA, n,
                                          dlam, &lwork) == CUSOLVER_STATUS_SUCCESS;
@@ -1106,24 +1112,75 @@ int eig_pair(int n, const std::vector<double>& K, const std::vector<double>& W,
   ok = ok && cudaMemcpy(&hinfo, info, sizeof(int), cudaMemcpyDeviceToHost) == cudaSuccess && hinfo == 0;
   ok = ok && cudaMemcpy(A.data(), dA, sizeof(double) * A.size(), cudaMemcpyDeviceToHost) == cudaSuccess;
   ok = ok && cudaMemcpy(lam.data(), dlam, sizeof(double) * n, cudaMemcpyDeviceToHost) == cudaSuccess;
-  if (h) cusolverDnDestroy(h);
   dfree(work);
   dfree(info);
   dfree(dA);
   dfree(dlam);
   if (!ok) return fail(SE_ERR_CUDA, "eigendecomposition of the 1-D operator failed (n=%d)", n);
-  for (int j = 0; j < n; j++)
-    for (int i = 0; i < n; i++) A[(size_t)j * n + i] /= std::sqrt(W[i]);
-  return refine_eig(n, K, W, A, lam);
+  return SE_OK;
+}
+
+// One symmetric pair (K, W diagonal; K row-major) and its generalised
+// eigenvectors E (E^T K E = diag(lam), E^T W E = I; column-major).
+struct EigPair {
+  int n = 0;
+  std::vector<double> K, W, E, lam;
+  double entry(int i, int j) const { return K[(size_t)i * n + j] / std::sqrt(W[i] * W[j]); }
+};
+
+// The eigenvectors of one pair, or of the two parts of a folded direction:
+// those of W^-1/2 K W^-1/2 (syevd), scaled by W^-1/2, then refined
+// (refine_eig). syevd's time hardly depends on the size below a few hundred
+// (n = 128 2.0 ms, 256 2.3), so the parts of a short direction share one, block
+// by block, the second's eigenvalues shifted past the first's: the
+// eigenvectors stay apart and the refinement has the unshifted pairs.
+constexpr int kEigTogether = 320;
+int eig_pairs(EigSolver& es, std::vector<EigPair>& parts) {
+  int total = 0;
+  for (const EigPair& p : parts) total += p.n;
+  const bool together = parts.size() == 2 && total <= kEigTogether;
+  for (size_t q = 0; q < parts.size(); q += together ? 2 : 1) {
+    const int nq = together ? total : parts[q].n, n0 = parts[q].n;
+    std::vector<double> A((size_t)nq * nq, 0.0), l;
+    double bound = 0.0;  // of the eigenvalues (row sums)
+    for (int b = 0; b < (together ? 2 : 1); b++) {
+      const EigPair& p = parts[q + b];
+      const int o = b ? n0 : 0;
+      for (int i = 0; i < p.n; i++) {
+        double row = 0.0;
+        for (int j = 0; j < p.n; j++) {
+          const double v = p.entry(i, j);
+          A[(size_t)(o + j) * nq + o + i] = v;
+          row += std::fabs(v);
+        }
+        bound = std::max(bound, row);
+      }
+    }
+    for (int i = n0; i < nq; i++) A[(size_t)i * nq + i] += 2.0 * bound;
+    if (int rc = syevd(es, nq, A, l)) return rc;
+    for (int b = 0; b < (together ? 2 : 1); b++) {
+      EigPair& p = parts[q + b];
+      const int o = b ? n0 : 0;
+      p.E.resize((size_t)p.n * p.n);
+      p.lam.resize(p.n);
+      for (int k = 0; k < p.n; k++) {
+        p.lam[k] = l[o + k] - (b ? 2.0 * bound : 0.0);
+        for (int i = 0; i < p.n; i++)
+          p.E[(size_t)k * p.n + i] = A[(size_t)(o + k) * nq + o + i] / std::sqrt(p.W[i]);
+      }
+      if (int rc = refine_eig(p.n, p.K, p.W, p.E, p.lam)) return rc;
+    }
+  }
+  return SE_OK;
 }
 
 // A direction is its own mirror image when it is periodic or both its ends
 // are of one kind: all elements are equal and the GLL nodes symmetric.
-FoldDir fold_of(const Dir& d, bool fold = true) {
+FoldDir fold_of(const Dir& d) {
   FoldDir f;
   f.n = d.hi - d.lo;
   f.periodic = d.periodic != 0;
-  f.on = fold && f.n > 1 && (d.periodic || d.lo == d.nV - d.hi);
+  f.on = f.n > 1 && (d.periodic || d.lo == d.nV - d.hi);
   f.ge = !f.on ? f.n : f.periodic ? f.n / 2 + 1 : (f.n + 1) / 2;
   f.go = f.n - f.ge;
   f.os = (f.ge + 1) & ~1;
@@ -1187,25 +1244,28 @@ void expand(const FoldDir& f, const std::vector<double>& FE, const std::vector<d
 // folded block is the pair's own eigenproblem on the sums (differences) of
 // mirrored unknowns: K and W summed over the mirrored entries (with the odd
 // part's signs), which has no degenerate pairs (a periodic direction's sine
-// and cosine modes fall into different blocks) and an eighth of the work each.
-int eig_1d(const Dir& d, const FoldDir& f, const double* Kh, const double* w, std::vector<double>& E,
-           std::vector<double>& lam, Factors& F) {
+// and cosine modes fall into different blocks).
+int eig_1d(EigSolver& es, const Dir& d, const FoldDir& f, const double* Kh, const double* w,
+           std::vector<double>& E, std::vector<double>& lam, Factors& F) {
   std::vector<double> K, W;
   assemble_1d(d, Kh, w, K, W);
   const int n = f.n;
-  if (!f.on) {
-    if (int rc = eig_pair(n, K, W, E, lam)) return rc;
-    F.append(n, E, lam);
-    return SE_OK;
-  }
-  for (int part = 0; part < 2; part++) {
-    const int first = part && f.periodic ? 1 : 0, m = part ? n - f.ge : f.ge;
-    if (m == 0) continue;
+  std::vector<EigPair> parts(f.on && f.go > 0 ? 2 : 1);
+  for (int part = 0; part < (int)parts.size(); part++) {
+    EigPair& p = parts[part];
+    if (!f.on) {
+      p.n = n;
+      p.K = std::move(K);
+      p.W = std::move(W);
+      break;
+    }
+    const int first = part && f.periodic ? 1 : 0, m = p.n = part ? f.go : f.ge;
     const double sg = part ? -1.0 : 1.0;
-    std::vector<double> Kp((size_t)m * m), Wp(m), A, l;
+    p.K.resize((size_t)m * m);
+    p.W.resize(m);
     for (int a = 0; a < m; a++) {
       const int i = a + first, im = fold_mirror(f, i);
-      Wp[a] = im != i ? W[i] + W[im] : W[i];
+      p.W[a] = im != i ? W[i] + W[im] : W[i];
       for (int b = 0; b < m; b++) {
         const int j = b + first, jm = fold_mirror(f, j);
         double v = K[(size_t)i * n + j];
@@ -1215,17 +1275,17 @@ int eig_1d(const Dir& d, const FoldDir& f, const double* Kh, const double* w, st
           if (jm != j) u += sg * K[(size_t)im * n + jm];
           v += sg * u;
         }
-        Kp[(size_t)a * m + b] = v;
+        p.K[(size_t)a * m + b] = v;
       }
     }
     for (int a = 0; a < m; a++)
       for (int b = 0; b < a; b++) {  // symmetric to the last bit
-        const double v = 0.5 * (Kp[(size_t)a * m + b] + Kp[(size_t)b * m + a]);
-        Kp[(size_t)a * m + b] = Kp[(size_t)b * m + a] = v;
+        const double v = 0.5 * (p.K[(size_t)a * m + b] + p.K[(size_t)b * m + a]);
+        p.K[(size_t)a * m + b] = p.K[(size_t)b * m + a] = v;
       }
-    if (int rc = eig_pair(m, Kp, Wp, A, l)) return rc;
-    F.append(m, A, l);
   }
+  if (int rc = eig_pairs(es, parts)) return rc;
+  for (const EigPair& p : parts) F.append(p.n, p.E, p.lam);
   expand(f, F.FE, F.lamF, E, lam);
   return SE_OK;
 }
@@ -1266,7 +1326,7 @@ struct Eig1D {
   double* lam = nullptr;  // eigenvalues, ascending
   double lmax = 0.0;
   // FP64 inverse: the direction folded where it can be, and whole where it
-  // cannot or is short (kPlainMax)
+  // cannot or (made when first used) is short (kPlainMax)
   EigForm folded, plain;
   void* low[3] = {nullptr, nullptr, nullptr};   // [2] BF16 copy of S = row-major E^T
   void* lowT[3] = {nullptr, nullptr, nullptr};  // and of ST = row-major E
@@ -1279,7 +1339,7 @@ typedef std::tuple<int, int, int, int, int, int> EigKey;
 std::mutex g_eig_mu;
 std::map<EigKey, Eig1D*> g_eig[64];
 
-// Longest direction kept whole beside its folded form.
+// Longest direction that may be kept whole beside its folded form.
 constexpr int kPlainMax = 256;
 
 int upload_doubles(double** dst, const std::vector<double>& v) {
@@ -1306,17 +1366,17 @@ int upload_form(EigForm& e, const FoldDir& f, const Factors& F) {
 
 // Full eigenvectors (column-major, ascending eigenvalues) from a direction's
 // factors on the device.
-int full_vectors(const Eig1D& e, std::vector<double>& E) {
+int full_vectors(const Eig1D& e, std::vector<double>& E, std::vector<double>* lam = nullptr) {
   const EigForm& q = e.folded.FE ? e.folded : e.plain;
   const FoldDir& f = q.fold;
-  std::vector<double> FE((size_t)f.ge * f.os + (size_t)f.go * (f.len - f.os)), lamF(f.len), lam;
+  std::vector<double> FE((size_t)f.ge * f.os + (size_t)f.go * (f.len - f.os)), lamF(f.len), l;
   CK(cudaMemcpy(FE.data(), q.FE, sizeof(double) * FE.size(), cudaMemcpyDeviceToHost));
   CK(cudaMemcpy(lamF.data(), q.lamF, sizeof(double) * lamF.size(), cudaMemcpyDeviceToHost));
-  expand(f, FE, lamF, E, lam);
+  expand(f, FE, lamF, E, lam ? *lam : l);
   return SE_OK;
 }
 
-int eig_get(const Dir& d, const double* Kh, const double* w, int prec, Eig1D** out) {
+int eig_get(EigSolver& es, const Dir& d, const double* Kh, const double* w, int prec, Eig1D** out) {
   int dev = 0;
   CK(cudaGetDevice(&dev));
   if (dev < 0 || dev >= 64) return fail(SE_ERR_UNSUPPORTED, "device index %d", dev);
@@ -1330,16 +1390,11 @@ int eig_get(const Dir& d, const double* Kh, const double* w, int prec, Eig1D** o
     std::vector<double> lam;
     Factors F;
     const FoldDir f = fold_of(d);
-    int rc = eig_1d(d, f, Kh, w, Sh, lam, F);
+    int rc = eig_1d(es, d, f, Kh, w, Sh, lam, F);
     if (!rc) {
       for (double v : lam) ne->lmax = std::max(ne->lmax, std::fabs(v));
       (void)((rc = upload_doubles(&ne->lam, lam)) ||
              (rc = upload_form(f.on ? ne->folded : ne->plain, f, F)));
-      if (!rc && f.on && n <= kPlainMax) {
-        Factors P;
-        P.append(n, Sh, lam);
-        rc = upload_form(ne->plain, fold_of(d, false), P);
-      }
     }
     if (rc) {
       dfree(ne->lam);
@@ -1532,10 +1587,34 @@ int bloch_get(const Dir& d, const double* Kh, const double* w, Bloch1D** out) {
 // and 289. Neither: 602,176 unknowns 315 us through the two passes, 291 without.
 constexpr long kFoldBoth = 4096, kFoldOne = 32768;
 bool fdm_folds(const Eig1D& x, const Eig1D& y) {
-  if (!x.plain.FE || !y.plain.FE) return true;
-  const long n = (long)x.n * y.n;
   const bool fx = x.folded.FE, fy = y.folded.FE;
+  if ((fx && x.n > kPlainMax) || (fy && y.n > kPlainMax)) return true;
+  const long n = (long)x.n * y.n;
   return fx && fy ? n > kFoldBoth : (fx || fy) && n > kFoldOne;
+}
+
+// A direction's whole form, made from the folded one on first use.
+int plain_form(Eig1D* e) {
+  std::lock_guard<std::mutex> lk(g_eig_mu);
+  if (e->plain.FE) return SE_OK;
+  std::vector<double> E, lam;
+  if (int rc = full_vectors(*e, E, &lam)) return rc;
+  Factors P;
+  P.append(e->n, E, lam);
+  FoldDir f = e->folded.fold;  // the same direction, not folded
+  f.on = 0;
+  f.ge = f.n;
+  f.go = 0;
+  f.os = f.len = (f.n + 1) & ~1;
+  EigForm q;
+  const int rc = upload_form(q, f, P);
+  if (rc) {
+    for (double* d : {q.FE, q.FT, q.lamF, q.low8})
+      if (d) cudaFree(d);
+    return rc;
+  }
+  e->plain = q;
+  return SE_OK;
 }
 
 int fdm_setup(se_linsys* ls, int prec) {
@@ -1546,11 +1625,17 @@ int fdm_setup(se_linsys* ls, int prec) {
   const size_t n = (size_t)ls->n;
   int rc;
   Eig1D *ex = nullptr, *ey = nullptr;
-  if ((rc = eig_get(op.d[0], op.Kh, op.w, prec, &ex)) || (rc = eig_get(op.d[1], op.Kh, op.w, prec, &ey)))
-    return rc;
+  {
+    EigSolver es;
+    if ((rc = eig_get(es, op.d[0], op.Kh, op.w, prec, &ex)) ||
+        (rc = eig_get(es, op.d[1], op.Kh, op.w, prec, &ey)))
+      return rc;
+  }
   ls->lx = ex->lam;
   ls->ly = ey->lam;
-  const bool folds = fdm_folds(*ex, *ey);
+  const bool bloch = bloch_ok(op.d[0]) && bloch_ok(op.d[1]);  // uses neither form
+  const bool folds = bloch || fdm_folds(*ex, *ey);
+  if (!folds && ((rc = plain_form(ex)) || (rc = plain_form(ey)))) return rc;
   ls->eigx = folds && ex->folded.FE ? &ex->folded : &ex->plain;
   ls->eigy = folds && ey->folded.FE ? &ey->folded : &ey->plain;
   ls->lmax[0] = ex->lmax;
@@ -1566,7 +1651,7 @@ int fdm_setup(se_linsys* ls, int prec) {
         (rc = dalloc(&ls->zlow, kFdmLow * kFdmLow)) || (rc = dalloc(&ls->fpart, 2 * (size_t)ls->fpart_n + 16)))
       return rc;
     CK(cudaMemsetAsync(ls->zlow, 0, sizeof(double) * kFdmLow * kFdmLow, g_stream));
-    if (bloch_ok(op.d[0]) && bloch_ok(op.d[1])) {
+    if (bloch) {
       Bloch1D *bx = nullptr, *by = nullptr;
       if ((rc = bloch_get(op.d[0], op.Kh, op.w, &bx)) || (rc = bloch_get(op.d[1], op.Kh, op.w, &by)))
         return rc;
