@@ -19,7 +19,9 @@ struct Eo {
   static constexpr int NC = E * E + H * H;    // coefficients: Ce [E][E], then Co [H][H]
 };
 
-// The coefficients of scale * Kh, each pair of mirrored entries averaged.
+// The coefficients of scale * Kh, each pair of mirrored entries averaged (in
+// double: the products' error is the same with long double coefficients at
+// every order).
 template <int N, class A>
 inline void eo_coefs(const double* Kh, double scale, A* cf) {
   constexpr int H = Eo<N>::H, E = Eo<N>::E, n = N + 1;
