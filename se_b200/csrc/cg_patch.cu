@@ -930,7 +930,8 @@ cudaError_t launch_cg_patch(const PatchLaunch& L, cudaStream_t s) { return dispa
 // latency (reductions through L2, block sums, scalars) they matched 16x16
 // p = 6 over 64 blocks (7900) and 64x64 p = 8 over 143 (12000); inside a
 // cluster the latency is about 3100 (16x16 p = 6 over 16 blocks: 5000). So
-// systems up to about 25,000 unknowns run as a cluster. What fits a grid runs
+// systems up to 21,000 to 37,000 unknowns, by order and element counts, run as a
+// cluster. What fits a grid runs
 // as one: with the state in shared memory (more than 2048 nodes a block) an
 // iteration takes 7.3 us at 322,560 unknowns, p = 8 (streaming 26.1), 8.3 at
 // 518,400, p = 6 (31.7), 10.6 at 484,416, p = 12 (39.4).
